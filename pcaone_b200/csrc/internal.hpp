@@ -175,7 +175,7 @@ struct pcaone_ctx {
   // kernels whose dynamic shared-memory limit was raised on this context's device
   std::set<const void*> smem_attr_set;
 
-  // resident clusters of the cluster kernels, by kernel and shape (gram.hpp)
+  // resident clusters of the cluster kernels, by kernel and shape (tall.hpp)
   std::map<std::pair<const void*, uint64_t>, int> cluster_occupancy;
 
   // timing

@@ -48,6 +48,7 @@
 #include <cstdlib>
 
 #include "internal.hpp"
+#include "quant.hpp"
 #include "rsvd.hpp"
 #include "tc_ptx.hpp"
 
@@ -65,17 +66,15 @@ using tc::smem_desc_sw128;
 using tc::smem_u32;
 
 constexpr int kRows = 128;                       // rows per tile
-constexpr int kChunk = 128;                      // codes per K chunk (32 packed bytes per row)
+constexpr int kChunk = kI8Chunk;                 // codes per K chunk (32 packed bytes per row)
 constexpr int kPairChunkBytes = 2 * kRows * 32;  // one chunk of a tile pair: 8192 bytes
 constexpr int kHalfBytes = kRows * 16;           // 64 codes of one tile: 2048 bytes
 constexpr int kThreads = 480;                    // 8 decoders + producer + 2 MMA + 4 readout warps
 constexpr int kTmemCols = 512;
 constexpr int kMinUnitsPerCta = 2;
 
-// Column layout of the quantised operand: piece p of column c is row p * LP + c of B (and
-// column p * LP + c of the accumulator), LP = l rounded up to 8.
-__host__ __device__ constexpr int lp_of(int l) { return (l + 7) / 8 * 8; }
-__host__ __device__ constexpr int np_of(int l) { return (3 * lp_of(l) + 15) / 16 * 16; }
+__host__ __device__ constexpr int lp_of(int l) { return i8_lp(l); }
+__host__ __device__ constexpr int np_of(int l) { return i8_np(l); }
 
 // Pipeline shape of variant V (chosen per product shape by the autotuner in run_i8):
 // bit 0 clear: units of two K chunks, two units in flight in tensor memory per tile; set:
@@ -449,60 +448,29 @@ __global__ void k_colmax(const T* __restrict__ X, int64_t K, int l, unsigned lon
     if (sm[c]) atomicMax(&qmax[c], sm[c]);
 }
 
-// Piece scales of column c from its maximum: sig0 = max / 127, sig1 = sig0 / 254,
-// sig2 = sig1 / 254, in FP32 (the same values in the quantiser and in the GEMM readout).
-__device__ __forceinline__ void piece_scales(unsigned long long bits, float* s) {
-  const double mx = __longlong_as_double((long long)bits);
-  s[0] = mx > 0.0 ? (float)(mx / 127.0) : 1.0f;
-  s[1] = s[0] / 254.0f;
-  s[2] = s[1] / 254.0f;
-}
-
 // Quantised B of one chunk per CTA: every byte of the chunk's NP x 128 image is written
-// (piece rows, zero rows past 3 LP and past l, zero K positions that hold no operand row).
-// The image is assembled in shared memory: thread task = one (K position kk, column c)
-// element, whose three pieces (each the rounded residual of the previous ones, |q| <= 127) go
-// to rows c, LP + c, 2 LP + c at the byte that the decoder's order gives code kk (16-byte
-// unit u = kk / 16, byte 8 (o & 1) + (o >> 1) for o = kk % 16, units 128-byte swizzled); the
-// image then leaves as 16-byte stores. Operand row k is present when it lies in the first
-// wlen rows of its window of kpw rows (windows w = k / kpw) and w * wlen + (k % kpw) < mtot.
-// CTA 0 also writes the 3 x LP scales.
+// (piece rows, zero rows past 3 LP and past l, zero K positions that hold no operand row). The
+// image is assembled in shared memory (quant.hpp), a thread task per element, and leaves as
+// 16-byte stores. Operand row k is present when it lies in the first wlen rows of its window of
+// kpw rows (windows w = k / kpw) and w * wlen + (k % kpw) < mtot. CTA 0 also writes the 3 x LP
+// scales.
 template <typename T>
 __global__ void __launch_bounds__(256) k_quant(const T* __restrict__ X, int64_t kpw, int64_t wlen, int64_t mtot,
                                                int l, int lp, int np, const unsigned long long* __restrict__ qmax,
                                                int8_t* __restrict__ bq, float* __restrict__ sig) {
   __shared__ __align__(16) uint8_t img[192 * 128];
-  __shared__ float sc[3][64];
+  __shared__ PieceTable tab;
   const int64_t kc = blockIdx.x;
-  for (int c = threadIdx.x; c < lp; c += blockDim.x) {
-    float s[3] = {1.0f, 1.0f, 1.0f};
-    if (c < l) piece_scales(qmax[c], s);
-    sc[0][c] = s[0];
-    sc[1][c] = s[1];
-    sc[2][c] = s[2];
-    if (kc == 0) {
-      sig[c] = s[0];
-      sig[lp + c] = s[1];
-      sig[2 * lp + c] = s[2];
-    }
-  }
+  tab.fill(qmax, l, lp, sig, kc == 0);
   uint4* img4 = reinterpret_cast<uint4*>(img);
   for (int t = threadIdx.x; t < np * 8; t += blockDim.x) img4[t] = make_uint4(0u, 0u, 0u, 0u);
   __syncthreads();
+#pragma unroll 4
   for (int e = threadIdx.x; e < kChunk * l; e += blockDim.x) {
     const int kk = e / l, c = e - kk * l;
     const int64_t k = kc * kChunk + kk, w = k / kpw, r = k - w * kpw;
     if (r >= wlen || w * wlen + r >= mtot) continue;
-    double x = (double)X[k * l + c];
-    const int u = kk >> 4, o = kk & 15, pp = 8 * (o & 1) + (o >> 1);
-#pragma unroll
-    for (int p = 0; p < 3; ++p) {
-      const double s = (double)sc[p][c];
-      const double q = fmin(127.0, fmax(-127.0, rint(x / s)));
-      x -= q * s;
-      const int n = p * lp + c;
-      img[n * 128 + ((u ^ (n & 7)) << 4) + pp] = (uint8_t)(int8_t)(int)q;
-    }
+    tab.put(img, kk, c, lp, (double)X[k * l + c]);
   }
   __syncthreads();
   uint4* dst = reinterpret_cast<uint4*>(bq + kc * (int64_t)np * 128);
@@ -771,6 +739,13 @@ void i8_omega(pcaone_ctx* c, const double* omega, int l, int64_t npad) {
   quantize<double>(c, omega, (int64_t)c->N, l, npad, "1", false);
 }
 
+// Where the fused Omega update leaves the operand copy i8_omega would make.
+OmegaI8 i8_omega_operand(pcaone_ctx* c, int l) {
+  return OmegaI8{(unsigned long long*)scratch(c, "i8_qmax1", 64 * sizeof(unsigned long long)),
+                 (int8_t*)scratch(c, "i8_bq1", (size_t)c->Npad * np_of(l)),
+                 (float*)scratch(c, "i8_sig1", 3 * 64 * sizeof(float))};
+}
+
 void i8_b2(pcaone_ctx* c, const float* B2, int l, int64_t m) {
   quantize<float>(c, B2, m, l, (int64_t)round_up(c->win.blocksize, 256), "2", c->i8_b2_max_ready);
   c->i8_b2_max_ready = false;
@@ -876,6 +851,7 @@ void i8_tile_window(pcaone_ctx* c, cudaStream_t st, const uint8_t* rec, int64_t 
 
 GemmFnT<float> gemm_i8() {
   GemmFnT<float> f{i8_ksplit, i8_p1, i8_p2, i8_omega, i8_b2, nullptr, nullptr, i8_b2_qmax};
+  f.omega_i8 = i8_omega_operand;
   f.seg_rows1 = i8_seg_rows1;
   f.seg_k2 = i8_seg_k2;
   f.ksplit_seg = i8_ksplit_seg;

@@ -1,214 +1,262 @@
-// FP64 kernels for the (k+p)-wide sketch outside the fused Omega update: Gram matrices,
-// Cholesky and triangular solves (CholeskyQR2 of the epoch tail), column sums and small
-// products.
+// FP64 kernels on tall row-major matrices (one sample or SNP per row, l <= kLmax columns) for the
+// Omega update and the epoch tail: Gram products, products with a small factor, the l x l
+// factorisations between them, column sums.
 //
-// Tall matrices are row-major n x l (one sample or SNP per row, l <= kLmax columns).
-// All reductions run in a fixed order (per-CTA or per-cluster partials, then a fixed-order
-// sum), so results are deterministic run to run.
-#include "gram.hpp"
-#include "internal.hpp"
+// CholeskyQR2 as a chain of passes (TallStep): every pass reads its rows once, applies the
+// inverse factor of the pass before, sums the Gram matrix, and its last CTA factors and inverts
+// it, so a pass is one launch. The passes over N x l matrices (0.2 - 6 MB, in L2) are bound by
+// latency: launch, one round of loads, the reductions, and the l x l factorisation in one CTA.
+// The passes over G (M x l) are bound by HBM.
 #include "linalg.hpp"
+
+#include <algorithm>
+
+#include "tall.hpp"
 
 namespace pg {
 
 namespace {
 
-// A^T B over rows: each CTA of a cluster streams its contiguous row block through two
-// shared-memory stages (cp.async, the next batch in flight while the current one is summed
-// into 4 x 4 register tiles, gram.hpp), sums its thread groups, and the cluster adds its CTAs'
-// sums through distributed shared memory into gpart[cluster] (ntiles * 16 values in tile
-// layout). SYM (A == B): only the tiles on and above the diagonal, one staged copy.
-constexpr int kCrossThreads = 256;
-constexpr int kCrossMaxClusters = kGramMaxParts;
-constexpr int kCrossSmemBudget = 96 * 1024;  // two CTAs an SM
+template <int NT, bool RECT>
+struct TallCfg {
+  static constexpr int NB = (NT + 1) / 2;  // column tiles of B per pass over the rows
+  static constexpr int kAcc = RECT ? NT * NB : Tall<NT>::kTiles;
+  static constexpr int kRed = kTallWarps * kAcc * 64;
+  static constexpr int kPost = RECT ? 0 : 4 * Tall<NT>::kSq + Tall<NT>::kWarpScratch;
+  static constexpr size_t smem(bool prod) {
+    return ((prod ? Tall<NT>::kSq : 0) + (size_t)kAcc * 64 + (kRed > kPost ? kRed : kPost)) * 8;
+  }
+};
 
-__device__ __forceinline__ void cp_async8(double* sdst, const double* gsrc) {
-  const unsigned d = (unsigned)__cvta_generic_to_shared(sdst);
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(d), "l"(gsrc) : "memory");
-}
-
-template <bool SYM>
-__global__ void __cluster_dims__(kGramCluster, 1, 1) __launch_bounds__(kCrossThreads)
-    k_cross(const double* __restrict__ A, int la, const double* __restrict__ Bm, int lb, int64_t n, int rows,
-            double* __restrict__ gpart) {
-  extern __shared__ double sm[];
-  const GramTiling g = gram_tiling(la, lb, SYM, blockDim.x);
-  const int w = g.la4 + (SYM ? 0 : g.lb4);  // staged doubles per row: A rows (la4), then B rows (lb4)
-  double* red = sm + 2 * rows * w;  // stages: sm and sm + rows * w
-  double* cpart = red + g.ngrp * g.ntiles * 16;
-  for (int t = threadIdx.x; t < 2 * rows; t += blockDim.x) {  // zero padding columns, never copied
-    double* base = sm + (t / rows) * rows * w;
-    const int r = t % rows;
-    for (int cc = la; cc < g.la4; ++cc) base[r * g.la4 + cc] = 0.0;
-    if (!SYM)
-      for (int cc = lb; cc < g.lb4; ++cc) base[rows * g.la4 + r * g.lb4 + cc] = 0.0;
+// See TallStep. Warp w of a CTA takes the 8-row groups w, w + 8, ... of the CTA's rows; the
+// next group's loads are in flight while the current one is multiplied (narrow matrices: the
+// registers of wider ones go to the accumulators).
+// Measured (ncu, us a launch; before: rows solved by substitution a thread each, 4 x 4 FMA tiles
+// from shared memory, Cholesky with a barrier a column, separate factorisation launches):
+//   Omega update without its operand copy, N = 20000, l = 40: 74 (was 176); N = 5003, l = 20: 44 (71)
+//   whole update with the int8 operand: 87 (216) and 52 (98)
+//   G passes of the epoch tail, M = 500000, l = 40: 71 + 105 (50 + 298, plus two Choleskys of 37);
+//   the tail at M = 50000, N = 2000, l = 20: 92 an epoch (176)
+template <int NT, bool PROD, bool RECT>
+__global__ void __cluster_dims__(kTallCluster, 1, 1) __launch_bounds__(kTallThreads) k_tall(TallStep a) {
+  using T = Tall<NT>;
+  using C = TallCfg<NT, RECT>;
+  constexpr int LD = T::LD, NB = C::NB, NACC = C::kAcc;
+  constexpr bool kPrefetch = NT <= 5;
+  extern __shared__ __align__(16) double sm[];
+  double* Rs = sm;
+  double* cpart = sm + (PROD ? T::kSq : 0);
+  double* red = cpart + NACC * 64;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, q4 = lane >> 2, r4 = lane & 3;
+  const int l = a.l, lb = a.lb;
+  if constexpr (PROD) {
+    load_square<NT>(a.Rinv, l, 0.0, Rs);
+    __syncthreads();
   }
   int64_t r0, r1;
-  row_range(n, r0, r1);
-  auto issue = [&](int64_t b, double* dst) {
-    const int nr = (int)(r1 - b < rows ? r1 - b : rows);
-    for (int t = threadIdx.x; t < nr * la; t += blockDim.x) {
-      const int r = t / la;
-      cp_async8(dst + r * g.la4 + (t - r * la), A + b * la + t);
-    }
-    if (!SYM)
-      for (int t = threadIdx.x; t < nr * lb; t += blockDim.x) {
-        const int r = t / lb;
-        cp_async8(dst + rows * g.la4 + r * g.lb4 + (t - r * lb), Bm + b * lb + t);
-      }
-    asm volatile("cp.async.commit_group;\n" ::: "memory");
-  };
-  GramThread gt;
-  gt.init(g);
-  int s = 0;
-  if (r0 < r1) issue(r0, sm);
-  for (int64_t b = r0; b < r1; b += rows) {
-    const int nr = (int)(r1 - b < rows ? r1 - b : rows);
-    if (b + rows < r1) {
-      issue(b + rows, sm + (s ^ 1) * rows * w);
-      asm volatile("cp.async.wait_group 1;\n" ::: "memory");
-    } else {
-      asm volatile("cp.async.wait_group 0;\n" ::: "memory");
-    }
-    __syncthreads();  // stage s complete (and the padding zeroed) for every thread
-    const double* sa = sm + s * rows * w;
-    gt.add_rows(sa, SYM ? sa : sa + rows * g.la4, nr, g);
-    __syncthreads();  // stage s is consumed before it is refilled
-    s ^= 1;
-  }
-  gt.finish(g, red, cpart);
-  cluster_sum(cpart, g.ntiles * 16, gpart);
-}
+  tall_rows(a.n, blockIdx.x, gridDim.x, r0, r1);
+  const int ncl = gridDim.x / kTallCluster;
+  const int passes = RECT ? ((lb + 7) / 8 + NB - 1) / NB : 1;
 
-// Gram of Q1 = A R^{-1} without writing Q1 (the second pass of CholeskyQR2 when only its R
-// is needed): k_cross<true> with a product step. Each staged batch of rows (row stride
-// la4 + 2, 16-byte aligned) is multiplied by Rinv = R^{-1} (upper, staged in shared memory
-// with row stride LMAX and zeros outside l x l) in 4 x 4 register tiles, a thread per tile
-// (the host sizes the batch so that one pass of the CTA covers it), written back in place
-// and then summed into the Gram tiles.
-template <int LMAX>
-__global__ void __cluster_dims__(kGramCluster, 1, 1) __launch_bounds__(kCrossThreads)
-    k_cross_solved(const double* __restrict__ A, const double* __restrict__ Rinv, int l, int64_t n, int rows,
-                   double* __restrict__ gpart) {
-  extern __shared__ double sm[];
-  const GramTiling g = gram_tiling(l, l, true, blockDim.x);
-  GramTiling gs = g;  // the tile reads with the staged row stride
-  gs.la4 = gs.lb4 = g.la4 + 2;
-  const int w = gs.la4;
-  double* Rs = sm;  // LMAX x LMAX
-  double* st = Rs + LMAX * LMAX;
-  double* red = st + 2 * rows * w;
-  double* cpart = red + g.ngrp * g.ntiles * 16;
-  for (int t = threadIdx.x; t < LMAX * LMAX; t += blockDim.x) {
-    const int i = t / LMAX, j = t - i * LMAX;
-    Rs[t] = (i < l && j < l) ? Rinv[i * l + j] : 0.0;
-  }
-  for (int t = threadIdx.x; t < 2 * rows; t += blockDim.x)  // padding columns, never copied or written
-    for (int cc = l; cc < w; ++cc) st[t * w + cc] = 0.0;
-  int64_t r0, r1;
-  row_range(n, r0, r1);
-  auto issue = [&](int64_t b, double* dst) {
-    const int nr = (int)(r1 - b < rows ? r1 - b : rows);
-    for (int t = threadIdx.x; t < nr * l; t += blockDim.x) {
-      const int r = t / l;
-      cp_async8(dst + r * w + (t - r * l), A + b * l + t);
-    }
-    asm volatile("cp.async.commit_group;\n" ::: "memory");
-  };
-  GramThread gt;
-  gt.init(g);
-  int s = 0;
-  if (r0 < r1) issue(r0, st);
-  for (int64_t b = r0; b < r1; b += rows) {
-    const int nr = (int)(r1 - b < rows ? r1 - b : rows);
-    if (b + rows < r1) {
-      issue(b + rows, st + (s ^ 1) * rows * w);
-      asm volatile("cp.async.wait_group 1;\n" ::: "memory");
-    } else {
-      asm volatile("cp.async.wait_group 0;\n" ::: "memory");
-    }
-    __syncthreads();  // stage s complete, R staged, padding zeroed
-    double* sa = st + s * rows * w;
-    {
-      const int nbc = g.la4 >> 2, nbr = (nr + 3) >> 2;
-      const bool act = (int)threadIdx.x < nbr * nbc;
-      const int rb = act ? (int)threadIdx.x / nbc : 0, cb = act ? (int)threadIdx.x - rb * nbc : 0;
-      const int rr0 = 4 * rb, cc0 = 4 * cb;
-      double q[4][4];
+  // this lane's 2 NT values of the rows base .. base + 7: the operand of the product (row q4,
+  // columns 4 i + r4), or that of the Gram itself (rows r4 and r4 + 4, columns 8 t + q4)
+  auto load = [&](int64_t base, double (&x)[2 * NT], bool sum) {
+    auto row = [&](int i) { return base + (PROD ? q4 : 4 * (i & 1) + r4); };
+    auto col = [&](int i) { return PROD ? 4 * i + r4 : 8 * (i >> 1) + q4; };
 #pragma unroll
-      for (int x = 0; x < 4; ++x)
+    for (int i = 0; i < 2 * NT; ++i) x[i] = row(i) < r1 && col(i) < l ? a.A[row(i) * l + col(i)] : 0.0;
+    if constexpr (!PROD) {
+      if (a.A2) {  // every load before the first store, which may alias for all the compiler knows
+        double y[2 * NT];
 #pragma unroll
-        for (int y = 0; y < 4; ++y) q[x][y] = 0.0;
-      if (act) {
-        const int kend = l < cc0 + 4 ? l : cc0 + 4;  // Rinv is upper: rows past the tile's last column add 0
-        for (int kk = 0; kk < kend; ++kk) {
-          const double2 r01 = *reinterpret_cast<const double2*>(Rs + kk * LMAX + cc0);
-          const double2 r23 = *reinterpret_cast<const double2*>(Rs + kk * LMAX + cc0 + 2);
-          const double rv[4] = {r01.x, r01.y, r23.x, r23.y};
-          double av[4];
+        for (int i = 0; i < 2 * NT; ++i) y[i] = row(i) < r1 && col(i) < l ? a.A2[row(i) * l + col(i)] : 0.0;
 #pragma unroll
-          for (int x = 0; x < 4; ++x) av[x] = rr0 + x < nr ? sa[(rr0 + x) * w + kk] : 0.0;
-#pragma unroll
-          for (int x = 0; x < 4; ++x)
-#pragma unroll
-            for (int y = 0; y < 4; ++y) q[x][y] = fma(av[x], rv[y], q[x][y]);
+        for (int i = 0; i < 2 * NT; ++i) {
+          x[i] += y[i];
+          if (sum && row(i) < r1 && col(i) < l) a.Asum[row(i) * l + col(i)] = x[i];
         }
       }
-      __syncthreads();  // every row of the batch read before any is overwritten
-      if (act)
-#pragma unroll
-        for (int x = 0; x < 4; ++x)
-#pragma unroll
-          for (int y = 0; y < 4; ++y)
-            if (rr0 + x < nr && cc0 + y < l) sa[(rr0 + x) * w + cc0 + y] = q[x][y];
     }
-    __syncthreads();
-    gt.add_rows(sa, sa, nr, gs);
-    __syncthreads();  // stage s is consumed before it is refilled
-    s ^= 1;
-  }
-  gt.finish(g, red, cpart);
-  cluster_sum(cpart, g.ntiles * 16, gpart);
-}
+  };
 
-// out (la x lb, global) = sum of the nparts cluster sums of k_cross.
-__global__ void __launch_bounds__(kCrossThreads) k_cross_final(const double* __restrict__ gpart, int nparts, int la,
-                                                               int lb, int sym, double* __restrict__ out) {
-  const GramTiling g = gram_tiling(la, lb, sym != 0, kCrossThreads);
-  gram_final(g, gpart, nparts, la, lb, out);
-}
-
-__global__ void k_cholesky(const double* __restrict__ W, int l, double* __restrict__ R,
-                           const double* __restrict__ Rprev, double* __restrict__ Racc,
-                           double* __restrict__ Rinv, int* __restrict__ status) {
-  extern __shared__ double s[];  // l x l, then l x l for R^-1
-  for (int t = threadIdx.x; t < l * l; t += blockDim.x) s[t] = W[t];
-  const int bad = chol_upper_smem(s, l);
-  for (int t = threadIdx.x; t < l * l; t += blockDim.x) R[t] = s[t];
-  if (Rinv) {  // column j of R^-1 by back substitution (thread j), zeros below the diagonal
-    double* si = s + l * l;
-    for (int j = threadIdx.x; j < l; j += blockDim.x) {
-      for (int i = l - 1; i > j; --i) si[i * l + j] = 0.0;
-      si[j * l + j] = 1.0 / s[j * l + j];
-      for (int i = j - 1; i >= 0; --i) {
-        double acc = 0.0;
-        for (int m = i + 1; m <= j; ++m) acc = fma(s[i * l + m], si[m * l + j], acc);
-        si[i * l + j] = -acc / s[i * l + i];
+  for (int pass = 0; pass < passes; ++pass) {
+    double acc[NACC][2];
+#pragma unroll
+    for (int t = 0; t < NACC; ++t) acc[t][0] = acc[t][1] = 0.0;
+    double x[2 * NT], nx[kPrefetch ? 2 * NT : 1];
+    int64_t base = r0 + 8 * warp;
+    if (kPrefetch && base < r1) load(base, x, pass == 0);
+    for (; base < r1; base += 8 * kTallWarps) {
+      if constexpr (kPrefetch) {
+        if (base + 8 * kTallWarps < r1) load(base + 8 * kTallWarps, nx, pass == 0);
+      } else {
+        load(base, x, pass == 0);
+      }
+      double f[NT][2];  // rows row(0), row(1) of column 8 t + q4
+      if constexpr (PROD) {
+#pragma unroll
+        for (int t = 0; t < NT; ++t) f[t][0] = f[t][1] = 0.0;
+#pragma unroll
+        for (int i = 0; i < 2 * NT; ++i)
+#pragma unroll
+          for (int t = i / 2; t < NT; ++t) dmma(f[t], Rs[(4 * i + r4) * LD + 8 * t + q4], x[i]);
+        if (a.Q && pass == 0) {
+#pragma unroll
+          for (int e = 0; e < 2; ++e) {
+            const int64_t row = base + 2 * r4 + e;
+#pragma unroll
+            for (int t = 0; t < NT; ++t)
+              if (row < r1 && 8 * t + q4 < l) a.Q[row * l + 8 * t + q4] = f[t][e];
+          }
+        }
+      } else {
+#pragma unroll
+        for (int t = 0; t < NT; ++t) {
+          f[t][0] = x[2 * t];
+          f[t][1] = x[2 * t + 1];
+        }
+      }
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        if constexpr (RECT) {
+          const int64_t row = base + (PROD ? 2 * r4 + e : 4 * e + r4);
+          double b[NB];
+#pragma unroll
+          for (int j = 0; j < NB; ++j) {
+            const int col = 8 * (pass * NB + j) + q4;
+            b[j] = row < r1 && col < lb ? a.B[row * lb + col] : 0.0;
+          }
+#pragma unroll
+          for (int i = 0; i < NT; ++i)
+#pragma unroll
+            for (int j = 0; j < NB; ++j) dmma(acc[i * NB + j], f[i][e], b[j]);
+        } else {
+#pragma unroll
+          for (int i = 0; i < NT; ++i)
+#pragma unroll
+            for (int j = i; j < NT; ++j) dmma(acc[T::tile(i, j)], f[i][e], f[j][e]);
+        }
+      }
+      if constexpr (kPrefetch) {
+#pragma unroll
+        for (int i = 0; i < 2 * NT; ++i) x[i] = nx[i];
       }
     }
+#pragma unroll
+    for (int t = 0; t < NACC; ++t)
+      *reinterpret_cast<double2*>(red + (warp * NACC + t) * 64 + q4 * 8 + 2 * r4) = make_double2(acc[t][0], acc[t][1]);
     __syncthreads();
-    for (int t = threadIdx.x; t < l * l; t += blockDim.x) Rinv[t] = si[t];
+    for (int e = threadIdx.x; e < NACC * 64; e += kTallThreads) {
+      double s = 0.0;
+#pragma unroll
+      for (int w = 0; w < kTallWarps; ++w) s += red[w * NACC * 64 + e];
+      cpart[e] = s;
+    }
+    cluster_sum(cpart, NACC * 64, NACC * 64, a.part + (int64_t)pass * ncl * NACC * 64);
   }
-  __syncthreads();
-  if (Rprev) {
-    for (int t = threadIdx.x; t < l * l; t += blockDim.x) {
-      int i = t / l, j = t % l;
-      double acc = 0.0;
-      for (int k = i; k <= j; ++k) acc += R[i * l + k] * Rprev[k * l + j];
-      Racc[t] = (j >= i) ? acc : 0.0;
+  if (!last_cta(a.counter)) return;
+
+  if constexpr (RECT) {
+    for (int pass = 0; pass < passes; ++pass)
+      for (int e = threadIdx.x; e < NACC * 64; e += kTallThreads) {
+        const int t = e >> 6, i = t / NB, j = pass * NB + t % NB;
+        const int row = 8 * i + ((e & 63) >> 3), col = 8 * j + (e & 7);
+        if (row < l && col < lb)
+          a.X[row * lb + col] = sum_parts(a.part + (int64_t)pass * ncl * NACC * 64 + e, ncl, NACC * 64);
+      }
+  } else {
+    double *W = red, *R = W + T::kSq, *X = R + T::kSq, *P = X + T::kSq, *sc = P + T::kSq;
+    for (int e = threadIdx.x; e < NACC * 64; e += kTallThreads) {
+      const double v = sum_parts(a.part + e, ncl, NACC * 64);
+      int i = 0, t = e >> 6;
+      while (t >= NT - i) t -= NT - i++;
+      const int row = 8 * i + ((e & 63) >> 3), col = 8 * (i + t) + (e & 7);
+      W[row * LD + col] = (row < l && col < l) ? v : (row == col ? 1.0 : 0.0);
+    }
+    if (a.Rprev) load_square<NT>(a.Rprev, l, 1.0, P);
+    __syncthreads();
+    const int bad = chol_inverse<NT>(W, R, X, sc);
+    if (bad && threadIdx.x == 0) atomicMax(a.status, bad);
+    if (a.R) store_square<NT>(R, l, a.R);
+    if (a.Ri) store_square<NT>(X, l, a.Ri);
+    if (a.Rprev) {
+      upper_product<NT>(R, P, W);
+      store_square<NT>(W, l, a.Racc);
+      if (a.Rprev_inv) {
+        __syncthreads();
+        load_square<NT>(a.Rprev_inv, l, 1.0, P);
+        upper_product<NT>(P, X, W);
+        store_square<NT>(W, l, a.Racc_inv);
+      }
     }
   }
-  if (threadIdx.x == 0 && bad && status) atomicMax(status, bad);
+}
+
+template <int NT, bool PROD, bool RECT>
+void launch_tall(pcaone_ctx* c, TallStep s) {
+  constexpr size_t smem = TallCfg<NT, RECT>::smem(PROD);
+  static_assert(smem <= 227 * 1024, "shared memory above the per-CTA limit");
+  const void* kern = (const void*)k_tall<NT, PROD, RECT>;
+  if (c->smem_attr_set.insert(kern).second)
+    PG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  // one 8-row group a warp (64 rows a CTA) while the clusters fit at once
+  int cap = kTallMaxParts;
+  const int resident = resident_clusters(c, kern, 0, kTallThreads, smem);
+  if (resident > 0) cap = std::min(cap, resident);
+  const int ncl = tall_clusters(s.n, cap);
+  const int passes = RECT ? 2 : 1;
+  s.part = tall_part(c, (size_t)passes * TallCfg<NT, RECT>::kAcc * 64);
+  s.counter = tall_counter(c);
+  k_tall<NT, PROD, RECT><<<ncl * kTallCluster, kTallThreads, smem, c->stream>>>(s);
+  PG_CHECK_LAUNCH();
+  c->launches++;
+}
+
+template <bool PROD, bool RECT>
+void launch_tall_nt(pcaone_ctx* c, const TallStep& s) {
+  switch ((s.l + 7) / 8) {
+    case 1: launch_tall<1, PROD, RECT>(c, s); break;
+    case 2: launch_tall<2, PROD, RECT>(c, s); break;
+    case 3: launch_tall<3, PROD, RECT>(c, s); break;
+    case 4: launch_tall<4, PROD, RECT>(c, s); break;
+    case 5: launch_tall<5, PROD, RECT>(c, s); break;
+    case 6: launch_tall<6, PROD, RECT>(c, s); break;
+    case 7: launch_tall<7, PROD, RECT>(c, s); break;
+    default: launch_tall<8, PROD, RECT>(c, s); break;
+  }
+}
+
+// Forward substitution for one row: x R = a with R upper l x l staged by stage_r (row stride
+// LMAX, so every R address is a constant offset; the diagonal slots hold 1 / R_jj, so the
+// dependent chain has no division), x kept in registers (LMAX >= l; the loops unroll over LMAX
+// and skip j >= l). Every element of a is read before out is written, so out may alias a.
+template <int LMAX>
+__device__ __forceinline__ void solve_row_upper(const double* a, const double* Rs, int l, double* out) {
+  double x[LMAX];
+#pragma unroll
+  for (int j = 0; j < LMAX; ++j) {
+    if (j < l) {
+      double v = a[j];
+#pragma unroll
+      for (int k = 0; k < j; ++k) v -= x[k] * Rs[k * LMAX + j];
+      x[j] = v * Rs[j * LMAX + j];
+    } else {
+      x[j] = 0.0;
+    }
+  }
+#pragma unroll
+  for (int j = 0; j < LMAX; ++j)
+    if (j < l) out[j] = x[j];
+}
+
+// Copy R (l x l row-major, upper) into shared memory with row stride LMAX for
+// solve_row_upper: the diagonal slots get 1 / R_jj.
+template <int LMAX>
+__device__ __forceinline__ void stage_r(const double* R, int l, double* Rs) {
+  for (int t = threadIdx.x; t < l * l; t += blockDim.x) {
+    const int i = t / l, j = t - i * l;
+    Rs[i * LMAX + j] = i == j ? 1.0 / R[t] : R[t];
+  }
 }
 
 // Q = A R^{-1} (row-wise forward substitution x R = a), R upper l x l. One thread per row;
@@ -275,83 +323,25 @@ __global__ void __launch_bounds__(128) k_rowmat(const double* __restrict__ X, in
 
 }  // namespace
 
-void cross(pcaone_ctx* c, const double* A, int la, const double* B, int lb, int64_t n, double* out) {
-  PG_REQUIRE(la >= 1 && lb >= 1 && la <= kLmax && lb <= kLmax, PCAONE_EBADARG, "cross product too wide");
-  const bool sym = A == B && la == lb;
-  const GramTiling g = gram_tiling(la, lb, sym, kCrossThreads);
-  const int w = g.la4 + (sym ? 0 : g.lb4);
-  const int fixed = gram_smem_doubles(g) * 8;
-  const int rows = std::max(8, std::min(128, (kCrossSmemBudget - fixed) / (2 * w * 8)));
-  const size_t smem = (size_t)fixed + (size_t)2 * rows * w * 8;
-  const int64_t want = (n + (int64_t)kGramCluster * 4 * rows - 1) / ((int64_t)kGramCluster * 4 * rows);
-  int cap = std::max(1, std::min(kCrossMaxClusters, 2 * c->sm_count / kGramCluster));
-  const void* kern = sym ? (const void*)k_cross<true> : (const void*)k_cross<false>;
-  PG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  const int resident = resident_clusters(c, kern, ((uint64_t)la << 32) | (uint64_t)lb, kCrossThreads, smem);
-  if (resident > 0) cap = std::min(cap, resident);
-  const int ncl = (int)std::max<int64_t>(1, std::min<int64_t>(cap, want));
-  double* gpart = (double*)scratch(c, "cross_part", (size_t)ncl * g.ntiles * 16 * 8);
-  if (sym) {
-    k_cross<true><<<ncl * kGramCluster, kCrossThreads, smem, c->stream>>>(A, la, A, lb, n, rows, gpart);
-  } else {
-    k_cross<false><<<ncl * kGramCluster, kCrossThreads, smem, c->stream>>>(A, la, B, lb, n, rows, gpart);
-  }
-  PG_CHECK_LAUNCH();
-  k_cross_final<<<1, kCrossThreads, 0, c->stream>>>(gpart, ncl, la, lb, sym ? 1 : 0, out);
-  PG_CHECK_LAUNCH();
-  c->launches += 2;
+unsigned* tall_counter(pcaone_ctx* c) {
+  const bool fresh = c->bufs.find("tall_cnt") == c->bufs.end();
+  unsigned* p = (unsigned*)scratch(c, "tall_cnt", sizeof(unsigned));
+  if (fresh) PG_CUDA(cudaMemsetAsync(p, 0, sizeof(unsigned), c->stream));
+  return p;
 }
 
-void cross_solved(pcaone_ctx* c, const double* A, const double* Rinv, int l, int64_t n, double* out) {
-  PG_REQUIRE(l >= 1 && l <= kLmax, PCAONE_EBADARG, "cross product too wide");
-  const GramTiling g = gram_tiling(l, l, true, kCrossThreads);
-  const int lmax = l <= 16 ? 16 : l <= 32 ? 32 : l <= 48 ? 48 : 64;
-  const int w = g.la4 + 2;
-  const int fixed = (gram_smem_doubles(g) + lmax * lmax) * 8;
-  // one 4 x 4 product tile per thread covers a batch of rows
-  const int rows_tiles = 4 * (kCrossThreads / (g.la4 / 4));
-  const int rows = std::max(4, std::min(std::min(128, rows_tiles), (kCrossSmemBudget - fixed) / (2 * w * 8)));
-  const size_t smem = (size_t)fixed + (size_t)2 * rows * w * 8;
-  const int64_t want = (n + (int64_t)kGramCluster * 4 * rows - 1) / ((int64_t)kGramCluster * 4 * rows);
-  int cap = std::max(1, std::min(kCrossMaxClusters, 2 * c->sm_count / kGramCluster));
-  auto go = [&](auto kern) {
-    PG_CUDA(cudaFuncSetAttribute((const void*)kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    const int resident = resident_clusters(c, (const void*)kern, ((uint64_t)l << 32) | 0x5u, kCrossThreads, smem);
-    if (resident > 0) cap = std::min(cap, resident);
-    const int ncl = (int)std::max<int64_t>(1, std::min<int64_t>(cap, want));
-    double* gpart = (double*)scratch(c, "cross_part", (size_t)ncl * g.ntiles * 16 * 8);
-    kern<<<ncl * kGramCluster, kCrossThreads, smem, c->stream>>>(A, Rinv, l, n, rows, gpart);
-    PG_CHECK_LAUNCH();
-    k_cross_final<<<1, kCrossThreads, 0, c->stream>>>(gpart, ncl, l, l, 1, out);
-    PG_CHECK_LAUNCH();
-  };
-  if (lmax == 16)
-    go(k_cross_solved<16>);
-  else if (lmax == 32)
-    go(k_cross_solved<32>);
-  else if (lmax == 48)
-    go(k_cross_solved<48>);
+double* tall_part(pcaone_ctx* c, size_t doubles) {
+  return (double*)scratch(c, "tall_part", (size_t)kTallMaxParts * doubles * 8);
+}
+
+void tall_step(pcaone_ctx* c, TallStep s) {
+  PG_REQUIRE(s.l >= 1 && s.l <= kLmax && s.lb <= s.l, PCAONE_EBADARG, "sketch width out of range");
+  PG_REQUIRE(s.n >= 1 && !(s.A2 && s.Rinv), PCAONE_EBADARG, "bad tall pass");
+  PG_REQUIRE(!s.B || s.Q != s.A, PCAONE_EBADARG, "a cross pass may not overwrite its input");
+  if (s.B)
+    s.Rinv ? launch_tall_nt<true, true>(c, s) : launch_tall_nt<false, true>(c, s);
   else
-    go(k_cross_solved<64>);
-  c->launches += 2;
-}
-
-void cholqr2_r(pcaone_ctx* c, const double* A, int l, int64_t n, double* R, int* d_status) {
-  double* W = (double*)scratch(c, "cq_W", (size_t)l * l * 8);
-  double* R1 = (double*)scratch(c, "cq_R1", (size_t)l * l * 8);
-  double* R2 = (double*)scratch(c, "cq_R2", (size_t)l * l * 8);
-  double* R1i = (double*)scratch(c, "cq_R1i", (size_t)l * l * 8);
-  cross(c, A, l, A, l, n, W);
-  cholesky(c, W, l, R1, nullptr, nullptr, d_status, R1i);
-  cross_solved(c, A, R1i, l, n, W);
-  cholesky(c, W, l, R2, R1, R, d_status);
-}
-
-void cholesky(pcaone_ctx* c, const double* W, int l, double* R, const double* Rprev, double* Racc,
-              int* d_status, double* Rinv) {
-  k_cholesky<<<1, 256, (size_t)(Rinv ? 2 : 1) * l * l * 8, c->stream>>>(W, l, R, Rprev, Racc, Rinv, d_status);
-  PG_CHECK_LAUNCH();
-  c->launches++;
+    s.Rinv ? launch_tall_nt<true, false>(c, s) : launch_tall_nt<false, false>(c, s);
 }
 
 void trsm_right_upper(pcaone_ctx* c, const double* A, const double* R, int l, int64_t n, double* Q) {
@@ -366,18 +356,6 @@ void trsm_right_upper(pcaone_ctx* c, const double* A, const double* R, int l, in
     k_trsm_right_upper<64><<<grid, 128, 64 * 64 * 8, c->stream>>>(A, R, l, n, Q);
   PG_CHECK_LAUNCH();
   c->launches++;
-}
-
-void cholqr2(pcaone_ctx* c, const double* A, int l, int64_t n, double* Q, double* R, int* d_status) {
-  double* W = (double*)scratch(c, "cq_W", (size_t)l * l * 8);
-  double* R1 = (double*)scratch(c, "cq_R1", (size_t)l * l * 8);
-  double* R2 = (double*)scratch(c, "cq_R2", (size_t)l * l * 8);
-  cross(c, A, l, A, l, n, W);
-  cholesky(c, W, l, R1, nullptr, nullptr, d_status);
-  trsm_right_upper(c, A, R1, l, n, Q);
-  cross(c, Q, l, Q, l, n, W);
-  cholesky(c, W, l, R2, R1, R, d_status);
-  trsm_right_upper(c, Q, R2, l, n, Q);
 }
 
 void colsum(pcaone_ctx* c, const double* A, int l, int64_t n, double* out) {

@@ -1,28 +1,27 @@
-// Fused Omega update: Omega = flipOmg(Omega2, thin Q of H) in four launches.
+// Fused Omega update: Omega = flipOmg(Omega_prev, thin Q of H) in four launches.
 //
 // Reference: the Householder QR + householderQ() + flipOmg block of the winSVD window loop
-// (src/Halko.cpp:213-216) and of the Halko epochs (src/Halko.cpp:118-122, src/RSVD.hpp:81-90).
+// (src/Halko.cpp:213-216) and of the Halko epochs (src/Halko.cpp:118-122, src/RSVD.hpp:81-90;
+// the reference's Omega2 is a copy of the previous Omega).
 //
-//   K1  H = H1 + H2 (winSVD), W1 = H^T H                     last CTA: R1 = chol(W1)
-//   K2  Q1 = H R1^-1, W2 = Q1^T Q1                          last CTA: R2 = chol(W2)
-//   K3  Q = Q1 R2^-1, flip sums |O2 - Q|, |O2 + Q|          last CTA: signs D, multipliers m = +-D
-//   K4  Omega = Q m, Omega2 = Omega, operand copies, column sums  last CTA: sum of Omega
+//   tall_step  H = H1 + H2 (winSVD), Gram of H             last CTA: R1^-1
+//   tall_step  Q1 = H R1^-1, Gram of Q1                    last CTA: R2^-1
+//   k_flip     Q = Q1 R2^-1; per column sum |O - Q|, sum |O + Q|, sum Q, max |Q|; one extra
+//              CTA: Householder signs D of Q                last CTA: multipliers m = +-D, column
+//                                                           sums and maxima of Omega
+//   k_apply    Omega = Q m and its operand copies (FP32, int8 pieces or split BF16)
 //
-// Each kernel runs as clusters of kGramCluster CTAs that own fixed row ranges. A CTA stages
-// its rows in shared memory and sums them into a CTA partial (Gram matrices: 4 x 4 register
-// tiles of the upper triangle, thread groups over rows, gram.hpp); the cluster adds its CTAs'
-// partials through distributed shared memory, and the CTA that finishes last (atomic ticket
-// after a __threadfence) adds the cluster sums in cluster order, so the result is
-// deterministic. The Householder column signs D come from the modified LU of the top l x l
-// block of Q (Ballard et al. 2015): pivot s -> D = -sign(s), sign(0) = +. Row solves keep the
-// row in registers (kernels templated on LMAX >= l).
+// The maxima of k_flip are what the int8 pieces are scaled by, so k_apply writes them in the
+// same pass (a separate maximum and quantisation pass over Omega before). The signs come from
+// the modified LU of the top l x l block of Q (Ballard et al. 2015), which a CTA of its own
+// works on while the others solve their rows.
 #include <cuda_bf16.h>
 
 #include <algorithm>
 
-#include "gram.hpp"
-#include "internal.hpp"
 #include "linalg.hpp"
+#include "quant.hpp"
+#include "tall.hpp"
 #include "tc_layout.hpp"
 #include "update.hpp"
 
@@ -30,298 +29,224 @@ namespace pg {
 
 namespace {
 
-constexpr int kThreads = 256;
+template <int NT>
+struct FlipCfg {
+  static constexpr int kRows = kTallWarps * 4 * Tall<NT>::LT;                           // warps' sums
+  static constexpr int kSigns = Tall<NT>::kSq + Tall<NT>::LT + Tall<NT>::kWarpScratch;  // T, D, scratch
+  static constexpr size_t smem = ((size_t)Tall<NT>::kSq + 4 * Tall<NT>::LT + (kRows > kSigns ? kRows : kSigns)) * 8;
+};
 
-// rows staged per batch: a batch of rows, the group sums and R fit in about 100 KB, so two
-// CTAs (two clusters' worth per 8 SMs) fit on an SM
-__host__ __device__ constexpr int stage_rows(int l) { return l <= 48 ? 128 : 64; }
-
-// Column-strided pass over this CTA's rows: thread t owns column t % l of rows
-// r0 + t / l, r0 + t / l + T / l, ... with T = l * (blockDim / l) threads.
-__device__ __forceinline__ int col_threads(int l) { return l * (blockDim.x / l); }
-
-// Shared memory of the Gram kernels: [LMAX x LMAX R] | group sums | CTA sum | staged rows
-// (stage_rows(l) x l4, at least l x l).
-__host__ __device__ inline int upd_gram_smem_doubles(int l, int rmax) {
-  const GramTiling g = gram_tiling(l, l, true, kThreads);
-  const int l4 = (l + 3) & ~3;
-  return rmax * rmax + gram_smem_doubles(g) + std::max(stage_rows(l) * l4, l * l);
+// q = rows base .. base + 7 of Q1 R2^-1 (rows < r1): q[t][e] is row base + 2 r4 + e, column 8 t + q4.
+template <int NT>
+__device__ __forceinline__ void solve_rows(const double* Q1, const double* Rs, int64_t base, int64_t r1, int l,
+                                           double (&q)[NT][2]) {
+  const int lane = threadIdx.x & 31, q4 = lane >> 2, r4 = lane & 3;
+  double x[2 * NT];
+  const int64_t row = base + q4;
+#pragma unroll
+  for (int i = 0; i < 2 * NT; ++i) x[i] = row < r1 && 4 * i + r4 < l ? Q1[row * l + 4 * i + r4] : 0.0;
+#pragma unroll
+  for (int t = 0; t < NT; ++t) q[t][0] = q[t][1] = 0.0;
+#pragma unroll
+  for (int i = 0; i < 2 * NT; ++i)
+#pragma unroll
+    for (int t = i / 2; t < NT; ++t) dmma(q[t], Rs[(4 * i + r4) * Tall<NT>::LD + 8 * t + q4], x[i]);
 }
 
-__global__ void __cluster_dims__(kGramCluster, 1, 1) __launch_bounds__(kThreads) k_upd1(UpdateArgs a) {
-  extern __shared__ double sm[];
-  const int l = a.l;
-  const GramTiling g = gram_tiling(l, l, true, blockDim.x);
-  double* red = sm;
-  double* cpart = red + g.ngrp * g.ntiles * 16;
-  double* stage = cpart + g.ntiles * 16;
-  const int rows = stage_rows(l);
-  GramThread gt;
-  gt.init(g);
-  int64_t r0, r1;
-  row_range(a.N, r0, r1);
-  for (int64_t b = r0; b < r1; b += rows) {
-    const int nr = (int)(r1 - b < rows ? r1 - b : rows);
-    __syncthreads();
-#pragma unroll 4
-    for (int t = threadIdx.x; t < nr * g.la4; t += blockDim.x) {
-      const int r = t / g.la4, cc = t - r * g.la4;
-      double v = 0.0;
-      if (cc < l) {
-        const int64_t o = (b + r) * l + cc;
-        if (a.H2) {
-          v = a.H1[o] + a.H2[o];
-          a.H[o] = v;
-        } else {
-          v = a.H[o];
-        }
-      }
-      stage[t] = v;
-    }
-    __syncthreads();
-    gt.add_rows(stage, stage, nr, g);
-  }
-  gt.finish(g, red, cpart);
-  cluster_sum(cpart, g.ntiles * 16, a.part);
-  if (!last_cta(&a.counters[0])) return;
-  gram_final(g, a.part, gridDim.x / kGramCluster, l, l, stage);
-  const int bad = chol_upper_smem(stage, l);
-  if (bad && threadIdx.x == 0) atomicMax(a.status, bad);
-  for (int t = threadIdx.x; t < l * l; t += blockDim.x) a.R1[t] = stage[t];
-  if (threadIdx.x == 0) a.counters[0] = 0;
-}
-
-template <int LMAX>
-__global__ void __cluster_dims__(kGramCluster, 1, 1) __launch_bounds__(kThreads) k_upd2(UpdateArgs a) {
-  extern __shared__ double sm[];
-  const int l = a.l;
-  const GramTiling g = gram_tiling(l, l, true, blockDim.x);
-  double* R = sm;  // LMAX x LMAX (row stride LMAX)
-  double* red = R + LMAX * LMAX;
-  double* cpart = red + g.ngrp * g.ntiles * 16;
-  double* stage = cpart + g.ntiles * 16;
-  const int rows = stage_rows(l);
-  stage_r<LMAX>(a.R1, l, R);
-  {
-    GramThread gt;
-    gt.init(g);
-    gt.park(g, red);  // the tiles live in red between batches (registers go to the row solves)
-  }
-  int64_t r0, r1;
-  row_range(a.N, r0, r1);
-  for (int64_t b = r0; b < r1; b += rows) {
-    const int nr = (int)(r1 - b < rows ? r1 - b : rows);
-    __syncthreads();  // R staged; the previous batch's rows are consumed
-    for (int r = threadIdx.x; r < nr; r += blockDim.x)
-      solve_row_upper<LMAX>(a.H + (b + r) * l, R, l, stage + r * g.la4);
-    __syncthreads();
-#pragma unroll 4
-    for (int t = threadIdx.x; t < nr * g.la4; t += blockDim.x) {
-      const int r = t / g.la4, cc = t - r * g.la4;
-      if (cc < l)
-        a.Q[(b + r) * l + cc] = stage[t];
-      else
-        stage[t] = 0.0;
-    }
-    __syncthreads();
-    GramThread gt;
-    gt.init(g);
-    gt.unpark(g, red);
-    gt.add_rows(stage, stage, nr, g);
-    gt.park(g, red);
-  }
+// The flip sums are taken without the signs: A_c = sum |O - Q| and B_c = sum |O + Q| per
+// column; with D_c = +1 they are |O - Q D| and |O + Q D|, with D_c = -1 swapped (the same values
+// bit for bit). The sums and maxima of Q give those of Omega = +-Q. The last cluster holds the
+// CTA that finds the signs and takes no rows. Q goes to a buffer of its own (the signs' CTA
+// reads the rows of Q1 meanwhile).
+template <int NT>
+__global__ void __cluster_dims__(kTallCluster, 1, 1) __launch_bounds__(kTallThreads)
+    k_flip(UpdateArgs a, const double* __restrict__ Q1, double* __restrict__ Q) {
+  using T = Tall<NT>;
+  constexpr int LT = T::LT, LD = T::LD;
+  extern __shared__ __align__(16) double sm[];
+  double* Rs = sm;
+  double* cpart = Rs + T::kSq;  // LT each: A, B, sums, maxima
+  double* red = cpart + 4 * LT;
+  const int l = a.l, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, q4 = lane >> 2, r4 = lane & 3;
+  const int ctas = gridDim.x - kTallCluster;
+  load_square<NT>(a.R2i, l, 0.0, Rs);
+  for (int t = threadIdx.x; t < 4 * LT; t += kTallThreads) cpart[t] = 0.0;
   __syncthreads();
-  {
-    const int n = g.ntiles * 16;  // CTA sum of the groups' tiles, fixed group order
-    for (int e = threadIdx.x; e < n; e += blockDim.x) {
+  if ((int)blockIdx.x < ctas) {
+    int64_t r0, r1;
+    tall_rows(a.N, blockIdx.x, ctas, r0, r1);
+    double sa[NT], sb[NT], sq[NT], mx[NT];
+#pragma unroll
+    for (int t = 0; t < NT; ++t) sa[t] = sb[t] = sq[t] = mx[t] = 0.0;
+    for (int64_t base = r0 + 8 * warp; base < r1; base += 8 * kTallWarps) {
+      double q[NT][2], o[NT][2];
+#pragma unroll
+      for (int e = 0; e < 2; ++e)
+#pragma unroll
+        for (int t = 0; t < NT; ++t) {
+          const int64_t row = base + 2 * r4 + e;
+          o[t][e] = row < r1 && 8 * t + q4 < l ? a.Omg[row * l + 8 * t + q4] : 0.0;
+        }
+      solve_rows<NT>(Q1, Rs, base, r1, l, q);
+#pragma unroll
+      for (int e = 0; e < 2; ++e)
+#pragma unroll
+        for (int t = 0; t < NT; ++t) {
+          const int64_t row = base + 2 * r4 + e;
+          if (row < r1 && 8 * t + q4 < l) Q[row * l + 8 * t + q4] = q[t][e];
+          sa[t] += fabs(o[t][e] - q[t][e]);
+          sb[t] += fabs(o[t][e] + q[t][e]);
+          sq[t] += q[t][e];
+          mx[t] = fmax(mx[t], fabs(q[t][e]));
+        }
+    }
+#pragma unroll
+    for (int t = 0; t < NT; ++t) {
+#pragma unroll
+      for (int d = 1; d < 4; d <<= 1) {
+        sa[t] += __shfl_xor_sync(0xffffffffu, sa[t], d);
+        sb[t] += __shfl_xor_sync(0xffffffffu, sb[t], d);
+        sq[t] += __shfl_xor_sync(0xffffffffu, sq[t], d);
+        mx[t] = fmax(mx[t], __shfl_xor_sync(0xffffffffu, mx[t], d));
+      }
+      if (r4 == 0) {
+        double* w = red + warp * 4 * LT + 8 * t + q4;
+        w[0] = sa[t];
+        w[LT] = sb[t];
+        w[2 * LT] = sq[t];
+        w[3 * LT] = mx[t];
+      }
+    }
+    __syncthreads();
+    for (int e = threadIdx.x; e < 4 * LT; e += kTallThreads) {
       double s = 0.0;
-      for (int q = 0; q < g.ngrp; ++q) s += red[q * n + e];
+#pragma unroll
+      for (int w = 0; w < kTallWarps; ++w) s = e < 3 * LT ? s + red[w * 4 * LT + e] : fmax(s, red[w * 4 * LT + e]);
       cpart[e] = s;
     }
-    __syncthreads();
-  }
-  cluster_sum(cpart, g.ntiles * 16, a.part);
-  if (!last_cta(&a.counters[1])) return;
-  double* Rn = stage;  // W2, then R2 (row stride l)
-  gram_final(g, a.part, gridDim.x / kGramCluster, l, l, Rn);
-  const int bad = chol_upper_smem(Rn, l);
-  if (bad && threadIdx.x == 0) atomicMax(a.status, bad);
-  for (int t = threadIdx.x; t < l * l; t += blockDim.x) a.R2[t] = Rn[t];
-  if (threadIdx.x == 0) a.counters[1] = 0;
-}
-
-// K3. The flip sums are taken without the signs: A_c = sum |O2 - Q| and B_c = sum |O2 + Q|
-// per column; with D_c = +1 they are |O2 - Q D| and |O2 + Q D|, with D_c = -1 swapped (the
-// same values bit for bit). The last CTA reads the top l x l block of the final Q for D.
-template <int LMAX>
-__global__ void __cluster_dims__(kGramCluster, 1, 1) __launch_bounds__(kThreads) k_upd3(UpdateArgs a) {
-  extern __shared__ double sm[];
-  const int l = a.l;
-  const int rows = stage_rows(l);
-  double* R = sm;                      // LMAX x LMAX (row stride LMAX)
-  double* sq = R + LMAX * LMAX;        // rows x l: Q
-  double* so = sq + rows * l;          // rows x l: Omega2
-  double* red = so + rows * l;         // kThreads x 2
-  double* cpart = red + kThreads * 2;  // 2 l
-  stage_r<LMAX>(a.R2, l, R);
-  int64_t r0, r1;
-  row_range(a.N, r0, r1);
-  const int T = col_threads(l);
-  const int c = threadIdx.x % l;
-  double sa = 0.0, sb = 0.0;
-  for (int64_t b = r0; b < r1; b += rows) {
-    const int nr = (int)(r1 - b < rows ? r1 - b : rows);
-    __syncthreads();  // R staged; the previous batch is consumed
-    for (int r = threadIdx.x; r < nr; r += blockDim.x) solve_row_upper<LMAX>(a.Q + (b + r) * l, R, l, sq + r * l);
-#pragma unroll 4
-    for (int t = threadIdx.x; t < nr * l; t += blockDim.x) so[t] = a.Omg2[b * l + t];
-    __syncthreads();
-#pragma unroll 4
-    for (int t = threadIdx.x; t < nr * l; t += blockDim.x) a.Q[b * l + t] = sq[t];
-    if (threadIdx.x < T) {
-      for (int r = threadIdx.x / l; r < nr; r += T / l) {
-        const double o = so[r * l + c], q = sq[r * l + c];
-        sa += fabs(o - q);
-        sb += fabs(o + q);
-      }
+  } else if ((int)blockIdx.x == ctas) {
+    double *top = red, *D = top + T::kSq, *sc = D + LT;
+    if (warp < NT) {  // the top l rows of Q, 8 a warp, zero past row l
+      double q[NT][2];
+      solve_rows<NT>(Q1, Rs, 8 * warp, l, l, q);
+#pragma unroll
+      for (int e = 0; e < 2; ++e)
+#pragma unroll
+        for (int t = 0; t < NT; ++t) top[(8 * warp + 2 * r4 + e) * LD + 8 * t + q4] = q[t][e];
     }
+    householder_signs<NT>(top, D, sc);
+    for (int j = threadIdx.x; j < l; j += kTallThreads) a.D[j] = D[j];
   }
-  red[threadIdx.x * 2] = sa;
-  red[threadIdx.x * 2 + 1] = sb;
-  __syncthreads();
-  for (int j = threadIdx.x; j < l; j += blockDim.x) {  // fixed-order sum over this column's threads
-    double m = 0.0, p = 0.0;
-    for (int t = j; t < T; t += l) {
-      m += red[t * 2];
-      p += red[t * 2 + 1];
-    }
-    cpart[j] = m;
-    cpart[l + j] = p;
-  }
-  cluster_sum(cpart, 2 * l, a.part);
-  if (!last_cta(&a.counters[2])) return;
-  double* top = R;  // the top l x l block of Q, written by this kernel's CTAs
-  for (int t = threadIdx.x; t < l * l; t += blockDim.x) top[t] = a.Q[t];
-  householder_signs_smem(top, l, a.D);
-  const int ncl = gridDim.x / kGramCluster;
-  for (int j = threadIdx.x; j < l; j += blockDim.x) {
-    const double A = sum_all<kGramMaxParts>(a.part + j, ncl, 2 * l);
-    const double B = sum_all<kGramMaxParts>(a.part + l + j, ncl, 2 * l);
+  cluster_sum(cpart, 4 * LT, 3 * LT, a.part);
+  if (!last_cta(a.counter)) return;
+  const int ncl = gridDim.x / kTallCluster;
+  for (int j = threadIdx.x; j < l; j += kTallThreads) {
+    const double A = sum_parts(a.part + j, ncl, 4 * LT), B = sum_parts(a.part + LT + j, ncl, 4 * LT);
+    const double s = sum_parts(a.part + 2 * LT + j, ncl, 4 * LT);
+    double top = 0.0;
+    for (int p = 0; p < ncl; ++p) top = fmax(top, a.part[(int64_t)p * 4 * LT + 3 * LT + j]);
     const double d = a.D[j];
     const double m = d > 0.0 ? A : B, p = d > 0.0 ? B : A;
-    a.mult[j] = (m > 2.0 * p) ? -d : d;  // src/RSVD.hpp:85
+    const double f = (m > 2.0 * p) ? -d : d;  // src/RSVD.hpp:85
+    a.mult[j] = f;
+    a.wsum[j] = f * s;
+    if (a.i8.qmax) a.i8.qmax[j] = (unsigned long long)__double_as_longlong(top);
   }
-  if (threadIdx.x == 0) a.counters[2] = 0;
 }
 
-// K4. Writes in row-major order (coalesced), column sums from the staged batch.
-__global__ void __cluster_dims__(kGramCluster, 1, 1) __launch_bounds__(kThreads) k_upd4(UpdateArgs a) {
-  extern __shared__ double sm[];
-  const int l = a.l;
-  const int rows = stage_rows(l);
-  double* red = sm;                // kThreads
-  double* cpart = red + kThreads;  // l
-  double* st = cpart + l;          // rows x l
-  int64_t r0, r1;
-  row_range(a.N, r0, r1);
-  const int T = col_threads(l);
-  double cs = 0.0;
-  for (int64_t b = r0; b < r1; b += rows) {
-    const int nr = (int)(r1 - b < rows ? r1 - b : rows);
-    __syncthreads();  // the previous batch is summed
-#pragma unroll 4
-    for (int t = threadIdx.x; t < nr * l; t += blockDim.x) {
-      const int rr = t / l, j = t - rr * l;
-      const int64_t r = b + rr, o = b * l + t;
-      const double v = a.Q[o] * a.mult[j];
-      a.Omg[o] = v;
-      a.Omg2[o] = v;
-      st[t] = v;
-      if (a.Omgf) a.Omgf[o] = (float)v;
-      if (a.bt1) {
-        const int64_t kp = tc_pos(r);
-        const float x = (float)v;
-        const __nv_bfloat16 hi = __float2bfloat16_rn(x);
-        a.bt1[bt_elem(j, kp, 2 * a.bt_half)] = hi;
-        a.bt1[bt_elem(a.bt_half + j, kp, 2 * a.bt_half)] = __float2bfloat16_rn(x - __bfloat162float(hi));
-      }
-    }
-    __syncthreads();
-    if (threadIdx.x < T)
-      for (int rr = threadIdx.x / l; rr < nr; rr += T / l) cs += st[rr * l + threadIdx.x % l];
+// Omega = Q m over the 128 rows of a CTA (one K chunk of the int8 operand), coalesced.
+constexpr int kApplyThreads = 512;
+__global__ void __launch_bounds__(kApplyThreads) k_apply(UpdateArgs a, const double* __restrict__ Q) {
+  extern __shared__ __align__(16) uint8_t img[];  // np x 128 bytes (int8 operand)
+  __shared__ PieceTable tab;
+  __shared__ double mult[kLmax];
+  const int l = a.l, lp = i8_lp(l), np = i8_np(l);
+  const int64_t base = (int64_t)blockIdx.x * kI8Chunk;
+  const int rows = (int)(a.N - base < kI8Chunk ? (a.N > base ? a.N - base : 0) : kI8Chunk);
+  for (int j = threadIdx.x; j < l; j += kApplyThreads) mult[j] = a.mult[j];
+  if (a.i8.bq) {
+    tab.fill(a.i8.qmax, l, lp, a.i8.sig, blockIdx.x == 0);
+    for (int t = threadIdx.x; t < np * 8; t += kApplyThreads)
+      reinterpret_cast<uint4*>(img)[t] = make_uint4(0u, 0u, 0u, 0u);
   }
-  red[threadIdx.x] = cs;
   __syncthreads();
-  for (int j = threadIdx.x; j < l; j += blockDim.x) {
-    double s = 0.0;
-    for (int t = j; t < T; t += l) s += red[t];
-    cpart[j] = s;
+#pragma unroll 4
+  for (int t = threadIdx.x; t < rows * l; t += kApplyThreads) {
+    const int rr = t / l, j = t - rr * l;
+    const int64_t o = base * l + t;
+    const double v = Q[o] * mult[j];
+    a.Omg[o] = v;
+    if (a.Omgf) a.Omgf[o] = (float)v;
+    if (a.i8.bq) tab.put(img, rr, j, lp, v);
+    if (a.bt1) {
+      const int64_t kp = tc_pos(base + rr);
+      const float x = (float)v;
+      const __nv_bfloat16 hi = __float2bfloat16_rn(x);
+      a.bt1[bt_elem(j, kp, 2 * a.bt_half)] = hi;
+      a.bt1[bt_elem(a.bt_half + j, kp, 2 * a.bt_half)] = __float2bfloat16_rn(x - __bfloat162float(hi));
+    }
   }
-  cluster_sum(cpart, l, a.part);
-  if (!last_cta(&a.counters[3])) return;
-  const int ncl = gridDim.x / kGramCluster;
-  for (int j = threadIdx.x; j < l; j += blockDim.x) a.wsum[j] = sum_all<kGramMaxParts>(a.part + j, ncl, l);
-  if (threadIdx.x == 0) a.counters[3] = 0;
+  if (!a.i8.bq) return;
+  __syncthreads();
+  uint4* dst = reinterpret_cast<uint4*>(a.i8.bq + (int64_t)blockIdx.x * np * 128);
+  for (int t = threadIdx.x; t < np * 8; t += kApplyThreads) dst[t] = reinterpret_cast<const uint4*>(img)[t];
 }
 
-// CTAs of the update kernels: whole clusters, about 64 rows or more per CTA, at most
-// kMaxClusters clusters (two CTAs an SM; the last CTA reads one partial per cluster).
-constexpr int kMaxClusters = kGramMaxParts;
-
-int update_ctas(pcaone_ctx* c, int64_t N, int resident) {
-  const int64_t want = (N + kGramCluster * 64 - 1) / (kGramCluster * 64);
-  int cap = std::max(1, std::min(kMaxClusters, 2 * c->sm_count / kGramCluster));
+template <int NT>
+void launch_flip(pcaone_ctx* c, UpdateArgs a, const double* Q1, double* Q) {
+  constexpr size_t smem = FlipCfg<NT>::smem;
+  static_assert(smem <= 227 * 1024, "shared memory above the per-CTA limit");
+  const void* kern = (const void*)k_flip<NT>;
+  if (c->smem_attr_set.insert(kern).second)
+    PG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  int cap = kTallMaxParts;
+  const int resident = resident_clusters(c, kern, 0, kTallThreads, smem);
   if (resident > 0) cap = std::min(cap, resident);
-  return (int)std::max<int64_t>(1, std::min<int64_t>(cap, want)) * kGramCluster;
-}
-
-template <int LMAX>
-void launch_all(pcaone_ctx* c, const UpdateArgs& a) {
-  const int l = a.l, rows = stage_rows(l);
-  const size_t s1 = (size_t)upd_gram_smem_doubles(l, 0) * 8;
-  const size_t s2 = (size_t)upd_gram_smem_doubles(l, LMAX) * 8;
-  const size_t s3 = ((size_t)LMAX * LMAX + 2 * (size_t)rows * l + 2 * kThreads + 2 * l) * 8;
-  const size_t s4 = ((size_t)kThreads + l + (size_t)rows * l) * 8;
-  PG_CUDA(cudaFuncSetAttribute(k_upd1, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)s1));
-  PG_CUDA(cudaFuncSetAttribute(k_upd2<LMAX>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)s2));
-  PG_CUDA(cudaFuncSetAttribute(k_upd3<LMAX>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)s3));
-  // every cluster of every kernel resident at once: the tightest of the four bounds
-  int resident = 0;
-  const void* ks[4] = {(const void*)k_upd1, (const void*)k_upd2<LMAX>, (const void*)k_upd3<LMAX>, (const void*)k_upd4};
-  const size_t ss[4] = {s1, s2, s3, s4};
-  for (int i = 0; i < 4; ++i) {
-    const int n = resident_clusters(c, ks[i], (uint64_t)l, kThreads, ss[i]);
-    if (n > 0) resident = resident > 0 ? std::min(resident, n) : n;
-  }
-  const int nblk = update_ctas(c, a.N, resident);
-  k_upd1<<<nblk, kThreads, s1, c->stream>>>(a);
+  const int ncl = tall_clusters(a.N, cap - 1) + 1;  // one for the signs
+  a.part = tall_part(c, 4 * Tall<NT>::LT);
+  a.counter = tall_counter(c);
+  k_flip<NT><<<ncl * kTallCluster, kTallThreads, smem, c->stream>>>(a, Q1, Q);
   PG_CHECK_LAUNCH();
-  k_upd2<LMAX><<<nblk, kThreads, s2, c->stream>>>(a);
-  PG_CHECK_LAUNCH();
-  k_upd3<LMAX><<<nblk, kThreads, s3, c->stream>>>(a);
-  PG_CHECK_LAUNCH();
-  k_upd4<<<nblk, kThreads, s4, c->stream>>>(a);
-  PG_CHECK_LAUNCH();
+  c->launches++;
 }
 
 }  // namespace
 
-size_t update_part_doubles(int l) {
-  const GramTiling g = gram_tiling(l, l, true, kThreads);
-  return (size_t)kMaxClusters * std::max(g.ntiles * 16, 2 * l);
-}
-
 void fused_update(pcaone_ctx* c, UpdateArgs a) {
   PG_REQUIRE(a.l >= 1 && a.l <= kLmax, PCAONE_EBADARG, "sketch width out of range");
-  if (a.l <= 16)
-    launch_all<16>(c, a);
-  else if (a.l <= 32)
-    launch_all<32>(c, a);
-  else if (a.l <= 48)
-    launch_all<48>(c, a);
-  else
-    launch_all<64>(c, a);
-  c->launches += 4;
+  TallStep s;
+  s.n = a.N;
+  s.l = a.l;
+  s.status = a.status;
+  s.A = a.H2 ? a.H1 : a.H;
+  s.A2 = a.H2;
+  s.Asum = a.H2 ? a.H : nullptr;
+  s.Ri = a.R1i;
+  tall_step(c, s);
+  double* Q1 = (double*)scratch(c, "upd_Q1", (size_t)a.N * a.l * 8);
+  TallStep t;
+  t.n = a.N;
+  t.l = a.l;
+  t.status = a.status;
+  t.A = a.H;
+  t.Rinv = a.R1i;
+  t.Q = Q1;
+  t.Ri = a.R2i;
+  tall_step(c, t);
+  switch ((a.l + 7) / 8) {
+    case 1: launch_flip<1>(c, a, Q1, a.Q); break;
+    case 2: launch_flip<2>(c, a, Q1, a.Q); break;
+    case 3: launch_flip<3>(c, a, Q1, a.Q); break;
+    case 4: launch_flip<4>(c, a, Q1, a.Q); break;
+    case 5: launch_flip<5>(c, a, Q1, a.Q); break;
+    case 6: launch_flip<6>(c, a, Q1, a.Q); break;
+    case 7: launch_flip<7>(c, a, Q1, a.Q); break;
+    default: launch_flip<8>(c, a, Q1, a.Q); break;
+  }
+  const size_t img = a.i8.bq ? (size_t)i8_np(a.l) * 128 : 0;  // at most 24 KB
+  k_apply<<<(unsigned)(a.kpad / kI8Chunk), kApplyThreads, img, c->stream>>>(a, a.Q);
+  PG_CHECK_LAUNCH();
+  c->launches++;
 }
 
 }  // namespace pg

@@ -23,16 +23,15 @@
 namespace pg {
 
 namespace {
-// Omega column-major N x l (host layout of the reference) -> row-major Npad x l FP64 copies
+// Omega column-major N x l (host layout of the reference) -> row-major Npad x l FP64 copy
 // (padding rows zero) and an optional FP32 copy.
 __global__ void k_omega_layout(const double* __restrict__ cm, int64_t N, int l, int64_t npad, double* __restrict__ O,
-                               double* __restrict__ O2, float* __restrict__ Of) {
+                               float* __restrict__ Of) {
   const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (t >= npad * l) return;
   const int64_t i = t / l, j = t - i * l;
   const double v = i < N ? cm[j * N + i] : 0.0;
   O[t] = v;
-  O2[t] = v;
   if (Of) Of[t] = (float)v;
 }
 
@@ -125,7 +124,7 @@ struct Engine {
   int64_t M, Npad;
   GemmFnT<T> gemm;
 
-  double *Omg, *Omg2, *wsum, *G, *H, *H1, *H2, *Tb, *Rg, *Rb, *Dsig, *Ucur, *Upre, *Ck;
+  double *Omg, *wsum, *G, *H, *H1, *H2, *Tb, *Rg, *Rb, *Dsig, *Ucur, *Upre, *Ck;
   // epoch tail outputs kept apart from the epoch body's buffers (so the next body may run
   // while the host finishes the tail): Q of the sketch B^T and Q_B^T U_pre (l x k)
   double *Tq, *Xk;
@@ -134,7 +133,6 @@ struct Engine {
   double* Gbuf[2];
   T* OmgT;   // Omega as the B operand of the first product (alias of Omg for FP64)
   int* d_status;
-  unsigned* upd_cnt;
   const double* Fcent;  // centring frequencies of the epilogues (zeros for the dense E)
 
   Engine(pcaone_ctx* c_, const pcaone_rsvd_opts& o_, GemmFnT<T> g) : c(c_), o(o_), gemm(g) {
@@ -146,7 +144,6 @@ struct Engine {
     l = o.k + o.oversamples;
     auto d = [&](const char* name, size_t n) { return (double*)scratch(c, name, n * sizeof(double)); };
     Omg = d("r_omg", Npad * l);
-    Omg2 = d("r_omg2", Npad * l);
     wsum = d("r_wsum", l);
     Gbuf[0] = G = d("r_G", (size_t)c->Mpad * l);
     Gbuf[1] = d("r_G1", (size_t)c->Mpad * l);
@@ -164,8 +161,6 @@ struct Engine {
     Ck = d("r_Ck", (size_t)kLmax * kLmax);
     d_status = (int*)scratch(c, "r_status", sizeof(int));
     PG_CUDA(cudaMemsetAsync(d_status, 0, sizeof(int), c->stream));
-    upd_cnt = (unsigned*)scratch(c, "upd_cnt", 4 * sizeof(unsigned));
-    PG_CUDA(cudaMemsetAsync(upd_cnt, 0, 4 * sizeof(unsigned), c->stream));
     if (std::is_same<T, double>::value)
       OmgT = reinterpret_cast<T*>(Omg);
     else
@@ -180,7 +175,7 @@ struct Engine {
     double* d_cm = (double*)scratch(c, "r_omg_cm", cm.size() * 8);
     PG_CUDA(cudaMemcpyAsync(d_cm, cm.data(), cm.size() * 8, cudaMemcpyHostToDevice, c->stream));
     const int64_t tot = Npad * l;
-    k_omega_layout<<<(unsigned)((tot + 255) / 256), 256, 0, c->stream>>>(d_cm, N, l, Npad, Omg, Omg2, omg_float());
+    k_omega_layout<<<(unsigned)((tot + 255) / 256), 256, 0, c->stream>>>(d_cm, N, l, Npad, Omg, omg_float());
     PG_CHECK_LAUNCH();
     c->launches++;
     colsum(c, Omg, l, N, wsum);
@@ -196,7 +191,7 @@ struct Engine {
     double* d_cm = (double*)scratch(c, "r_omg_cm", cm.size() * 8);
     PG_CUDA(cudaMemcpyAsync(d_cm, cm.data(), cm.size() * 8, cudaMemcpyHostToDevice, c->stream));
     const int64_t tot = Npad * l;
-    k_omega_layout<<<(unsigned)((tot + 255) / 256), 256, 0, c->stream>>>(d_cm, N, l, Npad, Omg, Omg2, omg_float());
+    k_omega_layout<<<(unsigned)((tot + 255) / 256), 256, 0, c->stream>>>(d_cm, N, l, Npad, Omg, omg_float());
     PG_CHECK_LAUNCH();
     c->launches++;
     colsum(c, Omg, l, N, wsum);
@@ -220,8 +215,8 @@ struct Engine {
     }
   }
 
-  // Omega = flipOmg(Omega2, thinQ(Householder QR of H)); Omega2 = Omega. With H2, the sketch
-  // is H = H1 + H2 (written to H); otherwise H1 is the sketch itself.
+  // Omega = flipOmg(Omega, thinQ(Householder QR of H)). With H2, the sketch is H = H1 + H2
+  // (written to H); otherwise H1 is the sketch itself.
   void update_omega(double* H1in, const double* H2in) {
     UpdateArgs a;
     a.H1 = H2in ? H1in : nullptr;
@@ -229,22 +224,63 @@ struct Engine {
     a.H = H2in ? H : H1in;
     a.Q = Tb;
     a.Omg = Omg;
-    a.Omg2 = Omg2;
     a.Omgf = omg_float();
+    if (gemm.omega_i8) a.i8 = gemm.omega_i8(c, l);
     a.bt1 = gemm.omega_bt ? gemm.omega_bt(c, l, &a.bt_half) : nullptr;
     a.kpad = Npad;
     a.wsum = wsum;
-    a.part = (double*)scratch(c, "upd_part", update_part_doubles(l) * 8);
-    a.R1 = (double*)scratch(c, "upd_R1", (size_t)l * l * 8);
-    a.R2 = (double*)scratch(c, "upd_R2", (size_t)l * l * 8);
+    a.R1i = (double*)scratch(c, "upd_R1i", (size_t)l * l * 8);
+    a.R2i = (double*)scratch(c, "upd_R2i", (size_t)l * l * 8);
     a.D = Dsig;
     a.mult = (double*)scratch(c, "upd_mult", (size_t)l * 8);
-    a.counters = upd_cnt;
     a.status = d_status;
     a.N = N;
     a.l = l;
     fused_update(c, a);
-    if (!a.bt1) gemm.omega_changed(c, Omg, l, Npad);
+    if (!a.bt1 && !a.i8.bq) gemm.omega_changed(c, Omg, l, Npad);
+  }
+
+  // Tail of an epoch: CholeskyQR2 of G (its R_G alone; Q_G is formed for the output V only), then of
+  // B^T = H R_G^-1: Tq (orthonormal), R_B, and Xk = Tq^T U_pre. A pass over the rows each, the
+  // l x l factorisations in the passes' last CTAs (linalg.hpp). U_pre is zero in the first epoch.
+  void epoch_tail() {
+    const size_t sq = (size_t)l * l * 8;
+    auto m = [&](const char* name) { return (double*)scratch(c, name, sq); };
+    TallStep g1, g2, b1, b2, x;
+    g1.l = g2.l = b1.l = b2.l = x.l = l;
+    g1.n = g2.n = M;
+    b1.n = b2.n = x.n = N;
+    g1.status = g2.status = b1.status = b2.status = d_status;
+    g1.A = g2.A = G;
+    g1.R = m("tl_R1");
+    g1.Ri = m("tl_R1i");
+    tall_step(c, g1);
+    g2.Rinv = g2.Rprev_inv = g1.Ri;
+    g2.Rprev = g1.R;
+    g2.Racc = Rg;
+    g2.Racc_inv = m("tl_Rgi");
+    tall_step(c, g2);
+    double* T1 = (double*)scratch(c, "r_Tq1", (size_t)Npad * l * 8);
+    b1.A = H;
+    b1.Rinv = g2.Racc_inv;
+    b1.Q = T1;
+    b1.R = m("tl_R3");
+    b1.Ri = m("tl_R3i");
+    tall_step(c, b1);
+    b2.A = T1;
+    b2.Rinv = b1.Ri;
+    b2.Q = T1;
+    b2.Rprev = b1.R;
+    b2.Racc = Rb;
+    b2.Ri = m("tl_R4i");
+    tall_step(c, b2);
+    x.A = T1;
+    x.Rinv = b2.Ri;
+    x.Q = Tq;
+    x.B = Upre;
+    x.lb = k;
+    x.X = Xk;
+    tall_step(c, x);
   }
 
   // G rows of window b and accumulation of Z_b G_b into Ht.
@@ -663,10 +699,7 @@ struct Engine {
       ran_ahead = false;
       // tail of computeUSV: QR(G) twice, B = R^-T H^T, SVD(B); Q_B^T U_pre for the test
       timed([&] {
-        cholqr2_r(c, G, l, M, Rg, d_status);  // Q_G itself only for the output V
-        trsm_right_upper(c, H, Rg, l, N, Tq);
-        cholqr2(c, Tq, l, N, Tq, Rb, d_status);
-        if (pi > 0) cross(c, Tq, l, Upre, k, N, Xk);
+        epoch_tail();
       }, 3);
       gap_mark(true);
       const bool tc = o.precision == PCAONE_PREC_MIXED || o.precision == PCAONE_PREC_BF16;

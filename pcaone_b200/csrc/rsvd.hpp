@@ -4,6 +4,7 @@
 #include <cuda_bf16.h>
 
 #include "internal.hpp"
+#include "update.hpp"
 
 namespace pg {
 
@@ -28,6 +29,8 @@ struct GemmFnT {
   __nv_bfloat16* (*b2_bt)(pcaone_ctx* c, int l, int64_t* kpad, int* half) = nullptr;
   // Zeroed per-column maxima of |B2| for the first epilogue to fill (int8 back end), or null.
   unsigned long long* (*b2_qmax)(pcaone_ctx* c, int l) = nullptr;
+  // int8 operand buffers of Omega that the fused Omega update writes directly (int8 back end).
+  OmegaI8 (*omega_i8)(pcaone_ctx* c, int l) = nullptr;
   // Runs of consecutive windows [b0, b1) as one product each (null: one window at a time).
   // The first product writes seg_rows1 rows per window (SNP rows, zero padding rows); the
   // second reads B2 with seg_k2 rows per window (window SNPs first, zero rows after);

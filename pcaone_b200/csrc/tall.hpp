@@ -1,0 +1,363 @@
+// Building blocks of the FP64 kernels on tall row-major matrices (n rows, l <= 64 columns):
+// Gram products, products with a small upper factor, and the l x l factorisations that one CTA
+// does between them.
+//
+// All of it runs on the FP64 tensor-core shape m8n8k4 (36 TFLOP/s measured here from eight warps
+// an SM on, against 28-34 for FMA chains), chosen for its operand layout rather than its rate:
+// a warp's operand of 4 rows x 8 columns (lane: row lane % 4, column lane / 4) is the same
+// register for A^T and for A, so the Gram of 4 rows needs one 8-byte load a lane and column
+// tile, straight from global memory, and no shared memory. A product Q = X Rinv computed
+// transposed (Rinv^T X^T) leaves its 8 x 8 result in exactly that layout (rows 0, 2, 4, 6 in
+// the lane's first register, 1, 3, 5, 7 in the second), so Q feeds the Gram from registers.
+//
+// Reductions run in a fixed order (warps of the CTA, CTAs of the cluster through distributed
+// shared memory, clusters by the CTA that finishes last), so results are deterministic.
+#pragma once
+
+#include <cooperative_groups.h>
+
+#include "internal.hpp"
+
+namespace pg {
+
+namespace cg = cooperative_groups;
+
+constexpr int kTallThreads = 256;  // 8 warps; a warp takes 8 rows at a time
+constexpr int kTallWarps = kTallThreads / 32;
+constexpr int kTallCluster = 8;    // CTAs per cluster
+constexpr int kTallMaxParts = 36;  // clusters of a launch: the last CTA reads one sum of each
+
+// d (8x8) += a (8x4) b (4x8): lane holds a[lane/4][lane%4], b[lane%4][lane/4] and
+// d[lane/4][2 (lane%4) + {0, 1}].
+__device__ __forceinline__ void dmma(double (&d)[2], double a, double b) {
+  asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
+      : "+d"(d[0]), "+d"(d[1])
+      : "d"(a), "d"(b));
+}
+
+// NT column tiles of 8: padded width and the row stride of l x l matrices in shared memory (the
+// stride 4 mod 16 makes the 4 x 4 element reads of a half warp conflict-free).
+template <int NT>
+struct Tall {
+  static constexpr int LT = 8 * NT, LD = LT + 4;
+  static constexpr int kTiles = NT * (NT + 1) / 2;    // tiles on and above the diagonal
+  static constexpr int kSq = LT * LD;                 // doubles of an l x l matrix
+  static constexpr int kWarpScratch = kTallWarps * 128;  // two 8 x 8 blocks a warp
+  static __device__ __forceinline__ constexpr int tile(int i, int j) { return i * NT - i * (i - 1) / 2 + (j - i); }
+};
+
+// Rows per CTA when at most `ctas` CTAs split n rows: a multiple of 64, so that every warp takes
+// the same number of 8-row groups.
+__host__ __device__ __forceinline__ int64_t tall_rows_per_cta(int64_t n, int64_t ctas) {
+  return ((n + ctas - 1) / ctas + 63) & ~int64_t(63);
+}
+// Clusters for n rows, at most cap of them.
+inline int tall_clusters(int64_t n, int cap) {
+  const int64_t per = kTallCluster * tall_rows_per_cta(n, (int64_t)cap * kTallCluster);
+  return (int)((n + per - 1) / per);
+}
+// Row range of CTA `cta` of `ctas`.
+__device__ __forceinline__ void tall_rows(int64_t n, int64_t cta, int64_t ctas, int64_t& r0, int64_t& r1) {
+  const int64_t rpb = tall_rows_per_cta(n, ctas);
+  r0 = cta * rpb < n ? cta * rpb : n;
+  r1 = r0 + rpb < n ? r0 + rpb : n;
+}
+
+// Copy the l x l row-major matrix src into shared memory (row stride LD); `diag` on the padded
+// diagonal, zeros elsewhere.
+template <int NT>
+__device__ __forceinline__ void load_square(const double* src, int l, double diag, double* dst) {
+  for (int t = threadIdx.x; t < Tall<NT>::LT * Tall<NT>::LT; t += blockDim.x) {
+    const int i = t / Tall<NT>::LT, j = t - i * Tall<NT>::LT;
+    dst[i * Tall<NT>::LD + j] = (i < l && j < l) ? src[i * l + j] : (i == j ? diag : 0.0);
+  }
+}
+
+template <int NT>
+__device__ __forceinline__ void store_square(const double* src, int l, double* dst) {
+  for (int t = threadIdx.x; t < l * l; t += blockDim.x) dst[t] = src[(t / l) * Tall<NT>::LD + t % l];
+}
+
+// d += op(A) B for 8 x 8 blocks in shared memory (row strides lda, ldb); op(A) = A^T when TA.
+template <bool TA>
+__device__ __forceinline__ void block_mma(double (&d)[2], const double* A, int lda, const double* B, int ldb,
+                                          double sign = 1.0) {
+  const int q = (threadIdx.x & 31) >> 2, r = threadIdx.x & 3;
+#pragma unroll
+  for (int h = 0; h < 8; h += 4)
+    dmma(d, sign * (TA ? A[(h + r) * lda + q] : A[q * lda + h + r]), B[(h + r) * ldb + q]);
+}
+__device__ __forceinline__ void block_load(double (&d)[2], const double* C, int ldc) {
+  const int q = (threadIdx.x & 31) >> 2, r = threadIdx.x & 3;
+  const double2 v = *reinterpret_cast<const double2*>(C + q * ldc + 2 * r);
+  d[0] = v.x;
+  d[1] = v.y;
+}
+__device__ __forceinline__ void block_store(const double (&d)[2], double* C, int ldc) {
+  const int q = (threadIdx.x & 31) >> 2, r = threadIdx.x & 3;
+  *reinterpret_cast<double2*>(C + q * ldc + 2 * r) = make_double2(d[0], d[1]);
+}
+
+// Cholesky W = R^T R of the l x l matrix in shared memory (tiles on and above the diagonal read,
+// W overwritten; padded to LT with a unit diagonal) and X = R^-1, both upper with zeros below.
+// Blocks of 8: every warp factors and inverts the diagonal block itself (8 steps in registers:
+// lane r holds row r, columns by shuffle), so a block costs two CTA barriers, then the block
+// row and the trailing tiles are block products spread over the warps. A pivot that is not
+// positive and finite is replaced by 1. Returns 1 + the first such column, else 0 (the same in
+// every thread). sc: kWarpScratch doubles.
+template <int NT>
+__device__ __forceinline__ int chol_inverse(double* W, double* R, double* X, double* sc) {
+  using T = Tall<NT>;
+  constexpr int LD = T::LD;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, r8 = lane & 7;
+  double* my = sc + warp * 128;
+  int bad = 0;
+  for (int t = threadIdx.x; t < T::kSq; t += blockDim.x) R[t] = X[t] = 0.0;
+  __syncthreads();
+  for (int b = 0; b < NT; ++b) {
+    const double* Wb = W + 8 * b * LD + 8 * b;
+    // unit lower factor first (one reciprocal in a step's dependent chain), then the square roots
+    // of all eight pivots at once, one a lane
+    double d[8], own = 1.0;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) d[j] = Wb[r8 * LD + j];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      double p = __shfl_sync(0xffffffffu, d[j], j);
+      if (!(p > 0.0) || !isfinite(p)) {
+        if (!bad) bad = 8 * b + j + 1;
+        p = 1.0;
+      }
+      if (r8 == j) own = p;
+      const double f = d[j] * __drcp_rn(p);
+#pragma unroll
+      for (int c = j + 1; c < 8; ++c) d[c] -= f * __shfl_sync(0xffffffffu, d[j], c);
+      d[j] = r8 > j ? f : 0.0;
+    }
+    const double root = sqrt(own), iroot = 1.0 / root;
+    double y[8];  // lane c: column c of the inverse of the lower factor
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      double a = i == r8 ? 1.0 : 0.0;
+#pragma unroll
+      for (int m = 0; m < i; ++m) a -= __shfl_sync(0xffffffffu, d[m], i) * y[m];
+      y[i] = i >= r8 ? a : 0.0;
+    }
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      const double s = __shfl_sync(0xffffffffu, root, j);
+      d[j] = r8 == j ? s : d[j] * s;
+      y[j] *= __shfl_sync(0xffffffffu, iroot, j);
+    }
+    if (lane < 8) {
+#pragma unroll
+      for (int i = 0; i < 8; ++i) my[i * 8 + r8] = y[i];  // inverse of the lower factor
+      if (warp == 0) {
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          R[(8 * b + j) * LD + 8 * b + r8] = d[j];
+          X[(8 * b + r8) * LD + 8 * b + j] = y[j];
+        }
+      }
+    }
+    __syncwarp();
+    for (int J = b + 1 + warp; J < NT; J += kTallWarps) {  // block row of R
+      double c[2] = {0.0, 0.0};
+      block_mma<false>(c, my, 8, W + 8 * b * LD + 8 * J, LD);
+      block_store(c, R + 8 * b * LD + 8 * J, LD);
+    }
+    __syncthreads();
+    int t = 0;
+    for (int I = b + 1; I < NT; ++I)
+      for (int J = I; J < NT; ++J, ++t) {
+        if (t % kTallWarps != warp) continue;
+        double c[2];
+        block_load(c, W + 8 * I * LD + 8 * J, LD);
+        block_mma<true>(c, R + 8 * b * LD + 8 * I, LD, R + 8 * b * LD + 8 * J, LD, -1.0);
+        block_store(c, W + 8 * I * LD + 8 * J, LD);
+      }
+    __syncthreads();
+  }
+  // block column J of the inverse by warp J: X_IJ = -X_II sum_{I < K <= J} R_IK X_KJ
+  for (int J = warp; J < NT; J += kTallWarps)
+    for (int I = J - 1; I >= 0; --I) {
+      double c[2] = {0.0, 0.0};
+      for (int K = I + 1; K <= J; ++K) block_mma<false>(c, R + 8 * I * LD + 8 * K, LD, X + 8 * K * LD + 8 * J, LD);
+      block_store(c, my, 8);
+      __syncwarp();
+      double e[2] = {0.0, 0.0};
+      block_mma<false>(e, X + 8 * I * LD + 8 * I, LD, my, 8, -1.0);
+      block_store(e, X + 8 * I * LD + 8 * J, LD);
+      __syncwarp();
+    }
+  __syncthreads();
+  return bad;
+}
+
+// C = A B for upper triangular A, B in shared memory (C may not alias them).
+template <int NT>
+__device__ __forceinline__ void upper_product(const double* A, const double* B, double* C) {
+  constexpr int LD = Tall<NT>::LD;
+  const int warp = threadIdx.x >> 5;
+  __syncthreads();
+  for (int t = warp; t < NT * NT; t += kTallWarps) {
+    const int I = t / NT, J = t - I * NT;
+    double c[2] = {0.0, 0.0};
+    for (int K = I; K <= J; ++K) block_mma<false>(c, A + 8 * I * LD + 8 * K, LD, B + 8 * K * LD + 8 * J, LD);
+    block_store(c, C + 8 * I * LD + 8 * J, LD);
+  }
+  __syncthreads();
+}
+
+// Householder column signs D (LT values, shared memory) of the thin QR whose orthonormal factor
+// has the top l x l block T (shared memory, zero padded, overwritten): modified LU, step i takes
+// the pivot s = T[i][i], D_i = -sign(s) with sign(0) = +, and eliminates with the shifted pivot
+// s - D_i (Ballard et al. 2015). Blocks of 8 as in chol_inverse: the diagonal block and the
+// inverses of its two factors in the registers of every warp, the rest as block products.
+template <int NT>
+__device__ __forceinline__ void householder_signs(double* T, double* D, double* sc) {
+  constexpr int LD = Tall<NT>::LD;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, r8 = lane & 7;
+  double *mL = sc + warp * 128, *mU = mL + 64;
+  __syncthreads();
+  for (int b = 0; b < NT; ++b) {
+    double t[8], ui[8];
+    {
+      const double* Tb = T + 8 * b * LD + 8 * b;
+#pragma unroll
+      for (int j = 0; j < 8; ++j) t[j] = Tb[r8 * LD + j];
+    }
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      const double piv = __shfl_sync(0xffffffffu, t[j], j);
+      const double di = piv >= 0.0 ? -1.0 : 1.0;
+      if (threadIdx.x == 0) D[8 * b + j] = di;
+      ui[j] = __drcp_rn(piv - di);
+      const double f = r8 > j ? t[j] * ui[j] : 0.0;
+#pragma unroll
+      for (int c = j + 1; c < 8; ++c) t[c] -= f * __shfl_sync(0xffffffffu, t[c], j);
+      if (r8 > j) t[j] = f;
+    }
+    double y[8], z[8];  // lane c: column c of L^-1 (unit lower) and of U^-1
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      double a = i == r8 ? 1.0 : 0.0;
+#pragma unroll
+      for (int m = 0; m < i; ++m) a -= __shfl_sync(0xffffffffu, t[m], i) * y[m];
+      y[i] = i >= r8 ? a : 0.0;
+    }
+#pragma unroll
+    for (int i = 7; i >= 0; --i) {
+      double a = i == r8 ? 1.0 : 0.0;
+#pragma unroll
+      for (int m = i + 1; m < 8; ++m) a -= __shfl_sync(0xffffffffu, t[m], i) * z[m];
+      z[i] = i <= r8 ? a * ui[i] : 0.0;
+    }
+    if (lane < 8) {
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        mL[i * 8 + r8] = y[i];
+        mU[i * 8 + r8] = z[i];
+      }
+    }
+    __syncwarp();
+    const int rest = NT - 1 - b;
+    for (int q = warp; q < 2 * rest; q += kTallWarps) {  // block row, then block column
+      const bool row = q < rest;
+      double* P = row ? T + 8 * b * LD + 8 * (b + 1 + q) : T + 8 * (b + 1 + q - rest) * LD + 8 * b;
+      double c[2] = {0.0, 0.0};
+      if (row)
+        block_mma<false>(c, mL, 8, P, LD);
+      else
+        block_mma<false>(c, P, LD, mU, 8);
+      __syncwarp();
+      block_store(c, P, LD);
+    }
+    __syncthreads();
+    for (int q = warp; q < rest * rest; q += kTallWarps) {
+      const int I = b + 1 + q / rest, J = b + 1 + q % rest;
+      double c[2];
+      block_load(c, T + 8 * I * LD + 8 * J, LD);
+      block_mma<false>(c, T + 8 * I * LD + 8 * b, LD, T + 8 * b * LD + 8 * J, LD, -1.0);
+      block_store(c, T + 8 * I * LD + 8 * J, LD);
+    }
+    __syncthreads();
+  }
+}
+
+// sum_{b < n} x[b * stride] in b order with every load issued before the adds (n <= kTallMaxParts).
+__device__ __forceinline__ double sum_parts(const double* x, int n, int64_t stride) {
+  double v[kTallMaxParts];
+#pragma unroll
+  for (int k = 0; k < kTallMaxParts; ++k) v[k] = k < n ? x[(int64_t)k * stride] : 0.0;
+  double s = 0.0;
+#pragma unroll
+  for (int k = 0; k < kTallMaxParts; ++k)
+    if (k < n) s += v[k];
+  return s;
+}
+
+// Cluster sum of the CTAs' part[n] (shared memory), in rank order, written to
+// gout[cluster index * n + e]. Every CTA of the cluster calls it; the rank-r CTA sums the
+// elements r * blockDim + t, ... through distributed shared memory. The second cluster barrier
+// keeps each CTA's shared memory alive until the others have read it. The elements from nsum on
+// are maxima (of non-negative values) instead of sums.
+__device__ __forceinline__ void cluster_sum(const double* part, int n, int nsum, double* gout) {
+  cg::cluster_group cl = cg::this_cluster();
+  cl.sync();
+  const int rank = (int)cl.block_rank();
+  const int64_t cid = blockIdx.x / kTallCluster;
+  for (int e = rank * blockDim.x + threadIdx.x; e < n; e += kTallCluster * blockDim.x) {
+    double v[kTallCluster];
+#pragma unroll
+    for (int q = 0; q < kTallCluster; ++q) v[q] = cl.map_shared_rank(part, q)[e];
+    double s = 0.0;
+#pragma unroll
+    for (int q = 0; q < kTallCluster; ++q) s = e < nsum ? s + v[q] : fmax(s, v[q]);
+    gout[cid * n + e] = s;
+  }
+  cl.sync();
+}
+
+// Ticket: true in the CTA that finishes last (after a fence, so it sees every CTA's writes).
+__device__ __forceinline__ bool last_cta(unsigned* counter) {
+  __shared__ bool last;
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    const unsigned t = atomicAdd(counter, 1u);
+    last = (t == gridDim.x - 1);
+    if (last) *counter = 0;  // ready for the next launch
+  }
+  __syncthreads();
+  if (last) __threadfence();
+  return last;
+}
+
+// Clusters of kTallCluster CTAs of kernel (threads, smem bytes) that fit on the device at
+// once, cached in the context by (kernel, key); 0 when the runtime cannot tell.
+inline int resident_clusters(pcaone_ctx* c, const void* kernel, uint64_t key, int threads, size_t smem) {
+  const auto k = std::make_pair(kernel, key);
+  auto it = c->cluster_occupancy.find(k);
+  if (it != c->cluster_occupancy.end()) return it->second;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(kTallCluster * 64);
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeClusterDimension;
+  attr.val.clusterDim.x = kTallCluster;
+  attr.val.clusterDim.y = 1;
+  attr.val.clusterDim.z = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  int n = 0;
+  if (cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess) {
+    (void)cudaGetLastError();
+    n = 0;
+  }
+  c->cluster_occupancy[k] = n;
+  return n;
+}
+
+}  // namespace pg

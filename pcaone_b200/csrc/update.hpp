@@ -7,31 +7,37 @@
 
 namespace pg {
 
+// The int8 back end's operand copy of Omega (kernels_gemm_i8.cu): column maxima (bits of
+// doubles), the chunked pieces (kpad / 128 chunk images) and their scales.
+struct OmegaI8 {
+  unsigned long long* qmax = nullptr;
+  int8_t* bq = nullptr;
+  float* sig = nullptr;
+};
+
 struct UpdateArgs {
-  const double* H1 = nullptr;  // winSVD: H = H1 + H2; Halko: H1 = nullptr, H2 = nullptr
+  double* H1 = nullptr;        // the sketch is H1 + H2 (written to H) when H2 is given, else H
   const double* H2 = nullptr;
-  double* H = nullptr;         // N x l: written when H2 is given, else the input sketch
+  double* H = nullptr;
   double* Q = nullptr;         // N x l work (Q1 then Q)
-  double* Omg = nullptr;       // N x l outputs
-  double* Omg2 = nullptr;
+  double* Omg = nullptr;       // N x l: the previous Omega in, the new one out
   float* Omgf = nullptr;       // FP32 operand copy (SIMT path) or null
+  OmegaI8 i8;                  // int8 operand (bq null: none)
   __nv_bfloat16* bt1 = nullptr;  // split-BF16 operand (tc_layout.hpp) or null
-  int64_t kpad = 0;
   int bt_half = 0;               // row offset of the lo half in bt1 (= NP / 2)
-  double* wsum = nullptr;      // l
-  double* part = nullptr;      // update_part_doubles(l) work
-  double* R1 = nullptr;        // l x l work
-  double* R2 = nullptr;
+  int64_t kpad = 0;            // padded rows of the operand copies (a multiple of 128)
+  double* wsum = nullptr;      // l column sums of the new Omega
   double* D = nullptr;         // l
   double* mult = nullptr;      // l
-  unsigned* counters = nullptr;  // 4 tickets, zero between calls
+  double *R1i = nullptr, *R2i = nullptr;  // l x l work
   int* status = nullptr;
   int64_t N = 0;
   int l = 0;
+  // set by fused_update
+  double* part = nullptr;
+  unsigned* counter = nullptr;
 };
 
-// doubles of UpdateArgs::part for sketch width l
-size_t update_part_doubles(int l);
 void fused_update(pcaone_ctx* c, UpdateArgs a);
 
 }  // namespace pg
