@@ -23,6 +23,7 @@
 
 #include "internal.hpp"
 #include "rsvd.hpp"
+#include "tall.hpp"
 
 namespace pg {
 
@@ -438,56 +439,76 @@ void dense_none_b2(pcaone_ctx*, const float*, int, int64_t) {}
 // i over the slice's sites of the chunk, in site order; e is written to E[(j - j0) * lde + i]
 // and the slice's diagonal sum is added to dpart[slice * N + i] (each entry has one owner and
 // the chunks run in stream order, so the sums are deterministic). US: N x k (U diag S) and
-// V: M x k row-major as in k_posterior_e; V null: pt = F_j.
+// V: M x k row-major as in k_posterior_e; V null: pt = F_j. KM >= k.
+// Bound by HBM (16 B read, 8 B written per sample-site). The values that depend on the site
+// alone (two divisions and a square root, and the loading row) are worked out once per CTA
+// into shared memory, kGrmSites sites at a time, and the sample's row of US stays in registers;
+// each sample-site is left with one division. N = 1501, M = 40000: 558 us = 2.6 TB/s (1245 with the
+// factors read per site from global memory and six divisions).
+constexpr int kGrmSites = 64;
+template <int KM>
 __global__ void __launch_bounds__(128) k_grm_e(const double* __restrict__ P, uint32_t N, uint32_t ldp,
                                                const double* __restrict__ F, const double* __restrict__ US,
                                                const double* __restrict__ V, int k, uint64_t j0, uint64_t mc,
                                                double* __restrict__ E, uint32_t lde, double* __restrict__ dpart) {
+  __shared__ double sf[kGrmSites], snorm[kGrmSites], sden[kGrmSites], sv[kGrmSites * KM];
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= N) return;
   const uint64_t per = (mc + gridDim.y - 1) / gridDim.y;
   const uint64_t a = (uint64_t)blockIdx.y * per, b = (a + per < mc ? a + per : mc);
+  double us[KM];
+#pragma unroll
+  for (int t = 0; t < KM; ++t) us[t] = (V && i < N && t < k) ? US[(uint64_t)i * k + t] : 0.0;
   double dc = 0.0;
-  for (uint64_t jl = a; jl < b; ++jl) {
-    const uint64_t j = j0 + jl;
-    const double f = F[j];
-    double pt = f;
-    if (V) {
-      double pred = 0.0;
-      for (int t = 0; t < k; ++t) pred += US[(uint64_t)i * k + t] * V[j * k + t];
-      pt = fmin(fmax((pred + 2.0 * f) / 2.0, 1e-4), 1.0 - 1e-4);
+  for (uint64_t s0 = a; s0 < b; s0 += kGrmSites) {
+    const int ns = (int)(b - s0 < kGrmSites ? b - s0 : kGrmSites);
+    __syncthreads();  // the previous sites are used up
+    for (int t = threadIdx.x; t < ns; t += blockDim.x) {
+      const double f = F[j0 + s0 + t], h = 2.0 * f * (1.0 - f), norm = sqrt(h);
+      sf[t] = f;
+      snorm[t] = norm > 1e-9 ? 1.0 / norm : 1.0;
+      sden[t] = 1.0 / h;
     }
-    const double2 pp = *reinterpret_cast<const double2*>(P + j * ldp + 2 * i);
-    double p0, p1, p2;
-    posterior(pp.x, pp.y, pt, p0, p1, p2);
-    const double sum = p0 + p1 + p2;
-    double e = (p1 + 2.0 * p2) / sum - 2.0 * f;
-    const double norm = sqrt(2.0 * f * (1.0 - f));
-    if (norm > 1e-9) e /= norm;
-    const double f2 = 2.0 * f;
-    double t = (0.0 - f2) * (0.0 - f2) * (p0 / sum);
-    t += (1.0 - f2) * (1.0 - f2) * (p1 / sum);
-    t += (2.0 - f2) * (2.0 - f2) * (p2 / sum);
-    dc += t / (2.0 * f * (1.0 - f));
-    E[jl * lde + i] = e;
+    if (V)
+      for (int t = threadIdx.x; t < ns * KM; t += blockDim.x)
+        sv[t] = t % KM < k ? V[(j0 + s0 + t / KM) * k + t % KM] : 0.0;
+    __syncthreads();
+    if (i >= N) continue;
+#pragma unroll 4
+    for (int q = 0; q < ns; ++q) {
+      const double2 pp = __ldcs(reinterpret_cast<const double2*>(P + (j0 + s0 + q) * ldp) + i);
+      const double f = sf[q], f2 = 2.0 * f;
+      double pt = f;
+      if (V) {
+        double pred = 0.0;
+#pragma unroll
+        for (int t = 0; t < KM; ++t) pred += us[t] * sv[q * KM + t];
+        pt = fmin(fmax((pred + f2) / 2.0, 1e-4), 1.0 - 1e-4);
+      }
+      double p0, p1, p2;
+      posterior(pp.x, pp.y, pt, p0, p1, p2);
+      const double inv = 1.0 / (p0 + p1 + p2);
+      E[(s0 + q) * lde + i] = ((p1 + 2.0 * p2) * inv - f2) * snorm[q];
+      const double t = (f2 * f2 * p0 + (1.0 - f2) * (1.0 - f2) * p1 + (2.0 - f2) * (2.0 - f2) * p2) * inv;
+      dc += t * sden[q];
+    }
   }
-  dpart[(uint64_t)blockIdx.y * N + i] += dc;
+  if (i < N) dpart[(uint64_t)blockIdx.y * N + i] += dc;
 }
 
-// C (N x N, column-major, full) = the lower triangle of L (E E^T from the SYRK) mirrored,
-// divided by M, with the diagonal replaced by Dc / M, Dc_i = sum over slices of dpart in
-// slice order (src/Halko.cpp:322-324).
-__global__ void k_grm_finish(const double* __restrict__ L, const double* __restrict__ dpart, int nsl, uint32_t N,
-                             double M, double* __restrict__ C) {
+// C (N x N, column-major, full) = the lower triangle of L (E E^T from the SYRK: the sum of its
+// nsplit partial matrices, in split order) mirrored, divided by M, with the diagonal replaced by
+// Dc / M, Dc_i = sum over slices of dpart in slice order (src/Halko.cpp:322-324).
+__global__ void k_grm_finish(const double* __restrict__ L, int nsplit, const double* __restrict__ dpart, int nsl,
+                             uint32_t N, double M, double* __restrict__ C) {
   const uint64_t n2 = (uint64_t)N * N;
   for (uint64_t t = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; t < n2; t += (uint64_t)gridDim.x * blockDim.x) {
     const uint32_t j = (uint32_t)(t / N), i = (uint32_t)(t - (uint64_t)j * N);
-    double v;
+    double v = 0.0;
     if (i == j) {
-      v = 0.0;
       for (int sl = 0; sl < nsl; ++sl) v += dpart[(uint64_t)sl * N + i];
     } else {
-      v = i > j ? L[t] : L[(uint64_t)i * N + j];
+      const double* src = L + (i > j ? t : (uint64_t)i * N + j);
+      for (int sp = 0; sp < nsplit; ++sp) v += src[(uint64_t)sp * n2];
     }
     C[t] = v / M;
   }
@@ -496,13 +517,19 @@ __global__ void k_grm_finish(const double* __restrict__ L, const double* __restr
 // Lower-triangular tiles of L = E E^T (N x N, column-major, ld N) over the sites of one
 // chunk of the standardised posterior matrix (E: site-major, column j = site j, ld lde): the
 // O(N^2 M) product of the GRM (src/Halko.cpp:320, G G^T). One CTA per 128 x 128 tile (I, J)
-// with I >= J, 256 threads, each owning an 8 x 8 block (rows 4 ty + {0..3} and 64 + 4 ty +
-// {0..3}, columns likewise from tx) accumulated in FP64 registers, site by site in order, so
-// the result is deterministic. The two 128-row panels of 16 sites stream through a
-// three-stage ring of 16-byte asynchronous copies (zero-filled past N and past the chunk).
-// accumulate: add to L (later chunks) instead of overwriting it.
-constexpr int kSyrkT = 128, kSyrkKC = 16, kSyrkStages = 3;
-constexpr size_t kSyrkSmem = (size_t)kSyrkStages * 2 * kSyrkKC * kSyrkT * sizeof(double);
+// with I >= J and range of sites (blockIdx.y of gridDim.y, each with a partial matrix of its
+// own), 8 warps of 64 x 32 outputs as m8n8k4 FP64 tensor tiles: an operand register is one
+// element E[site][sample], the same layout for both sides, and a warp's step of 4 sites is 12
+// shared-memory loads for 32 products. Sites are summed in order, so the result is
+// deterministic. The two 128-row panels of 16 sites stream through a four-stage ring of 16-byte
+// asynchronous copies (zero-filled past N and past the chunk); rows are 132 doubles apart, which
+// makes the 4 x 4 element reads of a half warp conflict-free. accumulate: add to L (later
+// chunks) instead of overwriting it.
+// Bound by the FP64 pipe (36 TFLOP/s). The splits fill the SMs when there are few tiles (78 at
+// N = 1501, on 148 SMs): N = 1501, M = 40000, 7 ranges: 3.47 ms (8.80 with 8 x 8 FMA blocks a thread
+// and one CTA a tile), 29 TFLOP/s.
+constexpr int kSyrkT = 128, kSyrkKC = 16, kSyrkStages = 4, kSyrkLd = kSyrkT + 4;
+constexpr size_t kSyrkSmem = (size_t)kSyrkStages * 2 * kSyrkKC * kSyrkLd * sizeof(double);
 
 __device__ __forceinline__ void cp_async16_zfill(double* sdst, const double* gsrc, int bytes) {
   const uint32_t d = (uint32_t)__cvta_generic_to_shared(sdst);
@@ -512,35 +539,38 @@ __device__ __forceinline__ void cp_async16_zfill(double* sdst, const double* gsr
 __global__ void __launch_bounds__(256, 1) k_syrk_lower(const double* __restrict__ E, uint32_t lde, uint32_t N,
                                                        uint64_t mc, double* __restrict__ L, int accumulate) {
   extern __shared__ __align__(16) double smem_syrk[];
-  const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, q4 = lane >> 2, r4 = lane & 3;
+  const int wr = (warp >> 2) * 64, wc = (warp & 3) * 32;
   const uint32_t t = blockIdx.x;
   uint32_t I = (uint32_t)((sqrt(8.0 * t + 1.0) - 1.0) * 0.5);
   while ((I + 1) * (I + 2) / 2 <= t) ++I;
   while (I * (I + 1) / 2 > t) --I;
   const uint32_t J = t - I * (I + 1) / 2;
   const uint32_t r0 = I * kSyrkT, c0 = J * kSyrkT;
-  const int64_t nk = (int64_t)((mc + kSyrkKC - 1) / kSyrkKC);
+  const int64_t nkt = (int64_t)((mc + kSyrkKC - 1) / kSyrkKC);
+  const int64_t k0 = nkt * blockIdx.y / gridDim.y, nk = nkt * (blockIdx.y + 1) / gridDim.y - k0;
+  constexpr int kPanel = kSyrkKC * kSyrkLd;
   auto issue = [&](int64_t kc, int stage) {
-    double* a = smem_syrk + (size_t)stage * 2 * kSyrkKC * kSyrkT;
-    double* b = a + kSyrkKC * kSyrkT;
+    double* a = smem_syrk + (size_t)stage * 2 * kPanel;
+    double* b = a + kPanel;
 #pragma unroll
     for (int u = 0; u < 4; ++u) {
       const int e = tid + 256 * u;  // 1024 16-byte pieces per panel: site kk, rows p, p + 1
       const int kk = e >> 6, p = (e & 63) * 2;
-      const uint64_t site = (uint64_t)kc * kSyrkKC + kk;
+      const uint64_t site = (uint64_t)(k0 + kc) * kSyrkKC + kk;
       const bool in = site < mc;
       const uint32_t ra = r0 + p, rb = c0 + p;
       const int ba = in && ra < N ? (int)min(16u, (N - ra) * 8u) : 0;
       const int bb = in && rb < N ? (int)min(16u, (N - rb) * 8u) : 0;
-      cp_async16_zfill(a + kk * kSyrkT + p, ba ? E + site * lde + ra : E, ba);
-      cp_async16_zfill(b + kk * kSyrkT + p, bb ? E + site * lde + rb : E, bb);
+      cp_async16_zfill(a + kk * kSyrkLd + p, ba ? E + site * lde + ra : E, ba);
+      cp_async16_zfill(b + kk * kSyrkLd + p, bb ? E + site * lde + rb : E, bb);
     }
   };
-  double acc[8][8];
+  double acc[8][4][2];
 #pragma unroll
-  for (int q = 0; q < 8; ++q)
+  for (int i = 0; i < 8; ++i)
 #pragma unroll
-    for (int c = 0; c < 8; ++c) acc[q][c] = 0.0;
+    for (int j = 0; j < 4; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
 #pragma unroll
   for (int st = 0; st < kSyrkStages - 1; ++st) {
     if (st < nk) issue(st, st);
@@ -551,38 +581,54 @@ __global__ void __launch_bounds__(256, 1) k_syrk_lower(const double* __restrict_
     __syncthreads();  // stage kc landed for every thread; stage kc - 1 is no longer read
     if (kc + kSyrkStages - 1 < nk) issue(kc + kSyrkStages - 1, (int)((kc + kSyrkStages - 1) % kSyrkStages));
     asm volatile("cp.async.commit_group;\n" ::: "memory");
-    const double* a = smem_syrk + (size_t)(kc % kSyrkStages) * 2 * kSyrkKC * kSyrkT;
-    const double* b = a + kSyrkKC * kSyrkT;
-#pragma unroll 4
-    for (int kk = 0; kk < kSyrkKC; ++kk) {
-      double av[8], bv[8];
-      const double2* ap = reinterpret_cast<const double2*>(a + kk * kSyrkT);
-      const double2* bp = reinterpret_cast<const double2*>(b + kk * kSyrkT);
-      const double2 a0 = ap[2 * ty], a1 = ap[2 * ty + 1], a2 = ap[32 + 2 * ty], a3 = ap[33 + 2 * ty];
-      const double2 b0 = bp[2 * tx], b1 = bp[2 * tx + 1], b2 = bp[32 + 2 * tx], b3 = bp[33 + 2 * tx];
-      av[0] = a0.x; av[1] = a0.y; av[2] = a1.x; av[3] = a1.y;
-      av[4] = a2.x; av[5] = a2.y; av[6] = a3.x; av[7] = a3.y;
-      bv[0] = b0.x; bv[1] = b0.y; bv[2] = b1.x; bv[3] = b1.y;
-      bv[4] = b2.x; bv[5] = b2.y; bv[6] = b3.x; bv[7] = b3.y;
+    const double* a = smem_syrk + (size_t)(kc % kSyrkStages) * 2 * kPanel + r4 * kSyrkLd + wr + q4;
+    const double* b = smem_syrk + (size_t)(kc % kSyrkStages) * 2 * kPanel + kPanel + r4 * kSyrkLd + wc + q4;
 #pragma unroll
-      for (int q = 0; q < 8; ++q)
+    for (int kk = 0; kk < kSyrkKC; kk += 4) {
+      double av[8], bv[4];
 #pragma unroll
-        for (int c = 0; c < 8; ++c) acc[q][c] = fma(av[q], bv[c], acc[q][c]);
+      for (int i = 0; i < 8; ++i) av[i] = a[kk * kSyrkLd + 8 * i];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) bv[j] = b[kk * kSyrkLd + 8 * j];
+#pragma unroll
+      for (int i = 0; i < 8; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) dmma(acc[i][j], av[i], bv[j]);
     }
   }
   asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+  double* Lp = L + (uint64_t)blockIdx.y * N * N;
 #pragma unroll
-  for (int c = 0; c < 8; ++c) {
-    const uint32_t col = c0 + (c < 4 ? 4 * tx + c : 64 + 4 * tx + c - 4);
-    if (col >= N) continue;
+  for (int j = 0; j < 4; ++j)
 #pragma unroll
-    for (int q = 0; q < 8; ++q) {
-      const uint32_t row = r0 + (q < 4 ? 4 * ty + q : 64 + 4 * ty + q - 4);
-      if (row >= N) continue;
-      double* dst = L + (uint64_t)col * N + row;
-      *dst = accumulate ? *dst + acc[q][c] : acc[q][c];
+    for (int e = 0; e < 2; ++e) {
+      const uint32_t col = c0 + wc + 8 * j + 2 * r4 + e;
+      if (col >= N) continue;
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        const uint32_t row = r0 + wr + 8 * i + q4;
+        if (row >= N) continue;
+        double* dst = Lp + (uint64_t)col * N + row;
+        *dst = accumulate ? *dst + acc[i][j][e] : acc[i][j][e];
+      }
+    }
+}
+
+// Site ranges of the SYRK: the count (at most 8) whose CTAs, one an SM, waste the least of their
+// last wave, while every range keeps 16 panels of sites and the partial matrices stay in 1 GiB.
+int syrk_splits(const pcaone_ctx* c, uint32_t ntile, uint64_t sites) {
+  const uint64_t tiles = (uint64_t)ntile * (ntile + 1) / 2, sms = (uint64_t)c->sm_count, n2 = (uint64_t)c->N * c->N * 8;
+  int best = 1;
+  double best_cost = 0.0;
+  for (int s = 1; s <= 8; ++s) {
+    if (s > 1 && (sites / kSyrkKC < 16ull * s || n2 * s > (1ull << 30))) break;
+    const double cost = (double)((tiles * s + sms - 1) / sms) / s;
+    if (s == 1 || cost < best_cost) {
+      best = s;
+      best_cost = cost;
     }
   }
+  return best;
 }
 
 }  // namespace
@@ -698,22 +744,33 @@ void gl_grm(pcaone_ctx* c, const double* US, const double* V, int k, double* C, 
   const int nsl = (int)std::max<uint64_t>(1, std::min<uint64_t>(64, (4ull * c->sm_count * 128 + N - 1) / N));
   double* E = (double*)scratch(c, "grm_E", (size_t)mc_max * lde * 8);
   double* dpart = (double*)scratch(c, "grm_dpart", (size_t)nsl * N * 8);
-  double* L = (double*)scratch(c, "grm_L", (size_t)N * N * 8);
+  const int nsplit = syrk_splits(c, ntile, std::min<uint64_t>(M, mc_max));
+  double* L = (double*)scratch(c, "grm_L", (size_t)nsplit * N * N * 8);
   double* dC = (double*)scratch(c, "grm_C", (size_t)N * N * 8);
   PG_CUDA(cudaMemsetAsync(dpart, 0, (size_t)nsl * N * 8, c->stream));
   for (uint64_t j0 = 0; j0 < M; j0 += mc_max) {
     const uint64_t mc = std::min<uint64_t>(mc_max, M - j0);
-    k_grm_e<<<dim3((N + 127) / 128, nsl), 128, 0, c->stream>>>(c->d_P, N, 2 * N, c->d_F, US, V, k, j0, mc, E, lde,
-                                                              dpart);
+    auto go = [&](auto kern) {
+      kern<<<dim3((N + 127) / 128, nsl), 128, 0, c->stream>>>(c->d_P, N, 2 * N, c->d_F, US, V, k, j0, mc, E, lde, dpart);
+    };
+    if (k <= 8)
+      go(k_grm_e<8>);
+    else if (k <= 16)
+      go(k_grm_e<16>);
+    else if (k <= 32)
+      go(k_grm_e<32>);
+    else
+      go(k_grm_e<64>);
     PG_CHECK_LAUNCH();
     c->launches++;
-    k_syrk_lower<<<ntile * (ntile + 1) / 2, 256, kSyrkSmem, c->stream>>>(E, lde, N, mc, L, j0 == 0 ? 0 : 1);
+    k_syrk_lower<<<dim3(ntile * (ntile + 1) / 2, nsplit), 256, kSyrkSmem, c->stream>>>(E, lde, N, mc, L,
+                                                                                   j0 == 0 ? 0 : 1);
     PG_CHECK_LAUNCH();
     c->launches++;
   }
   const uint64_t n2 = (uint64_t)N * N;
   k_grm_finish<<<(unsigned)std::min<uint64_t>(8ull * c->sm_count, (n2 + 255) / 256), 256, 0, c->stream>>>(
-      L, dpart, nsl, N, (double)M, dC);
+      L, nsplit, dpart, nsl, N, (double)M, dC);
   PG_CHECK_LAUNCH();
   c->launches++;
   if (C) PG_CUDA(cudaMemcpyAsync(C, dC, n2 * 8, cudaMemcpyDeviceToHost, c->stream));

@@ -86,3 +86,20 @@ def test_pcangsd_grm_matches_reference_cov(gpu):
     Cr = O.read_eigen_matrix(ref_out("g3_pcangsd", ".cov"))
     np.testing.assert_allclose(C, Cr, atol=1e-5)
     top_vectors_match(ev, Cr, 3, 2e-3)
+
+
+@pytest.mark.parametrize("N,M,k", [(5, 3, 1), (127, 40, 8), (128, 700, 9), (129, 1031, 17), (385, 2100, 2), (300, 515, 40)])
+def test_gl_grm_tile_edges_and_site_splits(gpu, N, M, k):
+    """The SYRK at the edges of its 128-sample tiles and 16-site panels, with one and several site
+    ranges, and the standardised posterior at each register width."""
+    rng = np.random.default_rng(N + M)
+    g = rng.dirichlet(np.ones(3) * 0.7, size=(M, N))
+    P = np.empty((2 * N, M))
+    P[0::2, :] = g[:, :, 0].T
+    P[1::2, :] = g[:, :, 1].T
+    gpu.load_gl(P)
+    F, _ = gpu.gl_freq(20, 1e-6)
+    U, V = rng.standard_normal((N, k)) / np.sqrt(N), rng.standard_normal((M, k)) / np.sqrt(M)
+    S = np.linspace(2.0, 1.0, k)
+    C, _, _ = gpu.gl_grm(U, S, V, vectors=False)
+    np.testing.assert_allclose(C, grm_oracle(P, F, U, S, V), rtol=1e-10, atol=1e-12)
