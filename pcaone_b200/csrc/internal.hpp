@@ -273,10 +273,9 @@ void i8_tile_window(pcaone_ctx* c, cudaStream_t st, const uint8_t* rec, int64_t 
 
 // ---------------------------------------------------------------- SIMT decode-GEMM
 // out[s][r][c] = sum_{k in split s} val(code[r][k]) * B[k][c], val(00,01,10,11) = (2,0,1,0)
-// codes: rows x pitch bytes; B: row-major K x ldb (T); out: ksplit x rows x l (T).
-template <typename T>
+// codes: rows x pitch bytes; B: row-major K x ldb; out: ksplit x rows x l, all FP32.
 void launch_decode_gemm_simt(pcaone_ctx* c, const uint8_t* codes, uint32_t pitch, int64_t rows,
-                             int64_t K, const T* B, int ldb, int l, int ksplit, T* out);
+                             int64_t K, const float* B, int ldb, int l, int ksplit, float* out);
 
 // ---------------------------------------------------------------- tcgen05 decode-GEMM
 // Same contract with BF16 hi/lo split of B; see kernels_gemm_tc.cu.

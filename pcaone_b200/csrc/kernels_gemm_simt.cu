@@ -6,13 +6,20 @@
 // raw product of the reference's G^T * Omega and G * G (src/Halko.cpp:123-124, 193-202);
 // centring, scaling and the missing-entry terms are applied by the epilogue kernels.
 //
-// Tiling: a CTA owns 128 rows; each thread owns 4 rows x 8 columns of the output; K is
-// streamed in chunks of 64 codes (16 packed bytes per row) staged in shared memory together
+// FP32 (k_decode_gemm): a CTA owns 128 rows; each thread owns 4 rows x 8 columns of the output; K
+// is streamed in chunks of 64 codes (16 packed bytes per row) staged in shared memory together
 // with the matching 64 rows of B.
+// FP64 (k_decode_dmma, k_decode_dmv): the FP64 tensor tiles m8n8k4 for three columns or more,
+// a matrix-vector form for one or two, where seven eighths of a tile would be padding.
+//
+// K may run over consecutive windows (KRun), so that a run of windows is one product: one launch
+// with rows or K enough to fill the SMs instead of one per window (470 SNPs at M = 30011 in 64
+// windows: four row tiles).
 #include <algorithm>
 
 #include "internal.hpp"
 #include "rsvd.hpp"
+#include "tall.hpp"
 
 namespace pg {
 
@@ -31,146 +38,385 @@ __device__ __forceinline__ uint32_t map_values(uint32_t w) {
   return v0 | (v1 << 1);
 }
 
-template <typename T>
-__device__ __forceinline__ T small_to_real(uint32_t x);
-template <>
-__device__ __forceinline__ float small_to_real<float>(uint32_t x) {
-  return __int_as_float(0x4B400000u | x) - 12582912.0f;
-}
-template <>
-__device__ __forceinline__ double small_to_real<double>(uint32_t x) {
-  return __longlong_as_double(0x4338000000000000ull | x) - 6755399441055744.0;
-}
+__device__ __forceinline__ float small_to_real(uint32_t x) { return __int_as_float(0x4B400000u | x) - 12582912.0f; }
 
-template <typename T, int G>
+// The K positions of a product: windows of cpw chunks of 64 codes (kpw = 64 cpw rows of B each),
+// window w's codes win_bytes after those of window w - 1; position r of window w is valid when
+// r < wlen and w * wlen + r < mtot (the others multiply nothing: B is not read there).
+struct KRun {
+  int64_t cpw, win_bytes, kpw, wlen, mtot;
+  __device__ __forceinline__ int64_t valid(int64_t w) const { return min(wlen, mtot - w * wlen); }
+};
+
+template <int G>
 __global__ void __launch_bounds__(32 * G)
-k_decode_gemm(const uint8_t* __restrict__ codes, uint32_t pitch, int64_t rows, int64_t K,
-              const T* __restrict__ B, int ldb, int l, int64_t kchunks_per_split,
-              T* __restrict__ out) {
+k_decode_gemm(const uint8_t* __restrict__ codes, uint32_t pitch, int64_t rows, int64_t chunks, KRun run,
+              const float* __restrict__ B, int ldb, int l, int64_t kchunks_per_split,
+              float* __restrict__ out) {
   constexpr int LDS = G * kCW;              // padded B columns in shared memory
   __shared__ uint32_t pk[kTR * 5];          // 128 rows x 4 words, row stride 5 words
-  __shared__ __align__(16) T bs[kKC * LDS];
+  __shared__ __align__(16) float bs[kKC * LDS];
 
   const int lane = threadIdx.x & 31, g = threadIdx.x >> 5;
   const int64_t r0 = (int64_t)blockIdx.x * kTR;
   const int64_t kc_begin = (int64_t)blockIdx.y * kchunks_per_split;
-  const int64_t kc_total = (K + kKC - 1) / kKC;
-  const int64_t kc_end = min(kc_begin + kchunks_per_split, kc_total);
+  const int64_t kc_end = min(kc_begin + kchunks_per_split, chunks);
 
-  T acc[kRPT][kCW];
+  float acc[kRPT][kCW];
 #pragma unroll
   for (int q = 0; q < kRPT; ++q)
 #pragma unroll
-    for (int c = 0; c < kCW; ++c) acc[q][c] = T(0);
+    for (int c = 0; c < kCW; ++c) acc[q][c] = 0.f;
 
   for (int64_t kc = kc_begin; kc < kc_end; ++kc) {
-    const int64_t k0 = kc * kKC;
+    const int64_t w = kc / run.cpw, k0 = (kc - w * run.cpw) * kKC, kv = run.valid(w) - k0;
     // packed codes: 128 rows x 16 bytes
+    const uint8_t* src = codes + w * run.win_bytes + (k0 >> 2);
     for (int t = threadIdx.x; t < kTR * 4; t += 32 * G) {
-      int r = t >> 2, wq = t & 3;
-      const uint32_t* src = reinterpret_cast<const uint32_t*>(codes + (r0 + r) * (int64_t)pitch + (k0 >> 2));
-      pk[r * 5 + wq] = map_values(__ldg(src + wq));
+      const int r = t >> 2, wq = t & 3;
+      const int64_t row = min(r0 + r, rows - 1);
+      pk[r * 5 + wq] = map_values(__ldg(reinterpret_cast<const uint32_t*>(src + row * (int64_t)pitch) + wq));
     }
-    // B chunk: 64 rows x LDS columns (zero beyond l and beyond K)
+    // B chunk: 64 rows x LDS columns (zero beyond l and beyond the valid positions)
+    const float* Bc = B + (w * run.kpw + k0) * ldb;
     for (int t = threadIdx.x; t < kKC * LDS; t += 32 * G) {
-      int kk = t / LDS, cc = t - kk * LDS;
-      int64_t k = k0 + kk;
-      bs[t] = (cc < l && k < K) ? B[k * ldb + cc] : T(0);
+      const int kk = t / LDS, cc = t - kk * LDS;
+      bs[t] = (cc < l && kk < kv) ? Bc[kk * ldb + cc] : 0.f;
     }
     __syncthreads();
 #pragma unroll
     for (int wq = 0; wq < 4; ++wq) {
-      uint32_t w[kRPT];
+      uint32_t x[kRPT];
 #pragma unroll
-      for (int q = 0; q < kRPT; ++q) w[q] = pk[(lane + 32 * q) * 5 + wq];
+      for (int q = 0; q < kRPT; ++q) x[q] = pk[(lane + 32 * q) * 5 + wq];
 #pragma unroll
       for (int e = 0; e < 16; ++e) {
-        const T* brow = bs + (wq * 16 + e) * LDS + g * kCW;
-        T b[kCW];
+        const float* brow = bs + (wq * 16 + e) * LDS + g * kCW;
+        float b[kCW];
 #pragma unroll
         for (int c = 0; c < kCW; ++c) b[c] = brow[c];
 #pragma unroll
         for (int q = 0; q < kRPT; ++q) {
-          T v = small_to_real<T>((w[q] >> (2 * e)) & 3u);
+          const float v = small_to_real((x[q] >> (2 * e)) & 3u);
 #pragma unroll
-          for (int c = 0; c < kCW; ++c) acc[q][c] = fma(v, b[c], acc[q][c]);
+          for (int c = 0; c < kCW; ++c) acc[q][c] = fmaf(v, b[c], acc[q][c]);
         }
       }
     }
     __syncthreads();
   }
-  T* o = out + (int64_t)blockIdx.y * rows * l;
+  float* o = out + (int64_t)blockIdx.y * rows * l;
 #pragma unroll
   for (int q = 0; q < kRPT; ++q) {
-    int64_t r = r0 + lane + 32 * q;
+    const int64_t r = r0 + lane + 32 * q;
     if (r >= rows) continue;
 #pragma unroll
     for (int c = 0; c < kCW; ++c) {
-      int col = g * kCW + c;
+      const int col = g * kCW + c;
       if (col < l) o[r * l + col] = acc[q][c];
     }
   }
 }
 
-template <typename T, int G>
-void launch_g(pcaone_ctx* c, const uint8_t* codes, uint32_t pitch, int64_t rows, int64_t K,
-              const T* B, int ldb, int l, int ksplit, T* out) {
-  int64_t kc_total = (K + kKC - 1) / kKC;
-  int64_t per = (kc_total + ksplit - 1) / ksplit;
-  dim3 grid((unsigned)((rows + kTR - 1) / kTR), (unsigned)ksplit);
-  k_decode_gemm<T, G><<<grid, 32 * G, 0, c->stream>>>(codes, pitch, rows, K, B, ldb, l, per, out);
+// ---------------------------------------------------------------- FP64
+// Value of raw code c (00 -> 2, 01 -> 0, 10 -> 1, 11 -> 0) as a double: its two high bytes are a
+// byte lookup (2.0 = 0x4000.., 1.0 = 0x3FF0..), the rest is zero.
+__device__ __forceinline__ double code_to_double(uint32_t c) {
+  return __hiloint2double((int)__byte_perm(0x00004000u, 0x00003FF0u, c * 0x2200u + 0x1022u), 0);
+}
+
+__device__ __forceinline__ void cp_async8_zfill(double* sdst, const double* gsrc, bool ok) {
+  const uint32_t d = (uint32_t)__cvta_generic_to_shared(sdst);
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(d), "l"(gsrc), "r"(ok ? 8 : 0) : "memory");
+}
+
+// A CTA owns 128 rows, a warp 16 (two row tiles), NT column tiles of 8. A lane's A element of the
+// four codes 4 s .. 4 s + 3 is code lane % 4 of byte s of row lane / 4, so the codes come
+// straight from global memory (16 bytes a row and chunk, the next chunk's in flight) and a
+// decoded value serves NT tensor tiles. B is staged 64 rows at a time in two buffers (8-byte
+// asynchronous copies, row stride 4 mod 16 doubles: conflict-free 4 x 4 reads).
+// Bound by the FP64 pipe for wide B. M = 60000, N = 5000, 10 columns: PLACEHOLDER_DMMA.
+constexpr int kDmmaThreads = 256;
+template <int NT>
+__global__ void __launch_bounds__(kDmmaThreads)
+k_decode_dmma(const uint8_t* __restrict__ codes, uint32_t pitch, int64_t rows, int64_t chunks, KRun run,
+              const double* __restrict__ B, int ldb, int l, int64_t kchunks_per_split, double* __restrict__ out) {
+  constexpr int LD = Tall<NT>::LD;
+  extern __shared__ __align__(16) double bsm[];  // 2 x 64 x LD
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, q4 = lane >> 2, r4 = lane & 3;
+  const int64_t row0 = (int64_t)blockIdx.x * kTR + warp * 16 + q4;  // and row0 + 8
+  const int64_t kc0 = (int64_t)blockIdx.y * kchunks_per_split, kc1 = min(kc0 + kchunks_per_split, chunks);
+  const uint8_t* rowp[2] = {codes + min(row0, rows - 1) * (int64_t)pitch, codes + min(row0 + 8, rows - 1) * (int64_t)pitch};
+  for (int t = threadIdx.x; t < 2 * kKC * LD; t += kDmmaThreads) bsm[t] = 0.0;  // padded columns stay zero
+  __syncthreads();
+  auto issue = [&](int64_t kc, int buf) {
+    const int64_t w = kc / run.cpw, k0 = (kc - w * run.cpw) * kKC, kv = run.valid(w) - k0;
+    const double* Bc = B + (w * run.kpw + k0) * ldb;
+    double* dst = bsm + buf * kKC * LD;
+    for (int t = threadIdx.x; t < kKC * l; t += kDmmaThreads) {
+      const int kk = t / l, cc = t - kk * l;
+      const bool ok = kk < kv;
+      cp_async8_zfill(dst + kk * LD + cc, ok ? Bc + (int64_t)kk * ldb + cc : B, ok);
+    }
+    asm volatile("cp.async.commit_group;\n" ::: "memory");
+  };
+  auto fetch = [&](int64_t kc, uint4 (&x)[2]) {
+    const int64_t w = kc / run.cpw, o = w * run.win_bytes + (kc - w * run.cpw) * (kKC / 4);
+#pragma unroll
+    for (int h = 0; h < 2; ++h) x[h] = __ldg(reinterpret_cast<const uint4*>(rowp[h] + o));
+  };
+  double acc[2][NT][2];
+#pragma unroll
+  for (int h = 0; h < 2; ++h)
+#pragma unroll
+    for (int t = 0; t < NT; ++t) acc[h][t][0] = acc[h][t][1] = 0.0;
+  uint4 cur[2], nxt[2];
+  if (kc0 < kc1) {
+    issue(kc0, 0);
+    fetch(kc0, cur);
+  }
+  for (int64_t kc = kc0; kc < kc1; ++kc) {
+    const int buf = (int)(kc - kc0) & 1;
+    if (kc + 1 < kc1) {
+      issue(kc + 1, buf ^ 1);
+      fetch(kc + 1, nxt);
+      asm volatile("cp.async.wait_group 1;\n" ::: "memory");
+    } else {
+      asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+    }
+    __syncthreads();
+    const double* bs = bsm + buf * kKC * LD + r4 * LD + q4;
+    const uint32_t x[2][4] = {{cur[0].x >> (2 * r4), cur[0].y >> (2 * r4), cur[0].z >> (2 * r4), cur[0].w >> (2 * r4)},
+                              {cur[1].x >> (2 * r4), cur[1].y >> (2 * r4), cur[1].z >> (2 * r4), cur[1].w >> (2 * r4)}};
+#pragma unroll
+    for (int s = 0; s < kKC / 4; ++s) {
+      const double a0 = code_to_double((x[0][s >> 2] >> (8 * (s & 3))) & 3u);
+      const double a1 = code_to_double((x[1][s >> 2] >> (8 * (s & 3))) & 3u);
+#pragma unroll
+      for (int t = 0; t < NT; ++t) {
+        const double b = bs[4 * s * LD + 8 * t];
+        dmma(acc[0][t], a0, b);
+        dmma(acc[1][t], a1, b);
+      }
+    }
+    __syncthreads();  // the buffer is read before it is refilled
+    cur[0] = nxt[0];
+    cur[1] = nxt[1];
+  }
+  double* o = out + (int64_t)blockIdx.y * rows * l;
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    const int64_t row = row0 + 8 * h;
+    if (row >= rows) continue;
+#pragma unroll
+    for (int t = 0; t < NT; ++t)
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        const int col = 8 * t + 2 * r4 + e;
+        if (col < l) o[row * l + col] = acc[h][t][e];
+      }
+  }
+}
+
+// One or two columns: a warp owns kDmvRows rows, a lane 16 codes of each in a step of 512, and
+// the matching values of B lie in shared memory in the lanes' order ([code of the word][word],
+// 2048 rows of B at a time). A value of B read from shared memory serves kDmvRows rows (at one
+// row a read, shared memory would hold the FP64 pipe to a quarter of its rate); the bound is
+// the integer work of the decode. M = 60001, N = 3000, one column: PLACEHOLDER_DMV.
+constexpr int kDmvThreads = 256, kDmvRows = 8, kDmvTile = kDmvThreads / 32 * kDmvRows, kDmvK = 2048;
+template <int L>
+__global__ void __launch_bounds__(kDmvThreads)
+k_decode_dmv(const uint8_t* __restrict__ codes, uint32_t pitch, int64_t rows, int64_t chunks, KRun run,
+             const double* __restrict__ B, int64_t kchunks_per_split, double* __restrict__ out) {
+  constexpr int kSpan = kDmvK / kKC, kWords = kDmvK / 16 + 1;  // (+ 1: the transposing writes spread over the banks)
+  __shared__ __align__(16) double bs[16 * kWords * L];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int64_t row0 = (int64_t)blockIdx.x * kDmvTile + warp * kDmvRows;
+  const int64_t kc0 = (int64_t)blockIdx.y * kchunks_per_split, kc1 = min(kc0 + kchunks_per_split, chunks);
+  double acc[kDmvRows][L];
+#pragma unroll
+  for (int r = 0; r < kDmvRows; ++r)
+#pragma unroll
+    for (int c = 0; c < L; ++c) acc[r][c] = 0.0;
+  for (int64_t kc = kc0; kc < kc1;) {
+    // up to kSpan chunks that stay inside one window
+    const int64_t w = kc / run.cpw, k0 = (kc - w * run.cpw) * kKC, kv = run.valid(w) - k0;
+    const int64_t n = min((int64_t)kSpan, min(kc1 - kc, (w + 1) * run.cpw - kc));
+    const int words = (int)n * (kKC / 16);
+    const double* Bc = B + (w * run.kpw + k0) * L;
+    __syncthreads();  // the previous values are used up
+    for (int t = threadIdx.x; t < words * 16; t += kDmvThreads) {
+      const int e = t & 15, wd = t >> 4;
+#pragma unroll
+      for (int c = 0; c < L; ++c) bs[(e * kWords + wd) * L + c] = t < kv ? Bc[t * L + c] : 0.0;
+    }
+    __syncthreads();
+    const uint8_t* src = codes + w * run.win_bytes + (k0 >> 2);
+    for (int wd = lane; wd < words; wd += 32) {
+      uint32_t x[kDmvRows];
+#pragma unroll
+      for (int r = 0; r < kDmvRows; ++r)
+        x[r] = __ldg(reinterpret_cast<const uint32_t*>(src + min(row0 + r, rows - 1) * (int64_t)pitch) + wd);
+#pragma unroll
+      for (int e = 0; e < 16; ++e) {
+        double b[L];
+#pragma unroll
+        for (int c = 0; c < L; ++c) b[c] = bs[(e * kWords + wd) * L + c];
+#pragma unroll
+        for (int r = 0; r < kDmvRows; ++r) {
+          const double v = code_to_double((x[r] >> (2 * e)) & 3u);
+#pragma unroll
+          for (int c = 0; c < L; ++c) acc[r][c] = fma(v, b[c], acc[r][c]);
+        }
+      }
+    }
+    kc += n;
+  }
+  double* o = out + (int64_t)blockIdx.y * rows * L;
+#pragma unroll
+  for (int r = 0; r < kDmvRows; ++r)
+#pragma unroll
+    for (int c = 0; c < L; ++c) {
+      double v = acc[r][c];
+      for (int d = 16; d; d >>= 1) v += __shfl_xor_sync(0xffffffffu, v, d);
+      if (lane == 0 && row0 + r < rows) o[(row0 + r) * L + c] = v;
+    }
+}
+
+KRun whole_k(int64_t K) {
+  const int64_t chunks = (K + kKC - 1) / kKC;
+  return KRun{chunks, 0, chunks * kKC, K, K};
+}
+
+void run_simt(pcaone_ctx* c, const uint8_t* codes, uint32_t pitch, int64_t rows, int64_t chunks, const KRun& run,
+              const float* B, int ldb, int l, int ksplit, float* out) {
+  const int64_t per = (chunks + ksplit - 1) / ksplit;
+  const dim3 grid((unsigned)((rows + kTR - 1) / kTR), (unsigned)ksplit);
+  auto go = [&](auto kern, int G) { kern<<<grid, 32 * G, 0, c->stream>>>(codes, pitch, rows, chunks, run, B, ldb, l, per, out); };
+  switch ((l + kCW - 1) / kCW) {
+    case 1: go(k_decode_gemm<1>, 1); break;
+    case 2: go(k_decode_gemm<2>, 2); break;
+    case 3: go(k_decode_gemm<3>, 3); break;
+    case 4: go(k_decode_gemm<4>, 4); break;
+    case 5: go(k_decode_gemm<5>, 5); break;
+    case 6: go(k_decode_gemm<6>, 6); break;
+    case 7: go(k_decode_gemm<7>, 7); break;
+    default: go(k_decode_gemm<8>, 8); break;
+  }
   PG_CHECK_LAUNCH();
+  c->launches++;
+  c->gemm_launches++;
+}
+
+void run_simt(pcaone_ctx* c, const uint8_t* codes, uint32_t pitch, int64_t rows, int64_t chunks, const KRun& run,
+              const double* B, int ldb, int l, int ksplit, double* out) {
+  PG_REQUIRE(ldb == l, PCAONE_EBADARG, "FP64 operand rows must be contiguous");
+  const int64_t per = (chunks + ksplit - 1) / ksplit;
+  if (l <= 2) {
+    const dim3 grid((unsigned)((rows + kDmvTile - 1) / kDmvTile), (unsigned)ksplit);
+    if (l == 1)
+      k_decode_dmv<1><<<grid, kDmvThreads, 0, c->stream>>>(codes, pitch, rows, chunks, run, B, per, out);
+    else
+      k_decode_dmv<2><<<grid, kDmvThreads, 0, c->stream>>>(codes, pitch, rows, chunks, run, B, per, out);
+  } else {
+    const dim3 grid((unsigned)((rows + kTR - 1) / kTR), (unsigned)ksplit);
+    auto go = [&](auto kern, int nt) {
+      const size_t smem = (size_t)2 * kKC * (8 * nt + 4) * 8;
+      if (c->smem_attr_set.insert((const void*)kern).second)
+        PG_CUDA(cudaFuncSetAttribute((const void*)kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+      kern<<<grid, kDmmaThreads, smem, c->stream>>>(codes, pitch, rows, chunks, run, B, ldb, l, per, out);
+    };
+    switch ((l + 7) / 8) {
+      case 1: go(k_decode_dmma<1>, 1); break;
+      case 2: go(k_decode_dmma<2>, 2); break;
+      case 3: go(k_decode_dmma<3>, 3); break;
+      case 4: go(k_decode_dmma<4>, 4); break;
+      case 5: go(k_decode_dmma<5>, 5); break;
+      case 6: go(k_decode_dmma<6>, 6); break;
+      case 7: go(k_decode_dmma<7>, 7); break;
+      default: go(k_decode_dmma<8>, 8); break;
+    }
+  }
+  PG_CHECK_LAUNCH();
+  c->launches++;
+  c->gemm_launches++;
 }
 
 }  // namespace
 
-template <typename T>
 void launch_decode_gemm_simt(pcaone_ctx* c, const uint8_t* codes, uint32_t pitch, int64_t rows,
-                             int64_t K, const T* B, int ldb, int l, int ksplit, T* out) {
+                             int64_t K, const float* B, int ldb, int l, int ksplit, float* out) {
   PG_REQUIRE(l >= 1 && l <= kLmax, PCAONE_EBADARG, "sketch width out of range");
-  int G = (l + kCW - 1) / kCW;
-  switch (G) {
-    case 1: launch_g<T, 1>(c, codes, pitch, rows, K, B, ldb, l, ksplit, out); break;
-    case 2: launch_g<T, 2>(c, codes, pitch, rows, K, B, ldb, l, ksplit, out); break;
-    case 3: launch_g<T, 3>(c, codes, pitch, rows, K, B, ldb, l, ksplit, out); break;
-    case 4: launch_g<T, 4>(c, codes, pitch, rows, K, B, ldb, l, ksplit, out); break;
-    case 5: launch_g<T, 5>(c, codes, pitch, rows, K, B, ldb, l, ksplit, out); break;
-    case 6: launch_g<T, 6>(c, codes, pitch, rows, K, B, ldb, l, ksplit, out); break;
-    case 7: launch_g<T, 7>(c, codes, pitch, rows, K, B, ldb, l, ksplit, out); break;
-    default: launch_g<T, 8>(c, codes, pitch, rows, K, B, ldb, l, ksplit, out); break;
-  }
-  c->launches++;
-  c->gemm_launches++;
+  const KRun run = whole_k(K);
+  run_simt(c, codes, pitch, rows, run.cpw, run, B, ldb, l, ksplit, out);
 }
 
 namespace {
 template <typename T>
 void simt_gemm(pcaone_ctx* c, const uint8_t* codes, uint32_t pitch, int64_t, int64_t rows, int64_t K,
                const T* B, int l, int ks, T* out) {
-  launch_decode_gemm_simt<T>(c, codes, pitch, rows, K, B, l, l, ks, out);
+  PG_REQUIRE(l >= 1 && l <= kLmax, PCAONE_EBADARG, "sketch width out of range");
+  const KRun run = whole_k(K);
+  run_simt(c, codes, pitch, rows, run.cpw, run, B, l, l, ks, out);
 }
-int simt_ksplit(pcaone_ctx* c, int64_t rows, int64_t K, int) {
-  int64_t tiles = (rows + kTR - 1) / kTR;
-  int64_t chunks = (K + kKC - 1) / kKC;
-  int64_t want = (2 * (int64_t)c->sm_count + tiles - 1) / tiles;
-  int64_t ks = std::max<int64_t>(1, std::min<int64_t>(want, chunks / 4));
+
+// K splits: CTAs for about 16 warps an SM (FP32: 1 to 8 warps a CTA; FP64: 8), each split at least
+// four chunks long; the matrix-vector form takes whole spans of its staged B.
+template <typename T>
+int simt_ksplit(pcaone_ctx* c, int64_t rows, int64_t K, int l) {
+  const bool dmv = sizeof(T) == 8 && l <= 2;
+  const int64_t tile = dmv ? kDmvTile : kTR, warps = sizeof(T) == 8 ? 8 : (l + kCW - 1) / kCW;
+  const int64_t tiles = (rows + tile - 1) / tile, chunks = (K + kKC - 1) / kKC;
+  const int64_t ctas = std::max<int64_t>(2, (dmv ? 32 : 16) / warps);
+  const int64_t want = (ctas * c->sm_count + tiles - 1) / tiles;
+  const int64_t ks = std::max<int64_t>(1, std::min<int64_t>(want, chunks / (dmv ? kDmvK / kKC / 2 : 4)));
   return (int)std::min<int64_t>(ks, 64);
 }
 void no_omega(pcaone_ctx*, const double*, int, int64_t) {}
 template <typename T>
 void no_b2(pcaone_ctx*, const T*, int, int64_t) {}
+
+// ---- runs of consecutive windows [b0, b1): the first product's rows are the run's SNPs (contiguous
+// records); the second product's K runs over the windows of the sample-major copies, each padded
+// to its pitch.
+int64_t simt_rows1(pcaone_ctx* c) { return (int64_t)c->win.blocksize; }
+int64_t simt_k2(pcaone_ctx* c) { return (int64_t)c->win.pitch * 4; }
+template <typename T>
+int simt_ksplit_seg(pcaone_ctx* c, int which, int nw, int l) {
+  return which == 1 ? simt_ksplit<T>(c, (int64_t)nw * (int64_t)c->win.blocksize, (int64_t)c->N, l)
+                    : simt_ksplit<T>(c, (int64_t)c->N, (int64_t)nw * simt_k2(c), l);
+}
+template <typename T>
+void simt_p1_seg(pcaone_ctx* c, int b0, int b1, const T* B, int l, int ks, T* out) {
+  const int64_t s = (int64_t)c->win.start[b0], m = (int64_t)c->win.stop[b1 - 1] - s;
+  simt_gemm<T>(c, c->streamed ? stream_codes(c, b0) : c->d_bed + s * (int64_t)c->pitch, c->pitch, s, m, (int64_t)c->N, B,
+               l, ks, out);
+}
+template <typename T>
+void simt_b2_seg(pcaone_ctx*, const T*, int, int, int) {}
+template <typename T>
+void simt_p2_seg(pcaone_ctx* c, int b0, int b1, const T* B2, int l, int ks, T* out) {
+  const int64_t k2 = simt_k2(c), win_bytes = (int64_t)c->Npad * c->win.pitch;
+  const KRun run{k2 / kKC, win_bytes, k2, (int64_t)c->win.blocksize, (int64_t)(c->win.stop[b1 - 1] - c->win.start[b0])};
+  run_simt(c, c->streamed ? stream_codesT(c, b0) : c->d_bedT + b0 * win_bytes, c->win.pitch, (int64_t)c->N,
+           (b1 - b0) * run.cpw, run, B2, l, l, ks, out);
+}
+
+template <typename T>
+GemmFnT<T> simt_backend() {
+  GemmFnT<T> f{simt_ksplit<T>, simt_gemm<T>, simt_gemm<T>, no_omega, no_b2<T>};
+  f.seg_rows1 = simt_rows1;
+  f.seg_k2 = simt_k2;
+  f.seg_exact_rows = true;
+  f.ksplit_seg = simt_ksplit_seg<T>;
+  f.p1_seg = simt_p1_seg<T>;
+  f.b2_seg = simt_b2_seg<T>;
+  f.p2_seg = simt_p2_seg<T>;
+  return f;
+}
 }  // namespace
 
-GemmFnT<float> gemm_simt_float() {
-  return GemmFnT<float>{simt_ksplit, simt_gemm<float>, simt_gemm<float>, no_omega, no_b2<float>};
-}
-GemmFnT<double> gemm_simt_double() {
-  return GemmFnT<double>{simt_ksplit, simt_gemm<double>, simt_gemm<double>, no_omega, no_b2<double>};
-}
-
-template void launch_decode_gemm_simt<float>(pcaone_ctx*, const uint8_t*, uint32_t, int64_t,
-                                             int64_t, const float*, int, int, int, float*);
-template void launch_decode_gemm_simt<double>(pcaone_ctx*, const uint8_t*, uint32_t, int64_t,
-                                              int64_t, const double*, int, int, int, double*);
+GemmFnT<float> gemm_simt_float() { return simt_backend<float>(); }
+GemmFnT<double> gemm_simt_double() { return simt_backend<double>(); }
 
 }  // namespace pg

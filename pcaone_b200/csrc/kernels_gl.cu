@@ -637,6 +637,7 @@ GemmFnT<float> gemm_dense_float() {
   GemmFnT<float> f{dense_ksplit, dense_p1, dense_p2, dense_none_omega, dense_none_b2};
   f.seg_rows1 = dense_seg_rows;
   f.seg_k2 = dense_seg_rows;
+  f.seg_exact_rows = true;
   f.ksplit_seg = dense_ksplit_seg;
   f.p1_seg = dense_p1_seg;
   f.b2_seg = dense_seg_b2;

@@ -124,7 +124,7 @@ void product_t_noalloc(pcaone_ctx* c, int standardize, int ploidy, const double*
   k_colsum<<<l, 256, 0, c->stream>>>(Bd, (uint32_t)N, l, wsum);
   PG_CHECK_LAUNCH();
   compute_scale(c, standardize, ploidy);
-  launch_decode_gemm_simt<float>(c, c->d_bed, c->pitch, (int64_t)M, (int64_t)N, Bf, l, l, (int)ks, D1);
+  launch_decode_gemm_simt(c, c->d_bed, c->pitch, (int64_t)M, (int64_t)N, Bf, l, l, (int)ks, D1);
   k_epilogue<<<(unsigned)((M * 32 + 255) / 256), 256, 0, c->stream>>>(
       D1, (int)ks, M, l, c->d_F, c->d_scale, wsum, Bd, c->d_miss_snp_ptr, c->d_miss_snp_idx,
       c->imputed ? c->d_miss_snp_val : nullptr, d_out);

@@ -356,9 +356,9 @@ struct Engine {
     const int nw = b1 - b0;
     const int64_t rows1 = gemm.seg_rows1(c), k2 = gemm.seg_k2(c);
     const int ks1 = gemm.ksplit_seg(c, 1, nw, l);
-    // D1 rows per split: the padded windows of the back end, or exactly the run's SNPs for the
-    // dense matrix (whose windows are contiguous rows without padding)
-    const int64_t d1rows = c->dense ? m : nw * rows1;
+    // D1 rows per split: the padded windows of the back end, or exactly the run's SNPs where its
+    // windows are contiguous rows without padding
+    const int64_t d1rows = gemm.seg_exact_rows ? m : nw * rows1;
     T* D1 = (T*)scratch(c, "r_D1", (size_t)ks1 * std::max<int64_t>(d1rows, nw * rows1) * l * sizeof(T));
     timed([&] { gemm.p1_seg(c, b0, b1, OmgT, l, ks1, D1); });
     EpiP1 p1;
@@ -382,7 +382,9 @@ struct Engine {
     T* B2 = (T*)scratch(c, "r_B2", (size_t)nw * k2 * l * sizeof(T));
     double* h0 = (double*)scratch(c, "r_h0", l * 8);
     p1.qmax = gemm.b2_qmax ? gemm.b2_qmax(c, l) : nullptr;
-    float* Gf = (float*)scratch(c, "r_Gf", (size_t)round_up(m, 256) * l * sizeof(float));
+    float* Gf = std::is_same<T, float>::value
+                    ? (float*)scratch(c, "r_Gf", (size_t)round_up(m, 256) * l * sizeof(float))
+                    : nullptr;
     p1.Gf = Gf;
     timed([&] {
       launch_prep<T>(c, p1, D1, B2, h0);

@@ -38,6 +38,8 @@ struct GemmFnT {
   int64_t (*seg_rows1)(pcaone_ctx* c) = nullptr;
   int64_t (*seg_k2)(pcaone_ctx* c) = nullptr;
   int (*ksplit_seg)(pcaone_ctx* c, int which, int nw, int l) = nullptr;
+  // The first product of a run writes exactly the run's SNP rows (no padding between windows).
+  bool seg_exact_rows = false;
   // B: the first product's operand (Omega, engine layout) / the run's B2 (seg_k2 rows per
   // window); back ends that keep their own packed copy ignore it.
   void (*p1_seg)(pcaone_ctx* c, int b0, int b1, const T* B, int l, int ks, T* out) = nullptr;

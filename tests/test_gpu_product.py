@@ -73,3 +73,34 @@ def test_gram_product_matches_dense(gpu, prec):
     X = np.random.default_rng(3).standard_normal((bed.N, 5))
     got = gpu.gram_product(X, precision=prec)
     assert rel_col_err(got, Z @ (Z.T @ X)) <= 2 * TOL[prec]
+
+
+@pytest.mark.parametrize("N,M", [(64, 63), (65, 129), (127, 2049), (2051, 128), (300, 4100)])
+@pytest.mark.parametrize("l", [1, 2, 3, 8, 9, 24, 41, 64])
+def test_fp64_products_at_tile_and_chunk_edges(gpu, N, M, l):
+    """The FP64 products at the edges of their row tiles (64 and 128), K chunks (64, spans of 2048)
+    and column tiles, in the matrix-vector (l <= 2) and the tensor form."""
+    bed = random_bed(N, M, seed=N + M + l, miss=0.03)
+    gpu.load_bed(bed.packed, N)
+    Z, _ = O.standardized_from_bed(bed)
+    rng = np.random.default_rng(l)
+    for Zx, got in ((Z.T, gpu.product_t), (Z, gpu.product)):
+        B = rng.standard_normal((Zx.shape[1], l))
+        ref = Zx @ B
+        # sums of at most 4100 terms of order 1: error below 4100 * 2^-53 of the largest
+        np.testing.assert_allclose(got(B, precision="fp64"), ref, rtol=0, atol=1e-12 * np.abs(ref).max())
+    X = rng.standard_normal((N, l))
+    ref = Z @ (Z.T @ X)
+    np.testing.assert_allclose(gpu.gram_product(X, precision="fp64"), ref, rtol=0, atol=1e-12 * np.abs(ref).max())
+
+
+@pytest.mark.parametrize("precision,tol", [("fp64", 1e-9), ("fp32", 1e-5)])
+@pytest.mark.parametrize("N,M,bands,k", [(203, 1501, 8, 4), (130, 641, 16, 1), (513, 4099, 4, 16)])
+def test_simt_window_runs_match_oracle(gpu, precision, tol, N, M, bands, k):
+    """winSVD on the FP32 and FP64 back ends, whose windows run as one product: uneven windows."""
+    bed = random_bed(N, M, seed=N, miss=0.02)
+    gpu.load_bed(bed.packed, N)
+    kw = dict(k=k, svd=2, bands=bands, maxp=5, tol=0.0)
+    r = gpu.rsvd(precision=precision, **kw)
+    S = O.run_pca(bed, shuffle=False, **kw)[1]
+    np.testing.assert_allclose(r.S, S, rtol=tol)
