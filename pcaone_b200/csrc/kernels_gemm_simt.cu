@@ -48,19 +48,50 @@ struct KRun {
   __device__ __forceinline__ int64_t valid(int64_t w) const { return min(wlen, mtot - w * wlen); }
 };
 
+// n bytes of asynchronous copy, zero-filled when !ok.
+template <int kBytes>
+__device__ __forceinline__ void cp_async_zfill(void* sdst, const void* gsrc, bool ok) {
+  const uint32_t d = (uint32_t)__cvta_generic_to_shared(sdst);
+  asm volatile("cp.async.ca.shared.global [%0], [%1], %2, %3;\n" ::"r"(d), "l"(gsrc), "n"(kBytes), "r"(ok ? kBytes : 0)
+               : "memory");
+}
+
+// The codes of a thread's four rows come straight from global memory (16 bytes a row and chunk)
+// and B through two shared-memory buffers of 4-byte asynchronous copies, both one chunk ahead:
+// with one to eight warps a CTA the copies' latency is what bounds it otherwise.
+// Runs of a winSVD, M = 30011, N = 1502, l = 15, mean of 266 products: 12.8 us with splits
+// down to one chunk (30.9 staged through registers with four chunks a split at least).
 template <int G>
 __global__ void __launch_bounds__(32 * G)
 k_decode_gemm(const uint8_t* __restrict__ codes, uint32_t pitch, int64_t rows, int64_t chunks, KRun run,
               const float* __restrict__ B, int ldb, int l, int64_t kchunks_per_split,
               float* __restrict__ out) {
   constexpr int LDS = G * kCW;              // padded B columns in shared memory
-  __shared__ uint32_t pk[kTR * 5];          // 128 rows x 4 words, row stride 5 words
-  __shared__ __align__(16) float bs[kKC * LDS];
+  __shared__ __align__(16) float bsm[2][kKC * LDS];
 
   const int lane = threadIdx.x & 31, g = threadIdx.x >> 5;
-  const int64_t r0 = (int64_t)blockIdx.x * kTR;
-  const int64_t kc_begin = (int64_t)blockIdx.y * kchunks_per_split;
-  const int64_t kc_end = min(kc_begin + kchunks_per_split, chunks);
+  const int64_t r0 = (int64_t)blockIdx.x * kTR + lane;
+  const int64_t kc0 = (int64_t)blockIdx.y * kchunks_per_split, kc1 = min(kc0 + kchunks_per_split, chunks);
+  const uint8_t* rowp[kRPT];
+#pragma unroll
+  for (int q = 0; q < kRPT; ++q) rowp[q] = codes + min(r0 + 32 * q, rows - 1) * (int64_t)pitch;
+  for (int t = threadIdx.x; t < 2 * kKC * LDS; t += 32 * G) (&bsm[0][0])[t] = 0.f;  // padded columns stay zero
+  __syncthreads();
+  auto issue = [&](int64_t kc, int buf) {
+    const int64_t w = kc / run.cpw, k0 = (kc - w * run.cpw) * kKC, kv = run.valid(w) - k0;
+    const float* Bc = B + (w * run.kpw + k0) * ldb;
+    for (int t = threadIdx.x; t < kKC * l; t += 32 * G) {
+      const int kk = t / l, cc = t - kk * l;
+      const bool ok = kk < kv;
+      cp_async_zfill<4>(&bsm[buf][kk * LDS + cc], ok ? Bc + (int64_t)kk * ldb + cc : B, ok);
+    }
+    asm volatile("cp.async.commit_group;\n" ::: "memory");
+  };
+  auto fetch = [&](int64_t kc, uint4 (&x)[kRPT]) {
+    const int64_t w = kc / run.cpw, o = w * run.win_bytes + (kc - w * run.cpw) * (kKC / 4);
+#pragma unroll
+    for (int q = 0; q < kRPT; ++q) x[q] = __ldg(reinterpret_cast<const uint4*>(rowp[q] + o));
+  };
 
   float acc[kRPT][kCW];
 #pragma unroll
@@ -68,33 +99,32 @@ k_decode_gemm(const uint8_t* __restrict__ codes, uint32_t pitch, int64_t rows, i
 #pragma unroll
     for (int c = 0; c < kCW; ++c) acc[q][c] = 0.f;
 
-  for (int64_t kc = kc_begin; kc < kc_end; ++kc) {
-    const int64_t w = kc / run.cpw, k0 = (kc - w * run.cpw) * kKC, kv = run.valid(w) - k0;
-    // packed codes: 128 rows x 16 bytes
-    const uint8_t* src = codes + w * run.win_bytes + (k0 >> 2);
-    for (int t = threadIdx.x; t < kTR * 4; t += 32 * G) {
-      const int r = t >> 2, wq = t & 3;
-      const int64_t row = min(r0 + r, rows - 1);
-      pk[r * 5 + wq] = map_values(__ldg(reinterpret_cast<const uint32_t*>(src + row * (int64_t)pitch) + wq));
-    }
-    // B chunk: 64 rows x LDS columns (zero beyond l and beyond the valid positions)
-    const float* Bc = B + (w * run.kpw + k0) * ldb;
-    for (int t = threadIdx.x; t < kKC * LDS; t += 32 * G) {
-      const int kk = t / LDS, cc = t - kk * LDS;
-      bs[t] = (cc < l && kk < kv) ? Bc[kk * ldb + cc] : 0.f;
+  uint4 cur[kRPT], nxt[kRPT];
+  if (kc0 < kc1) {
+    issue(kc0, 0);
+    fetch(kc0, cur);
+  }
+  for (int64_t kc = kc0; kc < kc1; ++kc) {
+    const int buf = (int)(kc - kc0) & 1;
+    if (kc + 1 < kc1) {
+      issue(kc + 1, buf ^ 1);
+      fetch(kc + 1, nxt);
+      asm volatile("cp.async.wait_group 1;\n" ::: "memory");
+    } else {
+      asm volatile("cp.async.wait_group 0;\n" ::: "memory");
     }
     __syncthreads();
+    const uint32_t* xw = reinterpret_cast<const uint32_t*>(cur);
 #pragma unroll
     for (int wq = 0; wq < 4; ++wq) {
       uint32_t x[kRPT];
 #pragma unroll
-      for (int q = 0; q < kRPT; ++q) x[q] = pk[(lane + 32 * q) * 5 + wq];
+      for (int q = 0; q < kRPT; ++q) x[q] = map_values(xw[4 * q + wq]);
 #pragma unroll
       for (int e = 0; e < 16; ++e) {
-        const float* brow = bs + (wq * 16 + e) * LDS + g * kCW;
-        float b[kCW];
-#pragma unroll
-        for (int c = 0; c < kCW; ++c) b[c] = brow[c];
+        const float4* brow = reinterpret_cast<const float4*>(&bsm[buf][(wq * 16 + e) * LDS + g * kCW]);
+        const float4 b0 = brow[0], b1 = brow[1];
+        const float b[kCW] = {b0.x, b0.y, b0.z, b0.w, b1.x, b1.y, b1.z, b1.w};
 #pragma unroll
         for (int q = 0; q < kRPT; ++q) {
           const float v = small_to_real((x[q] >> (2 * e)) & 3u);
@@ -103,12 +133,14 @@ k_decode_gemm(const uint8_t* __restrict__ codes, uint32_t pitch, int64_t rows, i
         }
       }
     }
-    __syncthreads();
+    __syncthreads();  // the buffer is read before it is refilled
+#pragma unroll
+    for (int q = 0; q < kRPT; ++q) cur[q] = nxt[q];
   }
   float* o = out + (int64_t)blockIdx.y * rows * l;
 #pragma unroll
   for (int q = 0; q < kRPT; ++q) {
-    const int64_t r = r0 + lane + 32 * q;
+    const int64_t r = r0 + 32 * q;
     if (r >= rows) continue;
 #pragma unroll
     for (int c = 0; c < kCW; ++c) {
@@ -125,17 +157,12 @@ __device__ __forceinline__ double code_to_double(uint32_t c) {
   return __hiloint2double((int)__byte_perm(0x00004000u, 0x00003FF0u, c * 0x2200u + 0x1022u), 0);
 }
 
-__device__ __forceinline__ void cp_async8_zfill(double* sdst, const double* gsrc, bool ok) {
-  const uint32_t d = (uint32_t)__cvta_generic_to_shared(sdst);
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(d), "l"(gsrc), "r"(ok ? 8 : 0) : "memory");
-}
-
 // A CTA owns 128 rows, a warp 16 (two row tiles), NT column tiles of 8. A lane's A element of the
 // four codes 4 s .. 4 s + 3 is code lane % 4 of byte s of row lane / 4, so the codes come
 // straight from global memory (16 bytes a row and chunk, the next chunk's in flight) and a
 // decoded value serves NT tensor tiles. B is staged 64 rows at a time in two buffers (8-byte
 // asynchronous copies, row stride 4 mod 16 doubles: conflict-free 4 x 4 reads).
-// Bound by the FP64 pipe for wide B. M = 60000, N = 5000, 10 columns: PLACEHOLDER_DMMA.
+// Bound by the FP64 pipe for wide B. M = 60000, N = 5000, 10 columns: 459 us (689 as FMA tiles).
 constexpr int kDmmaThreads = 256;
 template <int NT>
 __global__ void __launch_bounds__(kDmmaThreads)
@@ -156,7 +183,7 @@ k_decode_dmma(const uint8_t* __restrict__ codes, uint32_t pitch, int64_t rows, i
     for (int t = threadIdx.x; t < kKC * l; t += kDmmaThreads) {
       const int kk = t / l, cc = t - kk * l;
       const bool ok = kk < kv;
-      cp_async8_zfill(dst + kk * LD + cc, ok ? Bc + (int64_t)kk * ldb + cc : B, ok);
+      cp_async_zfill<8>(dst + kk * LD + cc, ok ? Bc + (int64_t)kk * ldb + cc : B, ok);
     }
     asm volatile("cp.async.commit_group;\n" ::: "memory");
   };
@@ -222,7 +249,7 @@ k_decode_dmma(const uint8_t* __restrict__ codes, uint32_t pitch, int64_t rows, i
 // the matching values of B lie in shared memory in the lanes' order ([code of the word][word],
 // 2048 rows of B at a time). A value of B read from shared memory serves kDmvRows rows (at one
 // row a read, shared memory would hold the FP64 pipe to a quarter of its rate); the bound is
-// the integer work of the decode. M = 60001, N = 3000, one column: PLACEHOLDER_DMV.
+// the integer work of the decode. M = 60001, N = 3000, one column: 84 us (449 in the tiled form, 7 of 8 columns padding).
 constexpr int kDmvThreads = 256, kDmvRows = 8, kDmvTile = kDmvThreads / 32 * kDmvRows, kDmvK = 2048;
 template <int L>
 __global__ void __launch_bounds__(kDmvThreads)
@@ -360,8 +387,10 @@ void simt_gemm(pcaone_ctx* c, const uint8_t* codes, uint32_t pitch, int64_t, int
   run_simt(c, codes, pitch, rows, run.cpw, run, B, l, l, ks, out);
 }
 
-// K splits: CTAs for about 16 warps an SM (FP32: 1 to 8 warps a CTA; FP64: 8), each split at least
-// four chunks long; the matrix-vector form takes whole spans of its staged B.
+// K splits: CTAs for about 16 warps an SM (FP32: 1 to 8 warps a CTA; FP64: 8). An FP32 warp's chunk
+// is some 3500 instructions with no other warp to hide behind in a small product, so its
+// splits go down to one chunk; the FP64 ones keep four, the matrix-vector form half a span of its
+// staged B.
 template <typename T>
 int simt_ksplit(pcaone_ctx* c, int64_t rows, int64_t K, int l) {
   const bool dmv = sizeof(T) == 8 && l <= 2;
@@ -369,7 +398,7 @@ int simt_ksplit(pcaone_ctx* c, int64_t rows, int64_t K, int l) {
   const int64_t tiles = (rows + tile - 1) / tile, chunks = (K + kKC - 1) / kKC;
   const int64_t ctas = std::max<int64_t>(2, (dmv ? 32 : 16) / warps);
   const int64_t want = (ctas * c->sm_count + tiles - 1) / tiles;
-  const int64_t ks = std::max<int64_t>(1, std::min<int64_t>(want, chunks / (dmv ? kDmvK / kKC / 2 : 4)));
+  const int64_t ks = std::max<int64_t>(1, std::min<int64_t>(want, chunks / (dmv ? kDmvK / kKC / 2 : sizeof(T) == 8 ? 4 : 1)));
   return (int)std::min<int64_t>(ks, 64);
 }
 void no_omega(pcaone_ctx*, const double*, int, int64_t) {}
