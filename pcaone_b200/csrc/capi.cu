@@ -6,6 +6,7 @@
 #include <random>
 
 #include "internal.hpp"
+#include "linalg.hpp"
 #include "rsvd.hpp"
 
 namespace pg {
@@ -92,22 +93,20 @@ int guarded(pcaone_ctx* c, F&& f) {
 
 namespace {
 
-// U diag(S) (N x k) and V (M x k), both row-major, on the device for the posterior kernels;
-// U and V are column-major host matrices.
-void upload_factors(pcaone_ctx* c, const double* U, const double* S, const double* V, uint32_t k, double** dUS,
-                    double** dV) {
+// U diag(S) (N x k) and V (rows x k), both row-major, into the named device buffers; U, S and V are
+// column-major host matrices, copied as they are and laid out by the device.
+void upload_factors(pcaone_ctx* c, const double* U, const double* S, const double* V, uint64_t rows, uint32_t k,
+                    const char* name_us, const char* name_v, double** dUS, double** dV) {
   PG_REQUIRE(S && V && k >= 1 && k <= (uint32_t)pg::kLmax, PCAONE_EBADARG, "bad factors");
-  std::vector<double> us((size_t)c->N * k), v((size_t)c->M * k);
-  // column by column: sequential reads of the column-major inputs
-  for (uint32_t t = 0; t < k; ++t)
-    for (uint32_t i = 0; i < c->N; ++i) us[(size_t)i * k + t] = U[(size_t)t * c->N + i] * S[t];
-  for (uint32_t t = 0; t < k; ++t)
-    for (uint64_t j = 0; j < c->M; ++j) v[(size_t)j * k + t] = V[(size_t)t * c->M + j];
-  *dUS = (double*)pg::scratch(c, "gl_US", us.size() * 8);
-  *dV = (double*)pg::scratch(c, "gl_V", v.size() * 8);
-  PG_CUDA(cudaMemcpyAsync(*dUS, us.data(), us.size() * 8, cudaMemcpyHostToDevice, c->stream));
-  PG_CUDA(cudaMemcpyAsync(*dV, v.data(), v.size() * 8, cudaMemcpyHostToDevice, c->stream));
-  PG_CUDA(cudaStreamSynchronize(c->stream));
+  const size_t nu = (size_t)c->N * k, nv = (size_t)rows * k;
+  double* cm = (double*)pg::scratch(c, "factors_cm", (nu + nv + k) * 8);
+  *dUS = (double*)pg::scratch(c, name_us, nu * 8);
+  *dV = (double*)pg::scratch(c, name_v, nv * 8);
+  PG_CUDA(cudaMemcpyAsync(cm, U, nu * 8, cudaMemcpyHostToDevice, c->stream));
+  if (nv) PG_CUDA(cudaMemcpyAsync(cm + nu, V, nv * 8, cudaMemcpyHostToDevice, c->stream));
+  PG_CUDA(cudaMemcpyAsync(cm + nu + nv, S, k * 8, cudaMemcpyHostToDevice, c->stream));
+  pg::to_rowmajor(c, cm, c->N, (int)k, c->N, cm + nu + nv, *dUS);
+  pg::to_rowmajor(c, cm + nu, (int64_t)rows, (int)k, (int64_t)rows, nullptr, *dV);
 }
 
 }  // namespace
@@ -353,16 +352,7 @@ int pcaone_gpu_fit_emu(pcaone_ctx* c, const double* U, const double* S, const do
     PG_REQUIRE(c->loaded, PCAONE_ESTATE, "no genotypes loaded");
     PG_REQUIRE(U && S && V && k >= 1 && k <= (uint32_t)kLmax, PCAONE_EBADARG, "bad EMU factors");
     build_missing_by_snp(c);
-    // US = U diag(S), row-major N x k; V row-major M x k
-    std::vector<double> us((size_t)c->N * k), v((size_t)c->M * k);
-    for (uint32_t t = 0; t < k; ++t)  // column by column: sequential reads of the inputs
-      for (uint32_t i = 0; i < c->N; ++i) us[(size_t)i * k + t] = U[(size_t)t * c->N + i] * S[t];
-    for (uint32_t t = 0; t < k; ++t)
-      for (uint64_t j = 0; j < c->M; ++j) v[(size_t)j * k + t] = V[(size_t)t * c->M + j];
-    c->d_imp_US = (double*)scratch(c, "d_imp_US", us.size() * 8);
-    c->d_imp_V = (double*)scratch(c, "d_imp_V", v.size() * 8);
-    PG_CUDA(cudaMemcpyAsync(c->d_imp_US, us.data(), us.size() * 8, cudaMemcpyHostToDevice, c->stream));
-    PG_CUDA(cudaMemcpyAsync(c->d_imp_V, v.data(), v.size() * 8, cudaMemcpyHostToDevice, c->stream));
+    upload_factors(c, U, S, V, c->M, k, "d_imp_US", "d_imp_V", &c->d_imp_US, &c->d_imp_V);
     c->imp_k = (int)k;
     c->imputed_compat = reference_index != 0;
     compute_imputed_snp(c);
@@ -430,27 +420,24 @@ void ld_r2_impl(pcaone_ctx* c, const double* U, uint32_t k, const int64_t* ws, c
     }
     double *dW = nullptr, *dY = nullptr;
     if (U) {
-      // W = Gc^T U (M x k) through the FP64 product path; Y = (2I - U^T U) W on the host
-      std::vector<double> W((size_t)c->M * k), C((size_t)k * k, 0.0), Wr((size_t)c->M * k), Yr((size_t)c->M * k);
-      run_product(c, PCAONE_PREC_FP64, 0, 0, 2, U, (int)k, W.data());
+      // W = Gc^T U (M x k) through the FP64 product path; Y = W (2I - U^T U), all on the device
+      std::vector<double> C((size_t)k * k, 0.0);
       for (uint32_t a = 0; a < k; ++a)
-        for (uint32_t b = 0; b < k; ++b) {
-          double acc = 0;
-          for (uint32_t i = 0; i < c->N; ++i) acc += U[(size_t)a * c->N + i] * U[(size_t)b * c->N + i];
-          C[(size_t)a * k + b] = (a == b ? 2.0 : 0.0) - acc;
+        for (uint32_t b = a; b < k; ++b) {
+          double acc[4] = {0, 0, 0, 0};  // four partial sums break the add-latency chain
+          const double *ua = U + (size_t)a * c->N, *ub = U + (size_t)b * c->N;
+          uint32_t i = 0;
+          for (; i + 4 <= c->N; i += 4)
+            for (int q = 0; q < 4; ++q) acc[q] += ua[i + q] * ub[i + q];
+          for (; i < c->N; ++i) acc[0] += ua[i] * ub[i];
+          C[(size_t)a * k + b] = C[(size_t)b * k + a] = (a == b ? 2.0 : 0.0) - ((acc[0] + acc[1]) + (acc[2] + acc[3]));
         }
-      for (uint64_t j = 0; j < c->M; ++j)
-        for (uint32_t a = 0; a < k; ++a) {
-          Wr[j * k + a] = W[(size_t)a * c->M + j];
-          double acc = 0;
-          for (uint32_t b = 0; b < k; ++b) acc += C[(size_t)a * k + b] * W[(size_t)b * c->M + j];
-          Yr[j * k + a] = acc;
-        }
-      dW = (double*)scratch(c, "ld_W", Wr.size() * 8);
-      dY = (double*)scratch(c, "ld_Y", Yr.size() * 8);
-      PG_CUDA(cudaMemcpyAsync(dW, Wr.data(), Wr.size() * 8, cudaMemcpyHostToDevice, c->stream));
-      PG_CUDA(cudaMemcpyAsync(dY, Yr.data(), Yr.size() * 8, cudaMemcpyHostToDevice, c->stream));
-      PG_CUDA(cudaStreamSynchronize(c->stream));
+      dW = product_t_device(c, U, (int)k);
+      dY = (double*)scratch(c, "ld_Y", (size_t)c->M * k * 8);
+      double* dC = (double*)scratch(c, "ld_C", C.size() * 8);
+      PG_CUDA(cudaMemcpyAsync(dC, C.data(), C.size() * 8, cudaMemcpyHostToDevice, c->stream));
+      rowmat(c, dW, (int)k, dC, (int)k, (int)k, (int64_t)c->M, dY);
+      PG_CUDA(cudaStreamSynchronize(c->stream));  // the host matrix goes out of scope
     }
     int64_t* d_ws = (int64_t*)scratch(c, "ld_ws", std::max<uint64_t>(nwin, 1) * 8);
     int32_t* d_we = (int32_t*)scratch(c, "ld_we", std::max<uint64_t>(nwin, 1) * 4);
@@ -592,17 +579,7 @@ int pcaone_gpu_residuals(pcaone_ctx* c, const double* U, const double* S, const 
     PG_REQUIRE(out && snp0 + nsnp <= c->M, PCAONE_EBADARG, "residual rows out of range");
     PG_REQUIRE(!U || (S && V && k >= 1 && k <= (uint32_t)kLmax), PCAONE_EBADARG, "bad factors");
     double *dUS = nullptr, *dV = nullptr;
-    if (U) {
-      std::vector<double> us((size_t)c->N * k), v((size_t)nsnp * k);
-      for (uint32_t i = 0; i < c->N; ++i)
-        for (uint32_t t = 0; t < k; ++t) us[(size_t)i * k + t] = U[(size_t)t * c->N + i] * S[t];
-      for (uint64_t j = 0; j < nsnp; ++j)
-        for (uint32_t t = 0; t < k; ++t) v[(size_t)j * k + t] = V[(size_t)t * nsnp + j];
-      dUS = (double*)scratch(c, "res_US", us.size() * 8);
-      dV = (double*)scratch(c, "res_V", std::max<size_t>(v.size(), 1) * 8);
-      PG_CUDA(cudaMemcpyAsync(dUS, us.data(), us.size() * 8, cudaMemcpyHostToDevice, c->stream));
-      PG_CUDA(cudaMemcpyAsync(dV, v.data(), v.size() * 8, cudaMemcpyHostToDevice, c->stream));
-    }
+    if (U) upload_factors(c, U, S, V, nsnp, k, "res_US", "res_V", &dUS, &dV);
     float* d_out = (float*)scratch(c, "res_out", std::max<uint64_t>(nsnp, 1) * c->N * 4);
     if (nsnp) residuals(c, dUS, dV, U ? (int)k : 0, snp0, nsnp, d_out);
     if (nsnp) PG_CUDA(cudaMemcpyAsync(out, d_out, nsnp * c->N * 4, cudaMemcpyDeviceToHost, c->stream));
@@ -631,7 +608,7 @@ int pcaone_gpu_gl_update(pcaone_ctx* c, const double* U, const double* S, const 
   return guarded(c, [&] {
     PG_REQUIRE(c->loaded && c->dense, PCAONE_ESTATE, "no likelihoods loaded");
     double *dUS = nullptr, *dV = nullptr;
-    if (U) upload_factors(c, U, S, V, k, &dUS, &dV);
+    if (U) upload_factors(c, U, S, V, c->M, k, "gl_US", "gl_V", &dUS, &dV);
     PG_CUDA(cudaEventRecord(c->ev0, c->stream));
     gl_posterior(c, dUS, dV, U ? (int)k : 0);
     PG_CUDA(cudaEventRecord(c->ev1, c->stream));
@@ -655,7 +632,7 @@ int pcaone_gpu_gl_grm(pcaone_ctx* c, const double* U, const double* S, const dou
     PG_REQUIRE(c->loaded && c->dense && c->d_P, PCAONE_ESTATE, "no likelihoods loaded");
     PG_REQUIRE(U, PCAONE_EBADARG, "the GRM needs the factors U, S, V");
     double *dUS = nullptr, *dV = nullptr;
-    upload_factors(c, U, S, V, k, &dUS, &dV);
+    upload_factors(c, U, S, V, c->M, k, "gl_US", "gl_V", &dUS, &dV);
     gl_grm(c, dUS, dV, (int)k, C, evecs, svals);
   });
 }

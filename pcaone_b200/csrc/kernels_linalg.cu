@@ -321,7 +321,63 @@ __global__ void __launch_bounds__(128) k_rowmat(const double* __restrict__ X, in
   }
 }
 
+// 32 rows x all columns through shared memory, so that both sides are read and written in whole
+// sectors (before, either the reads or the writes of a warp were l doubles apart).
+constexpr int kLayoutRows = 32;
+__global__ void __launch_bounds__(256) k_rowmajor(const double* __restrict__ cm, int64_t n, int l, int64_t npad,
+                                                  const double* __restrict__ scale, double* __restrict__ out,
+                                                  float* __restrict__ outf) {
+  extern __shared__ double tile[];  // l x 33
+  const int64_t i0 = (int64_t)blockIdx.x * kLayoutRows;
+  const int rows = (int)(npad - i0 < kLayoutRows ? npad - i0 : kLayoutRows);
+  for (int t = threadIdx.x; t < l * kLayoutRows; t += 256) {
+    const int j = t >> 5, r = t & 31;
+    const double v = i0 + r < n ? cm[j * n + i0 + r] : 0.0;
+    tile[j * 33 + r] = scale ? v * scale[j] : v;
+  }
+  __syncthreads();
+  for (int t = threadIdx.x; t < rows * l; t += 256) {
+    const int r = t / l, j = t - r * l;
+    const double v = tile[j * 33 + r];
+    out[i0 * l + t] = v;
+    if (outf) outf[i0 * l + t] = (float)v;
+  }
+}
+
+__global__ void __launch_bounds__(256) k_colmajor(const double* __restrict__ X, int64_t n, int l, int ld,
+                                                  double* __restrict__ out) {
+  extern __shared__ double tile[];  // l x 33
+  const int64_t i0 = (int64_t)blockIdx.x * kLayoutRows;
+  const int rows = (int)(n - i0 < kLayoutRows ? n - i0 : kLayoutRows);
+  for (int t = threadIdx.x; t < rows * l; t += 256) {
+    const int r = t / l, j = t - r * l;
+    tile[j * 33 + r] = X[(i0 + r) * ld + j];
+  }
+  __syncthreads();
+  for (int t = threadIdx.x; t < l * kLayoutRows; t += 256) {
+    const int j = t >> 5, r = t & 31;
+    if (r < rows) out[j * n + i0 + r] = tile[j * 33 + r];
+  }
+}
+
 }  // namespace
+
+void to_rowmajor(pcaone_ctx* c, const double* cm, int64_t n, int l, int64_t npad, const double* scale, double* out,
+                 float* outf) {
+  const unsigned grid = (unsigned)((npad + kLayoutRows - 1) / kLayoutRows);
+  if (!grid) return;
+  k_rowmajor<<<grid, 256, (size_t)l * 33 * 8, c->stream>>>(cm, n, l, npad, scale, out, outf);
+  PG_CHECK_LAUNCH();
+  c->launches++;
+}
+
+void to_colmajor(pcaone_ctx* c, const double* X, int64_t n, int l, int ld, double* out) {
+  const unsigned grid = (unsigned)((n + kLayoutRows - 1) / kLayoutRows);
+  if (!grid) return;
+  k_colmajor<<<grid, 256, (size_t)l * 33 * 8, c->stream>>>(X, n, l, ld, out);
+  PG_CHECK_LAUNCH();
+  c->launches++;
+}
 
 unsigned* tall_counter(pcaone_ctx* c) {
   const bool fresh = c->bufs.find("tall_cnt") == c->bufs.end();

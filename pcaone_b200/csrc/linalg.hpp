@@ -44,4 +44,10 @@ void colsum(pcaone_ctx* c, const double* A, int l, int64_t n, double* out);
 // Y (n x kc) = X (n x l) * C[:, :kc] with C l x ldc row-major.
 void rowmat(pcaone_ctx* c, const double* X, int l, const double* C, int ldc, int kc, int64_t n, double* Y);
 
+// Column-major n x l (the hosts' layout) -> row-major npad x l, zero past row n, column j scaled by
+// scale[j] when scale (device) is given, and an optional FP32 copy; and back (row stride ld).
+void to_rowmajor(pcaone_ctx* c, const double* cm, int64_t n, int l, int64_t npad, const double* scale, double* out,
+                 float* outf = nullptr);
+void to_colmajor(pcaone_ctx* c, const double* X, int64_t n, int l, int ld, double* out);
+
 }  // namespace pg

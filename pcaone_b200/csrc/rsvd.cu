@@ -22,28 +22,6 @@
 
 namespace pg {
 
-namespace {
-// Omega column-major N x l (host layout of the reference) -> row-major Npad x l FP64 copy
-// (padding rows zero) and an optional FP32 copy.
-__global__ void k_omega_layout(const double* __restrict__ cm, int64_t N, int l, int64_t npad, double* __restrict__ O,
-                               float* __restrict__ Of) {
-  const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (t >= npad * l) return;
-  const int64_t i = t / l, j = t - i * l;
-  const double v = i < N ? cm[j * N + i] : 0.0;
-  O[t] = v;
-  if (Of) Of[t] = (float)v;
-}
-
-// Row-major n x k (row stride ld) -> column-major n x k.
-__global__ void k_to_colmajor(const double* __restrict__ X, int64_t n, int k, int ld, double* __restrict__ Y) {
-  const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (t >= n * k) return;
-  const int64_t j = t / n, i = t - j * n;
-  Y[t] = X[i * ld + j];
-}
-}  // namespace
-
 // ---------------------------------------------------------------- host helpers
 // One-sided Jacobi SVD of a small square matrix A (n x n, row-major): A = U diag(s) V^T,
 // singular values sorted in decreasing order. U, V row-major n x n.
@@ -174,10 +152,7 @@ struct Engine {
     omega_host(o.seed, o.rand, N, l, cm.data());
     double* d_cm = (double*)scratch(c, "r_omg_cm", cm.size() * 8);
     PG_CUDA(cudaMemcpyAsync(d_cm, cm.data(), cm.size() * 8, cudaMemcpyHostToDevice, c->stream));
-    const int64_t tot = Npad * l;
-    k_omega_layout<<<(unsigned)((tot + 255) / 256), 256, 0, c->stream>>>(d_cm, N, l, Npad, Omg, omg_float());
-    PG_CHECK_LAUNCH();
-    c->launches++;
+    to_rowmajor(c, d_cm, N, l, Npad, nullptr, Omg, omg_float());
     colsum(c, Omg, l, N, wsum);
     PG_CUDA(cudaStreamSynchronize(c->stream));  // the host vector goes out of scope
     gemm.omega_changed(c, Omg, l, Npad);
@@ -190,26 +165,19 @@ struct Engine {
     std::vector<double> cm(X, X + (size_t)N * l);
     double* d_cm = (double*)scratch(c, "r_omg_cm", cm.size() * 8);
     PG_CUDA(cudaMemcpyAsync(d_cm, cm.data(), cm.size() * 8, cudaMemcpyHostToDevice, c->stream));
-    const int64_t tot = Npad * l;
-    k_omega_layout<<<(unsigned)((tot + 255) / 256), 256, 0, c->stream>>>(d_cm, N, l, Npad, Omg, omg_float());
-    PG_CHECK_LAUNCH();
-    c->launches++;
+    to_rowmajor(c, d_cm, N, l, Npad, nullptr, Omg, omg_float());
     colsum(c, Omg, l, N, wsum);
     gemm.omega_changed(c, Omg, l, Npad);
     G = Gbuf[0];
     zero(c, H, Npad * l);
     process_windows(0, c->win.bands, H);
     double* cmaj = (double*)scratch(c, "r_out_cm", (size_t)Npad * l * 8);
-    k_to_colmajor<<<(unsigned)(((int64_t)N * l + 255) / 256), 256, 0, c->stream>>>(H, N, l, l, cmaj);
-    PG_CHECK_LAUNCH();
-    c->launches++;
+    to_colmajor(c, H, N, l, l, cmaj);
     if (Y) PG_CUDA(cudaMemcpyAsync(Y, cmaj, (size_t)N * l * 8, cudaMemcpyDeviceToHost, c->stream));
     PG_CUDA(cudaStreamSynchronize(c->stream));  // cm (host) and Y complete
     if (Gt) {  // Z^T X of every window (G rows, current SNP order), column-major
       double* gm = (double*)scratch(c, "r_out_g", (size_t)M * l * 8);
-      k_to_colmajor<<<(unsigned)((M * l + 255) / 256), 256, 0, c->stream>>>(G, M, l, l, gm);
-      PG_CHECK_LAUNCH();
-      c->launches++;
+      to_colmajor(c, G, M, l, l, gm);
       PG_CUDA(cudaMemcpyAsync(Gt, gm, (size_t)M * l * 8, cudaMemcpyDeviceToHost, c->stream));
       PG_CUDA(cudaStreamSynchronize(c->stream));
     }
@@ -784,8 +752,7 @@ struct Engine {
     // U and V leave the device already column-major (the host layout of the outputs)
     double* cmaj = (double*)scratch(c, "r_out_cm", (size_t)std::max<int64_t>(M, N) * k * 8);
     if (U) {
-      k_to_colmajor<<<(unsigned)(((int64_t)N * k + 255) / 256), 256, 0, c->stream>>>(Ucur, N, k, k, cmaj);
-      PG_CHECK_LAUNCH();
+      to_colmajor(c, Ucur, N, k, k, cmaj);
       PG_CUDA(cudaMemcpyAsync(U, cmaj, (size_t)N * k * 8, cudaMemcpyDeviceToHost, c->stream));
       PG_CUDA(cudaStreamSynchronize(c->stream));
     }
@@ -795,8 +762,7 @@ struct Engine {
       double* Gl = Gbuf[(epochs - 1) & 1];  // G of the last epoch kept; Q_G = G R_G^-1 in place
       trsm_right_upper(c, Gl, Rg, l, M, Gl);
       rowmat(c, Gl, l, Ck, l, k, M, Vd);
-      k_to_colmajor<<<(unsigned)((M * k + 255) / 256), 256, 0, c->stream>>>(Vd, M, k, k, cmaj);
-      PG_CHECK_LAUNCH();
+      to_colmajor(c, Vd, M, k, k, cmaj);
       PG_CUDA(cudaMemcpyAsync(V, cmaj, (size_t)M * k * 8, cudaMemcpyDeviceToHost, c->stream));
       PG_CUDA(cudaStreamSynchronize(c->stream));
     }
@@ -822,71 +788,96 @@ struct Engine {
   }
 };
 
-// One standardised product through the same kernels as the RSVD (single window).
+namespace {
+// A column-major n x l host operand on the device, row-major FP64 (npad rows, zero past n) and,
+// for the FP32 back ends, as T.
 template <typename T>
-void product_t(pcaone_ctx* c, GemmFnT<T> gemm, int transpose, int standardize, int ploidy,
-               const double* B, int l, double* out) {
-  const int N = (int)c->N;
-  const int64_t M = (int64_t)c->M, Npad = c->Npad;
-  auto d = [&](const char* name, size_t n) { return (double*)scratch(c, name, n * sizeof(double)); };
-  double* G = d("r_G", (size_t)c->Mpad * l);
-  double* H = d("r_H", Npad * l);
-  double* Bd = d("r_omg", Npad * l);
-  double* wsum = d("r_wsum", l);
-  double* h0 = d("r_h0", l);
-  T* B2 = (T*)scratch(c, "r_B2", (size_t)round_up(c->win.blocksize, 256) * l * sizeof(T));
-  std::vector<double> rm;
-  if (transpose == 0) {
-    rm.assign((size_t)Npad * l, 0.0);
-    for (int i = 0; i < N; ++i)
-      for (int j = 0; j < l; ++j) rm[(size_t)i * l + j] = B[(size_t)j * N + i];
-    PG_CUDA(cudaMemcpyAsync(Bd, rm.data(), rm.size() * 8, cudaMemcpyHostToDevice, c->stream));
-    T* BT = std::is_same<T, double>::value ? reinterpret_cast<T*>(Bd) : (T*)scratch(c, "r_omgT", Npad * l * sizeof(T));
-    if (!std::is_same<T, double>::value) {
-      std::vector<float> f(rm.begin(), rm.end());
-      PG_CUDA(cudaMemcpyAsync(BT, f.data(), f.size() * 4, cudaMemcpyHostToDevice, c->stream));
-      PG_CUDA(cudaStreamSynchronize(c->stream));
-    }
-    colsum(c, Bd, l, N, wsum);
-    gemm.omega_changed(c, Bd, l, Npad);
-    const int ks = gemm.ksplit(c, M, N, l);
-    T* D1 = (T*)scratch(c, "r_D1", (size_t)ks * M * l * sizeof(T));
-    gemm.p1(c, c->d_bed, c->pitch, 0, M, N, BT, l, ks, D1);
-    EpiP1 p1;
-    p1.start = 0; p1.m = M; p1.l = l; p1.ksplit = ks;
-    p1.F = c->d_F; p1.scale = c->d_scale; p1.wsum = wsum; p1.omega = Bd; p1.miss_ptr = c->d_miss_snp_ptr;
-    p1.miss_idx = c->d_miss_snp_idx; p1.miss_val = c->imputed ? c->d_miss_snp_val : nullptr; p1.G = G;
-    launch_prep<T>(c, p1, D1, B2, h0);
-    rm.resize((size_t)M * l);
-    PG_CUDA(cudaMemcpyAsync(rm.data(), G, rm.size() * 8, cudaMemcpyDeviceToHost, c->stream));
-    PG_CUDA(cudaStreamSynchronize(c->stream));
-    for (int64_t i = 0; i < M; ++i)
-      for (int j = 0; j < l; ++j) out[(size_t)j * M + i] = rm[(size_t)i * l + j];
-  } else {
-    rm.assign((size_t)M * l, 0.0);
-    for (int64_t i = 0; i < M; ++i)
-      for (int j = 0; j < l; ++j) rm[(size_t)i * l + j] = B[(size_t)j * M + i];
-    PG_CUDA(cudaMemcpyAsync(G, rm.data(), rm.size() * 8, cudaMemcpyHostToDevice, c->stream));
-    EpiP1 p1;
-    p1.start = 0; p1.m = M; p1.l = l;
-    p1.F = c->d_F; p1.scale = c->d_scale; p1.G = G;
-    launch_scale_g<T>(c, p1, B2, h0);
-    gemm.b2_ready(c, B2, l, M);
-    const int ks = gemm.ksplit(c, N, M, l);
-    T* D2 = (T*)scratch(c, "r_D2", (size_t)ks * N * l * sizeof(T));
-    gemm.p2(c, c->d_bedT, c->win.pitch, 0, N, M, B2, l, ks, D2);
-    zero(c, H, Npad * l);
-    EpiP2 p2;
-    p2.b0 = 0; p2.b1 = 1; p2.nwin = c->win.bands; p2.n = N; p2.npad = Npad; p2.l = l; p2.ksplit = ks;
-    p2.F = c->d_F; p2.scale = c->d_scale; p2.G = G; p2.h0 = h0; p2.miss_ptr = c->d_miss_ws_ptr;
-    p2.miss_idx = c->d_miss_ws_idx; p2.miss_val = c->imputed ? c->d_miss_ws_val : nullptr; p2.H = H;
-    launch_accum<T>(c, p2, D2);
-    rm.resize((size_t)N * l);
-    PG_CUDA(cudaMemcpyAsync(rm.data(), H, rm.size() * 8, cudaMemcpyDeviceToHost, c->stream));
-    PG_CUDA(cudaStreamSynchronize(c->stream));
-    for (int i = 0; i < N; ++i)
-      for (int j = 0; j < l; ++j) out[(size_t)j * N + i] = rm[(size_t)i * l + j];
+struct Operand {
+  double* d;
+  T* t;
+  Operand(pcaone_ctx* c, const double* host, int64_t n, int64_t npad, int l, const char* name) {
+    double* cm = (double*)scratch(c, "r_omg_cm", (size_t)n * l * 8);
+    PG_CUDA(cudaMemcpyAsync(cm, host, (size_t)n * l * 8, cudaMemcpyHostToDevice, c->stream));
+    d = (double*)scratch(c, name, (size_t)npad * l * 8);
+    constexpr bool f32 = std::is_same<T, float>::value;
+    t = f32 ? (T*)scratch(c, std::string(name) + "T", (size_t)npad * l * sizeof(T)) : reinterpret_cast<T*>(d);
+    to_rowmajor(c, cm, n, l, npad, nullptr, d, f32 ? reinterpret_cast<float*>(t) : nullptr);
   }
+};
+
+void read_colmajor(pcaone_ctx* c, const double* X, int64_t n, int l, double* host) {
+  double* cm = (double*)scratch(c, "r_out_cm", (size_t)n * l * 8);
+  to_colmajor(c, X, n, l, l, cm);
+  PG_CUDA(cudaMemcpyAsync(host, cm, (size_t)n * l * 8, cudaMemcpyDeviceToHost, c->stream));
+  PG_CUDA(cudaStreamSynchronize(c->stream));
+}
+
+// First product and its epilogue over the whole matrix as one window: G = Z^T B (row-major, on the
+// device) and, for a second product, the window operand B2 = s/2 G and h0.
+template <typename T>
+double* first_product(pcaone_ctx* c, const GemmFnT<T>& gemm, const double* B, int l, T* B2, double* h0, bool second) {
+  const int N = (int)c->N;
+  const int64_t M = (int64_t)c->M;
+  double* G = (double*)scratch(c, "r_G", (size_t)c->Mpad * l * 8);
+  double* wsum = (double*)scratch(c, "r_wsum", l * 8);
+  const Operand<T> b(c, B, N, c->Npad, l, "r_omg");
+  colsum(c, b.d, l, N, wsum);
+  gemm.omega_changed(c, b.d, l, c->Npad);
+  const int ks = gemm.ksplit(c, M, N, l);
+  T* D1 = (T*)scratch(c, "r_D1", (size_t)ks * M * l * sizeof(T));
+  gemm.p1(c, c->d_bed, c->pitch, 0, M, N, b.t, l, ks, D1);
+  EpiP1 p1;
+  p1.start = 0; p1.m = M; p1.l = l; p1.ksplit = ks;
+  p1.F = c->d_F; p1.scale = c->d_scale; p1.wsum = wsum; p1.omega = b.d; p1.miss_ptr = c->d_miss_snp_ptr;
+  p1.miss_idx = c->d_miss_snp_idx; p1.miss_val = c->imputed ? c->d_miss_snp_val : nullptr; p1.G = G;
+  if (second && gemm.b2_bt) p1.bt2 = gemm.b2_bt(c, l, &p1.kpad2, &p1.bt_half);
+  if (second && gemm.b2_qmax) p1.qmax = gemm.b2_qmax(c, l);
+  launch_prep<T>(c, p1, D1, B2, h0);
+  if (second && !p1.bt2) gemm.b2_ready(c, B2, l, M);
+  return G;
+}
+
+// Second product and its epilogue: H = Z G for the window operand B2 of G (row-major, on the device).
+template <typename T>
+double* second_product(pcaone_ctx* c, const GemmFnT<T>& gemm, const double* G, int l, const T* B2, const double* h0) {
+  const int N = (int)c->N;
+  const int64_t M = (int64_t)c->M;
+  double* H = (double*)scratch(c, "r_H", (size_t)c->Npad * l * 8);
+  const int ks = gemm.ksplit(c, N, M, l);
+  T* D2 = (T*)scratch(c, "r_D2", (size_t)ks * N * l * sizeof(T));
+  gemm.p2(c, c->d_bedT, c->win.pitch, 0, N, M, B2, l, ks, D2);
+  zero(c, H, (int64_t)c->Npad * l);
+  EpiP2 p2;
+  p2.b0 = 0; p2.b1 = 1; p2.nwin = c->win.bands; p2.n = N; p2.npad = c->Npad; p2.l = l; p2.ksplit = ks;
+  p2.F = c->d_F; p2.scale = c->d_scale; p2.G = G; p2.h0 = h0; p2.miss_ptr = c->d_miss_ws_ptr;
+  p2.miss_idx = c->d_miss_ws_idx; p2.miss_val = c->imputed ? c->d_miss_ws_val : nullptr; p2.H = H;
+  launch_accum<T>(c, p2, D2);
+  return H;
+}
+
+template <typename T>
+T* window_operand(pcaone_ctx* c, int l) {
+  return (T*)scratch(c, "r_B2", (size_t)round_up(c->win.blocksize, 256) * l * sizeof(T));
+}
+}  // namespace
+
+// One standardised product through the same kernels as the RSVD (single window). The host's
+// column-major operands are laid out by device kernels.
+template <typename T>
+void product_t(pcaone_ctx* c, GemmFnT<T> gemm, int transpose, const double* B, int l, double* out) {
+  double* h0 = (double*)scratch(c, "r_h0", l * 8);
+  T* B2 = window_operand<T>(c, l);
+  if (transpose == 0) {
+    read_colmajor(c, first_product<T>(c, gemm, B, l, B2, h0, false), (int64_t)c->M, l, out);
+    return;
+  }
+  const Operand<double> g(c, B, (int64_t)c->M, c->Mpad, l, "r_G");
+  EpiP1 p1;
+  p1.start = 0; p1.m = (int64_t)c->M; p1.l = l;
+  p1.F = c->d_F; p1.scale = c->d_scale; p1.G = g.d;
+  launch_scale_g<T>(c, p1, B2, h0);
+  gemm.b2_ready(c, B2, l, (int64_t)c->M);
+  read_colmajor(c, second_product<T>(c, gemm, g.d, l, B2, h0), c->N, l, out);
 }
 
 // Y = Z (Z^T X) on the device: the first product and its epilogue give G = Z^T X and the
@@ -895,52 +886,10 @@ void product_t(pcaone_ctx* c, GemmFnT<T> gemm, int transpose, int standardize, i
 // src/Arnoldi.cpp:18-46, over the whole matrix as one window).
 template <typename T>
 void gram_t(pcaone_ctx* c, GemmFnT<T> gemm, const double* X, int l, double* Y) {
-  const int N = (int)c->N;
-  const int64_t M = (int64_t)c->M, Npad = c->Npad;
-  auto d = [&](const char* name, size_t n) { return (double*)scratch(c, name, n * sizeof(double)); };
-  double* G = d("r_G", (size_t)c->Mpad * l);
-  double* H = d("r_H", Npad * l);
-  double* Bd = d("r_omg", Npad * l);
-  double* wsum = d("r_wsum", l);
-  double* h0 = d("r_h0", l);
-  T* B2 = (T*)scratch(c, "r_B2", (size_t)round_up(c->win.blocksize, 256) * l * sizeof(T));
-  std::vector<double> rm((size_t)Npad * l, 0.0);
-  for (int i = 0; i < N; ++i)
-    for (int j = 0; j < l; ++j) rm[(size_t)i * l + j] = X[(size_t)j * N + i];
-  PG_CUDA(cudaMemcpyAsync(Bd, rm.data(), rm.size() * 8, cudaMemcpyHostToDevice, c->stream));
-  T* BT = std::is_same<T, double>::value ? reinterpret_cast<T*>(Bd) : (T*)scratch(c, "r_omgT", Npad * l * sizeof(T));
-  std::vector<float> f;
-  if (!std::is_same<T, double>::value) {
-    f.assign(rm.begin(), rm.end());
-    PG_CUDA(cudaMemcpyAsync(BT, f.data(), f.size() * 4, cudaMemcpyHostToDevice, c->stream));
-  }
-  colsum(c, Bd, l, N, wsum);
-  gemm.omega_changed(c, Bd, l, Npad);
-  const int ks1 = gemm.ksplit(c, M, N, l);
-  T* D1 = (T*)scratch(c, "r_D1", (size_t)ks1 * M * l * sizeof(T));
-  gemm.p1(c, c->d_bed, c->pitch, 0, M, N, BT, l, ks1, D1);
-  EpiP1 p1;
-  p1.start = 0; p1.m = M; p1.l = l; p1.ksplit = ks1;
-  p1.F = c->d_F; p1.scale = c->d_scale; p1.wsum = wsum; p1.omega = Bd; p1.miss_ptr = c->d_miss_snp_ptr;
-  p1.miss_idx = c->d_miss_snp_idx; p1.miss_val = c->imputed ? c->d_miss_snp_val : nullptr; p1.G = G;
-  if (gemm.b2_bt) p1.bt2 = gemm.b2_bt(c, l, &p1.kpad2, &p1.bt_half);
-  if (gemm.b2_qmax) p1.qmax = gemm.b2_qmax(c, l);
-  launch_prep<T>(c, p1, D1, B2, h0);
-  if (!p1.bt2) gemm.b2_ready(c, B2, l, M);
-  const int ks2 = gemm.ksplit(c, N, M, l);
-  T* D2 = (T*)scratch(c, "r_D2", (size_t)ks2 * N * l * sizeof(T));
-  gemm.p2(c, c->d_bedT, c->win.pitch, 0, N, M, B2, l, ks2, D2);
-  zero(c, H, Npad * l);
-  EpiP2 p2;
-  p2.b0 = 0; p2.b1 = 1; p2.nwin = c->win.bands; p2.n = N; p2.npad = Npad; p2.l = l; p2.ksplit = ks2;
-  p2.F = c->d_F; p2.scale = c->d_scale; p2.G = G; p2.h0 = h0; p2.miss_ptr = c->d_miss_ws_ptr;
-  p2.miss_idx = c->d_miss_ws_idx; p2.miss_val = c->imputed ? c->d_miss_ws_val : nullptr; p2.H = H;
-  launch_accum<T>(c, p2, D2);
-  rm.resize((size_t)N * l);
-  PG_CUDA(cudaMemcpyAsync(rm.data(), H, rm.size() * 8, cudaMemcpyDeviceToHost, c->stream));
-  PG_CUDA(cudaStreamSynchronize(c->stream));
-  for (int i = 0; i < N; ++i)
-    for (int j = 0; j < l; ++j) Y[(size_t)j * N + i] = rm[(size_t)i * l + j];
+  double* h0 = (double*)scratch(c, "r_h0", l * 8);
+  T* B2 = window_operand<T>(c, l);
+  const double* G = first_product<T>(c, gemm, X, l, B2, h0, true);
+  read_colmajor(c, second_product<T>(c, gemm, G, l, B2, h0), c->N, l, Y);
 }
 
 // The Gram product on streamed genotypes (the out-of-core matvec of ArnoldiOpData::perform_op,
@@ -1011,6 +960,16 @@ void run_gram(pcaone_ctx* c, int precision, int standardize, int ploidy, const d
   }
 }
 
+double* product_t_device(pcaone_ctx* c, const double* B, int l) {
+  PG_REQUIRE(c->loaded && !c->dense && !c->streamed, PCAONE_ESTATE, "products need resident packed genotypes");
+  PG_REQUIRE(B && l >= 1 && l <= kLmax, PCAONE_EBADARG, "bad product operands");
+  build_missing_by_snp(c);
+  compute_scale(c, 0, 2);
+  double* h0 = (double*)scratch(c, "r_h0", l * 8);
+  double* B2 = (double*)scratch(c, "r_B2", round_up(c->M, 256) * l * 8);  // written, not used
+  return first_product<double>(c, gemm_simt_double(), B, l, B2, h0, false);
+}
+
 void run_product(pcaone_ctx* c, int precision, int transpose, int standardize, int ploidy,
                  const double* B, int l, double* out) {
   PG_REQUIRE(c->loaded, PCAONE_ESTATE, "no genotypes loaded");
@@ -1029,14 +988,13 @@ void run_product(pcaone_ctx* c, int precision, int transpose, int standardize, i
   if (c->imputed) compute_imputed_ws(c);
   compute_scale(c, standardize, ploidy);
   if (precision == PCAONE_PREC_FP64) {
-    product_t<double>(c, gemm_simt_double(), transpose, standardize, ploidy, B, l, out);
+    product_t<double>(c, gemm_simt_double(), transpose, B, l, out);
   } else if (precision == PCAONE_PREC_FP32) {
-    product_t<float>(c, gemm_simt_float(), transpose, standardize, ploidy, B, l, out);
+    product_t<float>(c, gemm_simt_float(), transpose, B, l, out);
   } else if (precision == PCAONE_PREC_MIXED || precision == PCAONE_PREC_BF16) {
     PG_REQUIRE(tc_supported(c), PCAONE_ENODEV, "tcgen05 path needs an sm_100 device");
     tc_clear_error(c);
-    product_t<float>(c, precision == PCAONE_PREC_MIXED ? gemm_i8() : gemm_tc(), transpose, standardize, ploidy, B, l,
-                     out);
+    product_t<float>(c, precision == PCAONE_PREC_MIXED ? gemm_i8() : gemm_tc(), transpose, B, l, out);
     tc_check_error(c);
   } else {
     throw Error(PCAONE_EBADARG, "unknown precision");
