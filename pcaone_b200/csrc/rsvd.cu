@@ -311,6 +311,7 @@ struct Engine {
     p2.miss_idx = c->d_miss_ws_idx;
     p2.miss_val = c->imputed ? c->d_miss_ws_val : nullptr;
     p2.miss_w = ws_weights();
+    p2.entries = c->n_missing * (p2.b1 - p2.b0) / p2.nwin;
     p2.H = Ht;
     timed([&] { launch_accum<T>(c, p2, D2); }, 1);
   }
@@ -379,6 +380,7 @@ struct Engine {
     p2.miss_idx = c->d_miss_ws_idx;
     p2.miss_val = c->imputed ? c->d_miss_ws_val : nullptr;
     p2.miss_w = ws_weights();
+    p2.entries = c->n_missing * (p2.b1 - p2.b0) / p2.nwin;
     p2.H = Ht;
     timed([&] { launch_accum<T>(c, p2, D2); }, 1);
   }
@@ -851,6 +853,7 @@ double* second_product(pcaone_ctx* c, const GemmFnT<T>& gemm, const double* G, i
   p2.b0 = 0; p2.b1 = 1; p2.nwin = c->win.bands; p2.n = N; p2.npad = c->Npad; p2.l = l; p2.ksplit = ks;
   p2.F = c->d_F; p2.scale = c->d_scale; p2.G = G; p2.h0 = h0; p2.miss_ptr = c->d_miss_ws_ptr;
   p2.miss_idx = c->d_miss_ws_idx; p2.miss_val = c->imputed ? c->d_miss_ws_val : nullptr; p2.H = H;
+  p2.entries = c->n_missing / p2.nwin;
   launch_accum<T>(c, p2, D2);
   return H;
 }

@@ -104,3 +104,29 @@ def test_simt_window_runs_match_oracle(gpu, precision, tol, N, M, bands, k):
     r = gpu.rsvd(precision=precision, **kw)
     S = O.run_pca(bed, shuffle=False, **kw)[1]
     np.testing.assert_allclose(r.S, S, rtol=tol)
+
+
+@pytest.mark.parametrize("precision", ["mixed", "fp32", "fp64"])
+@pytest.mark.parametrize("N,M,l", [(61, 3000, 8), (300, 900, 20), (777, 4500, 15)])
+def test_products_with_uneven_missing_rates(gpu, precision, N, M, l):
+    """Z B where the samples' missing counts run from none to almost all SNPs: rows summed by one
+    warp, by a whole CTA, and empty ones."""
+    rng = np.random.default_rng(N)
+    bed = random_bed(N, M, seed=N, miss=0.0)
+    codes = O.decode_codes(bed).copy()
+    rate = np.where(np.arange(N) % 5 == 0, 0.0, rng.beta(1, 4, N))
+    rate[3] = 0.99
+    miss = rng.random((M, N)) < rate
+    miss[:, :8] &= np.arange(M)[:, None] % 7 != 0
+    codes = np.where(miss if codes.shape == miss.shape else miss.T, 1, codes).astype(np.uint8)
+    snp_major = codes if codes.shape == (M, N) else codes.T
+    pad = np.zeros((M, (N + 3) // 4 * 4), dtype=np.uint8)
+    pad[:, :N] = snp_major
+    pad = pad.reshape(M, -1, 4)
+    bed = O.Bed(N, M, (pad[:, :, 0] | pad[:, :, 1] << 2 | pad[:, :, 2] << 4 | pad[:, :, 3] << 6).astype(np.uint8))
+    gpu.load_bed(bed.packed, N)
+    Z, _ = O.standardized_from_bed(bed)
+    B = rng.standard_normal((M, l))
+    assert rel_col_err(gpu.product(B, precision=precision), Z @ B) <= TOL[precision]
+    X = rng.standard_normal((N, l))
+    assert rel_col_err(gpu.product_t(X, precision=precision), Z.T @ X) <= TOL[precision]
