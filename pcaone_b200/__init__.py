@@ -276,7 +276,7 @@ def _product(ctx: "GpuContext", B: np.ndarray, transpose: int, precision, standa
     if B.shape[0] != rows_in:
         raise ValueError(f"B must have {rows_in} rows")
     Bc = np.asfortranarray(B)
-    out = np.zeros((rows_out, B.shape[1]), order="F")
+    out = np.empty((rows_out, B.shape[1]), order="F")
     ctx._check(lib().pcaone_gpu_product(ctx._h, precision, transpose, int(standardize), ploidy,
                                         _ptr(Bc), B.shape[1], _ptr(out)))
     return np.ascontiguousarray(out)
@@ -300,7 +300,7 @@ def _gram_product(self, X, precision=PREC_FP64, standardize=True, ploidy=2):
     if X.shape[0] != self.N:
         raise ValueError(f"X must have {self.N} rows")
     Xc = np.asfortranarray(X)
-    Y = np.zeros(X.shape, order="F")
+    Y = np.empty(X.shape, order="F")
     self._check(lib().pcaone_gpu_gram_product(self._h, precision, int(standardize), ploidy, _ptr(Xc),
                                               X.shape[1], _ptr(Y)))
     return np.ascontiguousarray(Y)
@@ -313,7 +313,7 @@ def _residuals(self, U=None, S=None, V=None, snp0=0, nsnp=None):
     """Residual rows (nsnp x nsamples float32) of pcaone_gpu_residuals; V holds the loadings of
     the nsnp SNPs from snp0 (current SNP order); no factors gives the centred genotypes."""
     nsnp = self.M - snp0 if nsnp is None else nsnp
-    out = np.zeros((nsnp, self.N), dtype=np.float32)
+    out = np.empty((nsnp, self.N), dtype=np.float32)
     if U is None:
         self._check(lib().pcaone_gpu_residuals(self._h, None, None, None, 0, snp0, nsnp, _ptr(out)))
     else:
@@ -354,7 +354,7 @@ def _ld_r2(self, ws, we, U=None, f64=False):
     as divide_pos_by_window."""
     ws = np.ascontiguousarray(ws, dtype=np.int64)
     we = np.ascontiguousarray(we, dtype=np.int32)
-    out = np.zeros(int(np.maximum(we - 1, 0).sum()), dtype=np.float64 if f64 else np.float32)
+    out = np.empty(int(np.maximum(we - 1, 0).sum()), dtype=np.float64 if f64 else np.float32)
     Uf = None if U is None else np.asfortranarray(U, dtype=np.float64)
     k = 0 if U is None else U.shape[1]
     fn = lib().pcaone_gpu_ld_r2_f64 if f64 else lib().pcaone_gpu_ld_r2

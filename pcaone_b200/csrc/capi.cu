@@ -8,6 +8,7 @@
 #include "internal.hpp"
 #include "linalg.hpp"
 #include "rsvd.hpp"
+#include "xfer.hpp"
 
 namespace pg {
 
@@ -103,7 +104,7 @@ void upload_factors(pcaone_ctx* c, const double* U, const double* S, const doubl
   *dUS = (double*)pg::scratch(c, name_us, nu * 8);
   *dV = (double*)pg::scratch(c, name_v, nv * 8);
   PG_CUDA(cudaMemcpyAsync(cm, U, nu * 8, cudaMemcpyHostToDevice, c->stream));
-  if (nv) PG_CUDA(cudaMemcpyAsync(cm + nu, V, nv * 8, cudaMemcpyHostToDevice, c->stream));
+  copy_to_device(c, cm + nu, V, nv * 8);
   PG_CUDA(cudaMemcpyAsync(cm + nu + nv, S, k * 8, cudaMemcpyHostToDevice, c->stream));
   pg::to_rowmajor(c, cm, c->N, (int)k, c->N, cm + nu + nv, *dUS);
   pg::to_rowmajor(c, cm + nu, (int64_t)rows, (int)k, (int64_t)rows, nullptr, *dV);
@@ -134,6 +135,7 @@ int pcaone_gpu_create(int device, pcaone_ctx** out) {
     delete c;
     return st;
   }
+  xfer_open(c);
   *out = c;
   return PCAONE_OK;
 }
@@ -145,6 +147,7 @@ int pcaone_gpu_destroy(pcaone_ctx* c) {
   pg::gl_release(c);
   free_all(c);
   pg::stream_free(c);
+  pg::xfer_close(c);
   if (c->ev0) cudaEventDestroy(c->ev0);
   if (c->ev1) cudaEventDestroy(c->ev1);
   if (c->ev_tail) cudaEventDestroy(c->ev_tail);
@@ -176,12 +179,27 @@ int pcaone_gpu_load_bed(pcaone_ctx* c, const uint8_t* packed, uint64_t nsnps, ui
     c->d_F = (double*)scratch(c, "d_F", c->M * 8);
     c->d_F_load = (double*)scratch(c, "d_F_load", c->M * 8);
     c->d_scale = (double*)scratch(c, "d_scale", c->M * 8);
-    PG_CUDA(cudaMemsetAsync(c->d_bed, 0xFF, bytes, c->stream));
-    PG_CUDA(cudaMemcpy2DAsync(c->d_bed, c->pitch, packed, c->bpr, c->bpr, c->M,
-                              cudaMemcpyHostToDevice, c->stream));
-    launch_fix_padding(c);
-    launch_counts(c);
-    PG_CUDA(cudaMemcpyAsync(c->d_F_load, c->d_F, c->M * 8, cudaMemcpyDeviceToDevice, c->stream));
+    PG_CUDA(cudaMemsetAsync(c->d_bed + c->M * c->pitch, 0xFF, (c->Mpad - c->M) * c->pitch, c->stream));
+    // the records as they lie in the file, to a staging area from which k_unpack writes the rows
+    const size_t raw = (size_t)c->M * c->bpr;
+    if (raw < kXferMin || c->bpr > kXferSlot) {
+      uint8_t* stage = (uint8_t*)scratch(c, "bed_stage", raw + 8);
+      PG_CUDA(cudaMemcpyAsync(stage, packed, raw, cudaMemcpyHostToDevice, c->stream));
+      launch_unpack(c, c->stream, stage, 0, c->M);
+      c->launches++;
+    } else {
+      constexpr size_t slot_pad = kXferSlot + 256;
+      uint8_t* stage = (uint8_t*)scratch(c, "bed_stage", (size_t)xfer_workers() * slot_pad);
+      const uint64_t rows = kXferSlot / c->bpr;
+      const int64_t chunks = (int64_t)((c->M + rows - 1) / rows);
+      xfer_chunks(c, chunks, [&](int64_t i, int t, char* slot, cudaStream_t st) {
+        const uint64_t j0 = (uint64_t)i * rows, n = std::min(rows, c->M - j0);
+        std::memcpy(slot, packed + j0 * c->bpr, n * c->bpr);
+        PG_CUDA(cudaMemcpyAsync(stage + t * slot_pad, slot, n * c->bpr, cudaMemcpyHostToDevice, st));
+        launch_unpack(c, st, stage + t * slot_pad, j0, n);
+      });
+      c->launches += chunks;
+    }
     PG_CUDA(cudaStreamSynchronize(c->stream));
     c->loaded = true;
   });
@@ -413,9 +431,7 @@ void ld_r2_impl(pcaone_ctx* c, const double* U, uint32_t k, const int64_t* ws, c
         PG_CUDA(cudaMemcpyAsync(d_off, off.data(), (nwin + 1) * 8, cudaMemcpyHostToDevice, c->stream));
         ld_r2_dense(c, c->d_dense_norm, d_win_of, d_we, d_off, d_span, max_span, d_r2, f64);
       }
-      if (off[nwin] > 0)
-        PG_CUDA(cudaMemcpyAsync(r2, d_r2, off[nwin] * esz, cudaMemcpyDeviceToHost, c->stream));
-      PG_CUDA(cudaStreamSynchronize(c->stream));
+      copy_to_host(c, r2, d_r2, (size_t)off[nwin] * esz);
       return;
     }
     double *dW = nullptr, *dY = nullptr;
@@ -460,9 +476,7 @@ void ld_r2_impl(pcaone_ctx* c, const double* U, uint32_t k, const int64_t* ws, c
     } else {
       ld_r2(c, dW, dY, U ? (int)k : 0, d_ws, d_we, d_off, (int64_t)nwin, d_r2, f64);
     }
-    if (off[nwin] > 0)
-      PG_CUDA(cudaMemcpyAsync(r2, d_r2, off[nwin] * esz, cudaMemcpyDeviceToHost, c->stream));
-    PG_CUDA(cudaStreamSynchronize(c->stream));
+    copy_to_host(c, r2, d_r2, (size_t)off[nwin] * esz);
   }
 }
 }  // namespace
@@ -515,7 +529,7 @@ void load_gl_impl(pcaone_ctx* c, const T* P, uint64_t nsnps, uint32_t nsamples) 
   // updates amplify FP32 rounding of the likelihoods to about 1e-6 of the singular values
   c->d_P = (double*)scratch(c, "d_P", np * 8);
   if (std::is_same<T, double>::value)
-    PG_CUDA(cudaMemcpyAsync(c->d_P, P, np * 8, cudaMemcpyHostToDevice, c->stream));
+    copy_to_device(c, c->d_P, P, np * 8);
   else
     gl_widen_f32(c, reinterpret_cast<const float*>(P), np, c->d_P);
   c->d_E = (float*)scratch(c, "d_E", (size_t)c->Mpad * c->Npad * 4);
@@ -582,8 +596,7 @@ int pcaone_gpu_residuals(pcaone_ctx* c, const double* U, const double* S, const 
     if (U) upload_factors(c, U, S, V, nsnp, k, "res_US", "res_V", &dUS, &dV);
     float* d_out = (float*)scratch(c, "res_out", std::max<uint64_t>(nsnp, 1) * c->N * 4);
     if (nsnp) residuals(c, dUS, dV, U ? (int)k : 0, snp0, nsnp, d_out);
-    if (nsnp) PG_CUDA(cudaMemcpyAsync(out, d_out, nsnp * c->N * 4, cudaMemcpyDeviceToHost, c->stream));
-    PG_CUDA(cudaStreamSynchronize(c->stream));
+    copy_to_host(c, out, d_out, (size_t)nsnp * c->N * 4);
   });
 }
 

@@ -184,6 +184,8 @@ struct pcaone_ctx {
   void* h_pin = nullptr;
   size_t h_pin_bytes = 0;
   cudaEvent_t ev_tail = nullptr;
+  // streams of the large host copies' workers (xfer.cu)
+  std::vector<cudaStream_t> xfer_streams;
   double gemm_ms_accum = 0.0;
   int64_t launches = 0, gemm_launches = 0;
 };
@@ -194,7 +196,9 @@ void* scratch(pcaone_ctx* c, const std::string& name, size_t bytes);
 void free_all(pcaone_ctx* c);
 
 // ---------------------------------------------------------------- bed kernels (kernels_bed.cu)
-void launch_fix_padding(pcaone_ctx* c);
+// Raw records (bpr bytes each, back to back at src, which is readable for 8 bytes past its end) of
+// the SNPs j0 .. j0 + n - 1 -> padded rows of d_bed, with their counts and frequencies.
+void launch_unpack(pcaone_ctx* c, cudaStream_t st, const uint8_t* src, uint64_t j0, uint64_t n);
 void launch_counts(pcaone_ctx* c);
 void launch_permute(pcaone_ctx* c, const int32_t* d_perm, uint8_t* d_out);
 // Window layout: bands windows of ceil(M / bands) SNPs, or of blocksize SNPs when it is set

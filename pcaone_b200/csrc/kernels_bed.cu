@@ -15,13 +15,6 @@ namespace pg {
 
 namespace {
 
-__global__ void k_fix_padding(uint8_t* bed, uint64_t M, uint32_t bpr, uint32_t pitch, uint32_t N) {
-  uint64_t j = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
-  if (j >= M) return;
-  uint32_t r = N & 3u;
-  if (r) bed[j * pitch + bpr - 1] |= (uint8_t)(0xFFu << (2 * r));
-}
-
 // Warp per SNP record. n00 = code 00 (two A1), n10 = code 10 (het), n01 = code 01 (missing).
 __global__ void k_counts(const uint8_t* __restrict__ bed, uint64_t M, uint32_t pitch, uint32_t N,
                          uint32_t* __restrict__ a1x2, uint32_t* __restrict__ nonmiss) {
@@ -56,6 +49,45 @@ __global__ void k_freq(const uint32_t* a1x2, const uint32_t* nonmiss, uint64_t M
   if (j >= M) return;
   uint32_t c = nonmiss[j];
   F[j] = c == 0 ? 0.0 : ((double)a1x2[j] * 0.5) / (double)c;
+}
+
+// Records as they are in the file -> rows of the device pitch (samples past N code 11), with the
+// counts and F of k_counts and k_freq in the same pass. Warp per record, a lane per word of 16
+// codes; records start at any byte, so a word is cut from two aligned ones.
+__global__ void k_unpack(const uint8_t* __restrict__ src, uint64_t n, uint32_t bpr, uint32_t pitch, uint32_t N,
+                         uint8_t* __restrict__ bed, uint32_t* __restrict__ a1x2, uint32_t* __restrict__ nonmiss,
+                         double* __restrict__ F, double* __restrict__ F_load) {
+  const uint64_t j = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
+  const int lane = threadIdx.x & 31;
+  if (j >= n) return;
+  const uint64_t at = (uint64_t)(uintptr_t)src + j * bpr;
+  const uint32_t* base = reinterpret_cast<const uint32_t*>(at & ~uint64_t(3));
+  const uint32_t sh = 8 * (uint32_t)(at & 3);
+  uint32_t* row = reinterpret_cast<uint32_t*>(bed + j * pitch);
+  uint32_t c00 = 0, c10 = 0, c01 = 0;
+  for (uint32_t w = lane; w < pitch / 4; w += 32) {
+    uint32_t x = 0xFFFFFFFFu;
+    if (16 * w < N) {
+      x = __funnelshift_r(__ldg(base + w), __ldg(base + w + 1), sh);
+      if (N - 16 * w < 16) x |= 0xFFFFFFFFu << (2 * (N - 16 * w));
+    }
+    row[w] = x;
+    const uint32_t b0 = x & 0x55555555u, b1 = (x >> 1) & 0x55555555u;
+    c00 += __popc(~(b0 | b1) & 0x55555555u);
+    c10 += __popc(b1 & ~b0);
+    c01 += __popc(b0 & ~b1);
+  }
+  for (int o = 16; o; o >>= 1) {
+    c00 += __shfl_xor_sync(0xffffffffu, c00, o);
+    c10 += __shfl_xor_sync(0xffffffffu, c10, o);
+    c01 += __shfl_xor_sync(0xffffffffu, c01, o);
+  }
+  if (lane == 0) {
+    const uint32_t c = N - c01;
+    a1x2[j] = 2 * c00 + c10;
+    nonmiss[j] = c;
+    F[j] = F_load[j] = c == 0 ? 0.0 : ((double)(2 * c00 + c10) * 0.5) / (double)c;
+  }
 }
 
 // out row j = in row perm[j]; 16-byte copies (pitch is a multiple of 64).
@@ -234,12 +266,11 @@ __global__ void k_fill_missing_rows(const uint8_t* __restrict__ base, uint32_t p
 
 }  // namespace
 
-void launch_fix_padding(pcaone_ctx* c) {
-  if ((c->N & 3u) == 0) return;
-  k_fix_padding<<<(unsigned)((c->M + 255) / 256), 256, 0, c->stream>>>(c->d_bed, c->M, c->bpr,
-                                                                         c->pitch, c->N);
+void launch_unpack(pcaone_ctx* c, cudaStream_t st, const uint8_t* src, uint64_t j0, uint64_t n) {
+  k_unpack<<<(unsigned)((n * 32 + 255) / 256), 256, 0, st>>>(src, n, c->bpr, c->pitch, c->N, c->d_bed + j0 * c->pitch,
+                                                            c->d_a1x2 + j0, c->d_nonmiss + j0, c->d_F + j0,
+                                                            c->d_F_load + j0);
   PG_CHECK_LAUNCH();
-  c->launches++;
 }
 
 void launch_counts(pcaone_ctx* c) {

@@ -24,6 +24,7 @@
 #include "internal.hpp"
 #include "rsvd.hpp"
 #include "tall.hpp"
+#include "xfer.hpp"
 
 namespace pg {
 
@@ -651,16 +652,25 @@ __global__ void k_widen(const float* __restrict__ in, size_t n, double* __restri
 }
 
 void gl_widen_f32(pcaone_ctx* c, const float* P, size_t n, double* dP) {
-  const size_t chunk = size_t(16) << 20;  // floats per staging pass (64 MB)
-  float* stage = (float*)scratch(c, "gl_stage", std::min(n, chunk) * 4);
-  for (size_t a = 0; a < n; a += chunk) {
-    const size_t m = std::min(chunk, n - a);
-    PG_CUDA(cudaMemcpyAsync(stage, P + a, m * 4, cudaMemcpyHostToDevice, c->stream));
-    const unsigned nblk = (unsigned)std::min<size_t>(4 * (size_t)c->sm_count, (m + 255) / 256);
-    k_widen<<<nblk, 256, 0, c->stream>>>(stage, m, dP + a);
+  constexpr size_t chunk = kXferSlot / 4;  // floats
+  float* stage = (float*)scratch(c, "gl_stage", (size_t)xfer_workers() * kXferSlot);
+  if (n <= chunk) {
+    PG_CUDA(cudaMemcpyAsync(stage, P, n * 4, cudaMemcpyHostToDevice, c->stream));
+    k_widen<<<(unsigned)((n + 2047) / 2048), 256, 0, c->stream>>>(stage, n, dP);
     PG_CHECK_LAUNCH();
     c->launches++;
+    return;
   }
+  const int64_t chunks = (int64_t)((n + chunk - 1) / chunk);
+  xfer_chunks(c, chunks, [&](int64_t i, int t, char* slot, cudaStream_t st) {
+    const size_t o = (size_t)i * chunk, m = std::min(chunk, n - o);
+    float* dst = stage + (size_t)t * chunk;
+    std::memcpy(slot, P + o, m * 4);
+    PG_CUDA(cudaMemcpyAsync(dst, slot, m * 4, cudaMemcpyHostToDevice, st));
+    k_widen<<<(unsigned)((m + 2047) / 2048), 256, 0, st>>>(dst, m, dP + o);
+    PG_CHECK_LAUNCH();
+  });
+  c->launches += chunks;
 }
 
 void gl_from_bed(pcaone_ctx* c) {
@@ -774,7 +784,7 @@ void gl_grm(pcaone_ctx* c, const double* US, const double* V, int k, double* C, 
       L, nsplit, dpart, nsl, N, (double)M, dC);
   PG_CHECK_LAUNCH();
   c->launches++;
-  if (C) PG_CUDA(cudaMemcpyAsync(C, dC, n2 * 8, cudaMemcpyDeviceToHost, c->stream));
+  if (C) copy_to_host(c, C, dC, n2 * 8);
   if (evecs || svals) {
     // singular vectors of the symmetric C (JacobiSVD in the reference, src/Halko.cpp:328):
     // eigenvectors ordered by decreasing |eigenvalue|
@@ -797,7 +807,7 @@ void gl_grm(pcaone_ctx* c, const double* US, const double* V, int k, double* C, 
     int hinfo = 0;
     PG_CUDA(cudaMemcpyAsync(w.data(), W, (size_t)N * 8, cudaMemcpyDeviceToHost, c->stream));
     PG_CUDA(cudaMemcpyAsync(&hinfo, info, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
-    if (evecs) PG_CUDA(cudaMemcpyAsync(vec.data(), dC, n2 * 8, cudaMemcpyDeviceToHost, c->stream));
+    if (evecs) copy_to_host(c, vec.data(), dC, n2 * 8);
     PG_CUDA(cudaStreamSynchronize(c->stream));
     PG_REQUIRE(hinfo == 0, PCAONE_ENUMERIC, "eigendecomposition of the PCAngsd GRM failed (info " +
                                                 std::to_string(hinfo) + ")");

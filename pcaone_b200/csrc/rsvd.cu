@@ -19,6 +19,7 @@
 #include "linalg.hpp"
 #include "rsvd.hpp"
 #include "update.hpp"
+#include "xfer.hpp"
 
 namespace pg {
 
@@ -178,8 +179,7 @@ struct Engine {
     if (Gt) {  // Z^T X of every window (G rows, current SNP order), column-major
       double* gm = (double*)scratch(c, "r_out_g", (size_t)M * l * 8);
       to_colmajor(c, G, M, l, l, gm);
-      PG_CUDA(cudaMemcpyAsync(Gt, gm, (size_t)M * l * 8, cudaMemcpyDeviceToHost, c->stream));
-      PG_CUDA(cudaStreamSynchronize(c->stream));
+      copy_to_host(c, Gt, gm, (size_t)M * l * 8);
     }
   }
 
@@ -755,8 +755,7 @@ struct Engine {
     double* cmaj = (double*)scratch(c, "r_out_cm", (size_t)std::max<int64_t>(M, N) * k * 8);
     if (U) {
       to_colmajor(c, Ucur, N, k, k, cmaj);
-      PG_CUDA(cudaMemcpyAsync(U, cmaj, (size_t)N * k * 8, cudaMemcpyDeviceToHost, c->stream));
-      PG_CUDA(cudaStreamSynchronize(c->stream));
+      copy_to_host(c, U, cmaj, (size_t)N * k * 8);
     }
     if (V) {
       double* Vd = (double*)scratch(c, "r_V", (size_t)c->Mpad * k * 8);
@@ -765,8 +764,7 @@ struct Engine {
       trsm_right_upper(c, Gl, Rg, l, M, Gl);
       rowmat(c, Gl, l, Ck, l, k, M, Vd);
       to_colmajor(c, Vd, M, k, k, cmaj);
-      PG_CUDA(cudaMemcpyAsync(V, cmaj, (size_t)M * k * 8, cudaMemcpyDeviceToHost, c->stream));
-      PG_CUDA(cudaStreamSynchronize(c->stream));
+      copy_to_host(c, V, cmaj, (size_t)M * k * 8);
     }
     if (rep) {
       rep->epochs = epochs;
@@ -810,8 +808,7 @@ struct Operand {
 void read_colmajor(pcaone_ctx* c, const double* X, int64_t n, int l, double* host) {
   double* cm = (double*)scratch(c, "r_out_cm", (size_t)n * l * 8);
   to_colmajor(c, X, n, l, l, cm);
-  PG_CUDA(cudaMemcpyAsync(host, cm, (size_t)n * l * 8, cudaMemcpyDeviceToHost, c->stream));
-  PG_CUDA(cudaStreamSynchronize(c->stream));
+  copy_to_host(c, host, cm, (size_t)n * l * 8);
 }
 
 // First product and its epilogue over the whole matrix as one window: G = Z^T B (row-major, on the

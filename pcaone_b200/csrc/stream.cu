@@ -217,7 +217,7 @@ void stream_load(pcaone_ctx* c, const uint8_t* packed, size_t slot_bytes) {
     c->h_bed_bytes = bytes;
   }
   if (!c->copy_stream) PG_CUDA(cudaStreamCreateWithFlags(&c->copy_stream, cudaStreamNonBlocking));
-  // records at the device pitch, padding codes 11 past the samples (as k_fix_padding sets
+  // records at the device pitch, padding codes 11 past the samples (as k_unpack sets
   // them in the resident copy), copied by a few host threads
   const uint32_t bpr = c->bpr, pitch = c->pitch, r = c->N & 3u;
   const uint8_t last_or = r ? (uint8_t)(0xFFu << (2 * r)) : 0;
