@@ -49,6 +49,7 @@ struct EpiP2 {          // after the Z * G product of one window or of a run of 
   const double* miss_w = nullptr;    // when set: per-entry weights s_j (e_ij + F_j) (replaces the
                                      // per-entry gathers of s and F)
   int64_t entries = 0;               // about the missing entries of the windows (all of them evenly spread)
+  unsigned long long* qmax_clear = nullptr;  // when set: kLmax values to zero (the run's EpiP1::qmax, used up)
   double* H = nullptr;               // Npad x l accumulator
 };
 

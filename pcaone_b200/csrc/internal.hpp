@@ -165,6 +165,7 @@ struct pcaone_ctx {
   void* tile81_ptr = nullptr;
   void* tile82_ptr = nullptr;
   bool i8_b2_max_ready = false;  // the first epilogue filled the window operand's column maxima
+  bool i8_qmax_clear = false;    // those maxima are zero again once the work queued so far is done
 
   // cuSOLVER handle of the PCAngsd GRM's N x N eigendecomposition (created on first use)
   void* solver = nullptr;

@@ -14,11 +14,38 @@
 //   H_i = (R B2)_i - h0 + sum_{j miss} s_j (e_ij + F_j) G_j,  B2_j = s_j/2 G_j,
 //                                                             h0 = sum_j s_j F_j G_j
 #include "epilogue.hpp"
+#include "linalg.hpp"
+#include "tall.hpp"
 #include "tc_layout.hpp"
 
 namespace pg {
 
 namespace {
+
+// The CTA that finishes last sums the CTAs' partials part[b][c] into out[c]: thread t takes column
+// t % l of the partials t / l, t / l + T / l, ... (T = l (256 / l) threads), the threads of a column
+// combine in order (deterministic). red: 256 doubles of shared memory.
+__device__ __forceinline__ void reduce_parts(const double* part, int l, double* out, unsigned* counter, double* red) {
+  if (!last_cta(counter)) return;
+  const int per = blockDim.x / l, c = threadIdx.x % l, q = threadIdx.x / l;
+  double s = 0.0;
+  if (q < per) {
+    int b = q;
+    for (; b + 3 * per < (int)gridDim.x; b += 4 * per) {
+      const double v0 = part[(int64_t)b * l + c], v1 = part[(int64_t)(b + per) * l + c];
+      const double v2 = part[(int64_t)(b + 2 * per) * l + c], v3 = part[(int64_t)(b + 3 * per) * l + c];
+      s += (v0 + v1) + (v2 + v3);
+    }
+    for (; b < (int)gridDim.x; b += per) s += part[(int64_t)b * l + c];
+  }
+  red[threadIdx.x] = s;
+  __syncthreads();
+  for (int j = threadIdx.x; j < l; j += blockDim.x) {
+    double t = 0.0;
+    for (int p = 0; p < per; ++p) t += red[p * l + j];
+    out[j] = t;
+  }
+}
 
 // Warp-cooperative sparse gather: out[c] = sum_{e in [e0, e1)} w_e * rows[idx_e][c] for all
 // c < l. The warp loads 32 entries (index and weight) at once; then four 8-lane groups each
@@ -182,8 +209,8 @@ __device__ __forceinline__ void sum_rows(int64_t e0, int64_t e1, const int32_t* 
 // l % 4 == 0), 2 = weighted float4 row sums (imputed values, FP32 rows, l % 4 == 0).
 template <typename T, int CPL, int kMode>
 __global__ void __launch_bounds__(256, CPL <= 5 ? 3 : 2) k_prep(EpiP1 p, const T* __restrict__ D1, T* __restrict__ B2,
-                       double* __restrict__ h0_part) {
-  extern __shared__ double sh0[];  // warps x l partial h0, then warps x l sparse sums
+                       double* h0_part, double* __restrict__ h0, unsigned* counter) {
+  extern __shared__ double sh0[];  // warps x l partial h0, then warps x l sparse sums; the reduction's 256
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
   double* ssp = sh0 + nwarps * p.l + warp * p.l;
   unsigned long long* smax = (unsigned long long*)(sh0 + 2 * nwarps * p.l);  // l column maxima
@@ -249,14 +276,15 @@ __global__ void __launch_bounds__(256, CPL <= 5 ? 3 : 2) k_prep(EpiP1 p, const T
     h0_part[(int64_t)blockIdx.x * p.l + c] = acc;
     if (p.qmax && smax[c]) atomicMax(&p.qmax[c], smax[c]);
   }
+  reduce_parts(h0_part, p.l, h0, counter, sh0);
 }
 
 // B2_j = s_j/2 G_j and per-CTA partials of h0 = sum_j s_j F_j G_j, for a given G.
 template <typename T>
 __global__ void k_scale_g(int64_t start, int64_t m, int l, const double* __restrict__ scale,
                           const double* __restrict__ F, const double* __restrict__ G,
-                          T* __restrict__ B2, double* __restrict__ h0_part) {
-  extern __shared__ double sh0[];
+                          T* __restrict__ B2, double* h0_part, double* __restrict__ h0, unsigned* counter) {
+  extern __shared__ double sh0[];  // warps x l partial h0; the reduction's 256
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
   for (int c = lane; c < l; c += 32) sh0[warp * l + c] = 0.0;
   for (int64_t jl = (int64_t)blockIdx.x * nwarps + warp; jl < m; jl += (int64_t)gridDim.x * nwarps) {
@@ -274,34 +302,7 @@ __global__ void k_scale_g(int64_t start, int64_t m, int l, const double* __restr
     for (int w = 0; w < nwarps; ++w) acc += sh0[w * l + c];
     h0_part[(int64_t)blockIdx.x * l + c] = acc;
   }
-}
-
-// out[c] = sum_b part[b][c]: one CTA of kRedThreads per column; thread t sums the rows
-// t, t + kRedThreads, ... (eight loads in flight), then a fixed shuffle tree and a fixed
-// combination of the warps' sums (deterministic).
-constexpr int kRedThreads = 128;
-__global__ void __launch_bounds__(kRedThreads) k_reduce_cols(const double* __restrict__ part, int nblk, int l,
-                                                             double* __restrict__ out) {
-  __shared__ double ws[kRedThreads / 32];
-  const int c = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  double v[8];
-#pragma unroll
-  for (int u = 0; u < 8; ++u) {
-    const int b = threadIdx.x + u * kRedThreads;
-    v[u] = b < nblk ? part[(int64_t)b * l + c] : 0.0;
-  }
-  double t = 0.0;
-#pragma unroll
-  for (int u = 0; u < 8; ++u) t += v[u];
-  for (int b = threadIdx.x + 8 * kRedThreads; b < nblk; b += kRedThreads) t += part[(int64_t)b * l + c];
-  for (int o = 16; o; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
-  if (lane == 0) ws[warp] = t;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    double acc = 0.0;
-    for (int w = 0; w < kRedThreads / 32; ++w) acc += ws[w];
-    out[c] = acc;
-  }
+  reduce_parts(h0_part, l, h0, counter, sh0);
 }
 
 // H[i] += sum_split D2 - h0 + sparse, the sparse term over the sample's missing entries in the
@@ -329,6 +330,7 @@ __global__ void __launch_bounds__(256, CPL <= 5 ? 3 : 2) k_accum(EpiP2 p, const 
       gather_rows<CPL>(e0, e1, p.miss_idx, p.G, 0, p.l, w, out);
   };
   const int slot = warp / wpr, sub = warp - slot * wpr;
+  if (p.qmax_clear && blockIdx.x == 0 && threadIdx.x < kLmax) p.qmax_clear[threadIdx.x] = 0ull;
   for (int64_t i0 = (int64_t)blockIdx.x * rows; i0 < p.n; i0 += (int64_t)gridDim.x * rows) {
     const int64_t i = i0 + slot;
     if (i < p.n) {
@@ -364,16 +366,14 @@ int resident_ctas(const void* fn, int threads, size_t smem) {
 template <typename T>
 void launch_prep(pcaone_ctx* c, const EpiP1& p, const T* D1, T* B2, double* h0) {
   const int threads = 256, nwarps = threads / 32;
-  const size_t smem = (size_t)2 * nwarps * p.l * 8 + (size_t)p.l * 8;
+  const size_t smem = std::max<size_t>((size_t)2 * nwarps * p.l * 8 + (size_t)p.l * 8, threads * 8);
   const int mode = (p.omega_f && (p.l & 3) == 0) ? (p.miss_val ? 2 : 1) : 0;
   auto go = [&](auto kern) {
     const int per_sm = resident_ctas((const void*)kern, threads, smem);
     const int nblk = (int)std::min<int64_t>((int64_t)per_sm * c->sm_count,
                                             std::max<int64_t>(1, (p.m + nwarps - 1) / nwarps));
     double* part = (double*)scratch(c, "h0_part", (size_t)nblk * p.l * 8);
-    kern<<<nblk, threads, smem, c->stream>>>(p, D1, B2, part);
-    PG_CHECK_LAUNCH();
-    k_reduce_cols<<<p.l, kRedThreads, 0, c->stream>>>(part, nblk, p.l, h0);
+    kern<<<nblk, threads, smem, c->stream>>>(p, D1, B2, part, h0, tall_counter(c));
   };
   switch ((p.l + 7) / 8) {
     case 1: mode == 1 ? go(k_prep<T, 1, 1>) : mode == 2 ? go(k_prep<T, 1, 2>) : go(k_prep<T, 1, 0>); break;
@@ -386,7 +386,7 @@ void launch_prep(pcaone_ctx* c, const EpiP1& p, const T* D1, T* B2, double* h0) 
     default: mode == 1 ? go(k_prep<T, 8, 1>) : mode == 2 ? go(k_prep<T, 8, 2>) : go(k_prep<T, 8, 0>); break;
   }
   PG_CHECK_LAUNCH();
-  c->launches += 2;
+  c->launches++;
 }
 
 template <typename T>
@@ -403,6 +403,7 @@ void launch_accum(pcaone_ctx* c, const EpiP2& p, const T* D2) {
     const int per_sm = resident_ctas((const void*)kern, threads, smem);
     const int nblk = (int)std::min<int64_t>((int64_t)per_sm * c->sm_count, (p.n * wpr + nwarps - 1) / nwarps);
     kern<<<nblk, threads, smem, c->stream>>>(p, D2, wpr);
+    if (p.qmax_clear) c->i8_qmax_clear = true;
   };
   switch ((p.l + 7) / 8) {
     case 1: mode == 1 ? go(k_accum<T, 1, 1>) : mode == 2 ? go(k_accum<T, 1, 2>) : go(k_accum<T, 1, 0>); break;
@@ -423,12 +424,10 @@ void launch_scale_g(pcaone_ctx* c, const EpiP1& p, T* B2, double* h0) {
   const int threads = 256, nwarps = threads / 32;
   int nblk = (int)std::min<int64_t>(4 * c->sm_count, std::max<int64_t>(1, (p.m + nwarps - 1) / nwarps));
   double* part = (double*)scratch(c, "h0_part", (size_t)nblk * p.l * 8);
-  k_scale_g<T><<<nblk, threads, (size_t)nwarps * p.l * 8, c->stream>>>(p.start, p.m, p.l, p.scale,
-                                                                       p.F, p.G, B2, part);
+  const size_t smem = std::max<size_t>((size_t)nwarps * p.l * 8, threads * 8);
+  k_scale_g<T><<<nblk, threads, smem, c->stream>>>(p.start, p.m, p.l, p.scale, p.F, p.G, B2, part, h0, tall_counter(c));
   PG_CHECK_LAUNCH();
-  k_reduce_cols<<<p.l, kRedThreads, 0, c->stream>>>(part, nblk, p.l, h0);
-  PG_CHECK_LAUNCH();
-  c->launches += 2;
+  c->launches++;
 }
 
 void zero(pcaone_ctx* c, double* a, int64_t n) {

@@ -454,27 +454,33 @@ __global__ void k_colmax(const T* __restrict__ X, int64_t K, int l, unsigned lon
 // 16-byte stores. Operand row k is present when it lies in the first wlen rows of its window of
 // kpw rows (windows w = k / kpw) and w * wlen + (k % kpw) < mtot. CTA 0 also writes the 3 x LP
 // scales.
+// Bound by latency on the runs of a small winSVD (13 to 100 CTAs): 512 threads for a chunk, and
+// what depends on the chunk alone (its window, its valid rows) worked out once:
+// N = 5003, M = 80021, l = 20, mean of 133 runs: 7.1 us (13.3).
+constexpr int kQuantThreads = 512;
 template <typename T>
-__global__ void __launch_bounds__(256) k_quant(const T* __restrict__ X, int64_t kpw, int64_t wlen, int64_t mtot,
-                                               int l, int lp, int np, const unsigned long long* __restrict__ qmax,
-                                               int8_t* __restrict__ bq, float* __restrict__ sig) {
+__global__ void __launch_bounds__(kQuantThreads) k_quant(const T* __restrict__ X, int64_t kpw, int64_t wlen,
+                                                         int64_t mtot, int l, int lp, int np,
+                                                         const unsigned long long* __restrict__ qmax,
+                                                         int8_t* __restrict__ bq, float* __restrict__ sig) {
   __shared__ __align__(16) uint8_t img[192 * 128];
   __shared__ PieceTable tab;
-  const int64_t kc = blockIdx.x;
+  const int64_t kc = blockIdx.x, w = kc * kChunk / kpw, r0 = kc * kChunk - w * kpw;  // kpw: whole chunks
+  const int64_t valid = min(wlen, mtot - w * wlen) - r0;
+  const int rows = (int)(valid < 0 ? 0 : valid < kChunk ? valid : kChunk);
   tab.fill(qmax, l, lp, sig, kc == 0);
   uint4* img4 = reinterpret_cast<uint4*>(img);
-  for (int t = threadIdx.x; t < np * 8; t += blockDim.x) img4[t] = make_uint4(0u, 0u, 0u, 0u);
+  for (int t = threadIdx.x; t < np * 8; t += kQuantThreads) img4[t] = make_uint4(0u, 0u, 0u, 0u);
   __syncthreads();
+  const T* Xc = X + kc * kChunk * l;
 #pragma unroll 4
-  for (int e = threadIdx.x; e < kChunk * l; e += blockDim.x) {
-    const int kk = e / l, c = e - kk * l;
-    const int64_t k = kc * kChunk + kk, w = k / kpw, r = k - w * kpw;
-    if (r >= wlen || w * wlen + r >= mtot) continue;
-    tab.put(img, kk, c, lp, (double)X[k * l + c]);
+  for (int e = threadIdx.x; e < rows * l; e += kQuantThreads) {
+    const int kk = e / l;
+    tab.put(img, kk, e - kk * l, lp, (double)Xc[e]);
   }
   __syncthreads();
   uint4* dst = reinterpret_cast<uint4*>(bq + kc * (int64_t)np * 128);
-  for (int t = threadIdx.x; t < np * 8; t += blockDim.x) dst[t] = img4[t];
+  for (int t = threadIdx.x; t < np * 8; t += kQuantThreads) dst[t] = img4[t];
 }
 
 // ------------------------------------------------------------------ host side
@@ -717,6 +723,7 @@ void quantize(pcaone_ctx* c, const T* X, int64_t K, int l, int64_t kpad, const c
   auto* bq = (int8_t*)scratch(c, "i8_bq" + t, (size_t)kpad * np);
   auto* sig = (float*)scratch(c, "i8_sig" + t, 3 * 64 * sizeof(float));
   if (!have_max) {
+    if (t == "2") c->i8_qmax_clear = false;  // filled here, outside the epilogues' cycle
     PG_CUDA(cudaMemsetAsync(qmax, 0, (size_t)l * sizeof(unsigned long long), c->stream));
     const int64_t tot = K * l;
     const int nblk = (int)std::max<int64_t>(1, std::min<int64_t>(2 * c->sm_count, (tot + 1023) / 1024));
@@ -728,7 +735,8 @@ void quantize(pcaone_ctx* c, const T* X, int64_t K, int l, int64_t kpad, const c
     kpw = kpad;
     wlen = mtot = K;
   }
-  k_quant<T><<<(unsigned)(kpad / kChunk), 256, 0, c->stream>>>(X, kpw, wlen, mtot, l, lp, np, qmax, bq, sig);
+  PG_REQUIRE(kpw % kChunk == 0 && kpad % kChunk == 0, PCAONE_EBADARG, "windows must be whole chunks");
+  k_quant<T><<<(unsigned)(kpad / kChunk), kQuantThreads, 0, c->stream>>>(X, kpw, wlen, mtot, l, lp, np, qmax, bq, sig);
   PG_CHECK_LAUNCH();
   c->launches++;
 }
@@ -753,7 +761,9 @@ void i8_b2(pcaone_ctx* c, const float* B2, int l, int64_t m) {
 
 unsigned long long* i8_b2_qmax(pcaone_ctx* c, int) {
   auto* qmax = (unsigned long long*)scratch(c, "i8_qmax2", 64 * sizeof(unsigned long long));
-  PG_CUDA(cudaMemsetAsync(qmax, 0, 64 * sizeof(unsigned long long), c->stream));
+  // the accumulation epilogue of the run before leaves them zero (EpiP2::qmax_clear)
+  if (!c->i8_qmax_clear) PG_CUDA(cudaMemsetAsync(qmax, 0, 64 * sizeof(unsigned long long), c->stream));
+  c->i8_qmax_clear = false;
   c->i8_b2_max_ready = true;
   return qmax;
 }

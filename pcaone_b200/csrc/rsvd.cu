@@ -312,6 +312,7 @@ struct Engine {
     p2.miss_val = c->imputed ? c->d_miss_ws_val : nullptr;
     p2.miss_w = ws_weights();
     p2.entries = c->n_missing * (p2.b1 - p2.b0) / p2.nwin;
+    p2.qmax_clear = p1.qmax;
     p2.H = Ht;
     timed([&] { launch_accum<T>(c, p2, D2); }, 1);
   }
@@ -381,6 +382,7 @@ struct Engine {
     p2.miss_val = c->imputed ? c->d_miss_ws_val : nullptr;
     p2.miss_w = ws_weights();
     p2.entries = c->n_missing * (p2.b1 - p2.b0) / p2.nwin;
+    p2.qmax_clear = p1.qmax;
     p2.H = Ht;
     timed([&] { launch_accum<T>(c, p2, D2); }, 1);
   }

@@ -130,3 +130,19 @@ def test_products_with_uneven_missing_rates(gpu, precision, N, M, l):
     assert rel_col_err(gpu.product(B, precision=precision), Z @ B) <= TOL[precision]
     X = rng.standard_normal((N, l))
     assert rel_col_err(gpu.product_t(X, precision=precision), Z.T @ X) <= TOL[precision]
+
+
+def test_mixed_operand_maxima_across_calls(gpu):
+    """The window operand's column maxima are cleared by the epilogue that used them last: an RSVD, a
+    product with a much larger operand and the RSVD again give the first RSVD's results."""
+    bed = random_bed(333, 2100, seed=8, miss=0.02)
+    gpu.load_bed(bed.packed, bed.N)
+    kw = dict(k=4, svd=2, bands=8, maxp=4, tol=0.0, precision="mixed")
+    a = gpu.rsvd(**kw)
+    B = 1e6 * np.random.default_rng(2).standard_normal((bed.M, 14))
+    gpu.product(B, precision="mixed")
+    gpu.gram_product(1e6 * np.ones((bed.N, 14)), precision="mixed")
+    b = gpu.rsvd(**kw)
+    np.testing.assert_allclose(b.S, a.S, rtol=1e-6)
+    S = O.run_pca(bed, k=4, svd=2, bands=8, maxp=4, tol=0.0, shuffle=False)[1]
+    np.testing.assert_allclose(b.S, S, rtol=1e-6)
