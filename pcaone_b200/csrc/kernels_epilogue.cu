@@ -15,6 +15,7 @@
 //                                                             h0 = sum_j s_j F_j G_j
 #include "epilogue.hpp"
 #include "linalg.hpp"
+#include "pdl.hpp"
 #include "tall.hpp"
 #include "tc_layout.hpp"
 
@@ -214,6 +215,7 @@ __global__ void __launch_bounds__(256, CPL <= 5 ? 3 : 2) k_prep(EpiP1 p, const T
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
   double* ssp = sh0 + nwarps * p.l + warp * p.l;
   unsigned long long* smax = (unsigned long long*)(sh0 + 2 * nwarps * p.l);  // l column maxima
+  pdl_begin();
   for (int c = lane; c < p.l; c += 32) sh0[warp * p.l + c] = 0.0;
   if (p.qmax) {
     for (int c = threadIdx.x; c < p.l; c += blockDim.x) smax[c] = 0ull;
@@ -330,6 +332,7 @@ __global__ void __launch_bounds__(256, CPL <= 5 ? 3 : 2) k_accum(EpiP2 p, const 
       gather_rows<CPL>(e0, e1, p.miss_idx, p.G, 0, p.l, w, out);
   };
   const int slot = warp / wpr, sub = warp - slot * wpr;
+  pdl_begin();
   if (p.qmax_clear && blockIdx.x == 0 && threadIdx.x < kLmax) p.qmax_clear[threadIdx.x] = 0ull;
   for (int64_t i0 = (int64_t)blockIdx.x * rows; i0 < p.n; i0 += (int64_t)gridDim.x * rows) {
     const int64_t i = i0 + slot;
@@ -373,7 +376,7 @@ void launch_prep(pcaone_ctx* c, const EpiP1& p, const T* D1, T* B2, double* h0) 
     const int nblk = (int)std::min<int64_t>((int64_t)per_sm * c->sm_count,
                                             std::max<int64_t>(1, (p.m + nwarps - 1) / nwarps));
     double* part = (double*)scratch(c, "h0_part", (size_t)nblk * p.l * 8);
-    kern<<<nblk, threads, smem, c->stream>>>(p, D1, B2, part, h0, tall_counter(c));
+    launch_pdl(kern, nblk, threads, smem, c->stream, p, D1, B2, part, h0, tall_counter(c));
   };
   switch ((p.l + 7) / 8) {
     case 1: mode == 1 ? go(k_prep<T, 1, 1>) : mode == 2 ? go(k_prep<T, 1, 2>) : go(k_prep<T, 1, 0>); break;
@@ -402,7 +405,7 @@ void launch_accum(pcaone_ctx* c, const EpiP2& p, const T* D2) {
   auto go = [&](auto kern) {
     const int per_sm = resident_ctas((const void*)kern, threads, smem);
     const int nblk = (int)std::min<int64_t>((int64_t)per_sm * c->sm_count, (p.n * wpr + nwarps - 1) / nwarps);
-    kern<<<nblk, threads, smem, c->stream>>>(p, D2, wpr);
+    launch_pdl(kern, nblk, threads, smem, c->stream, p, D2, wpr);
     if (p.qmax_clear) c->i8_qmax_clear = true;
   };
   switch ((p.l + 7) / 8) {

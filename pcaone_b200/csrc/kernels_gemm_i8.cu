@@ -48,6 +48,7 @@
 #include <cstdlib>
 
 #include "internal.hpp"
+#include "pdl.hpp"
 #include "quant.hpp"
 #include "rsvd.hpp"
 #include "tc_ptx.hpp"
@@ -170,8 +171,11 @@ __global__ void __launch_bounds__(kThreads, 1) k_decode_gemm_i8(const __grid_con
     *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  for (int i = threadIdx.x; i < 3 * args.lp; i += blockDim.x) sig_s[i] = args.sig[i];
+  // before the allocation: a CTA that waits here must not hold the tensor memory that a CTA of the
+  // kernel it waits for has yet to allocate on the same SM
+  pdl_begin();
   if (warp == 9) tc::tmem_alloc(smem_u32((const void*)tmem_slot), kTmemCols);
+  for (int i = threadIdx.x; i < 3 * args.lp; i += blockDim.x) sig_s[i] = args.sig[i];
   tc::fence_before();
   __syncthreads();
   tc::fence_after();
@@ -468,6 +472,7 @@ __global__ void __launch_bounds__(kQuantThreads) k_quant(const T* __restrict__ X
   const int64_t kc = blockIdx.x, w = kc * kChunk / kpw, r0 = kc * kChunk - w * kpw;  // kpw: whole chunks
   const int64_t valid = min(wlen, mtot - w * wlen) - r0;
   const int rows = (int)(valid < 0 ? 0 : valid < kChunk ? valid : kChunk);
+  pdl_begin();
   tab.fill(qmax, l, lp, sig, kc == 0);
   uint4* img4 = reinterpret_cast<uint4*>(img);
   for (int t = threadIdx.x; t < np * 8; t += kQuantThreads) img4[t] = make_uint4(0u, 0u, 0u, 0u);
@@ -536,8 +541,7 @@ void launch_np(pcaone_ctx* c, const I8Args& a) {
   static_assert(smem <= 227 * 1024, "shared memory above the per-CTA limit");
   if (c->smem_attr_set.insert((const void*)k_decode_gemm_i8<NP, V>).second)
     PG_CUDA(cudaFuncSetAttribute(k_decode_gemm_i8<NP, V>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  k_decode_gemm_i8<NP, V><<<a.grid, kThreads, smem, c->stream>>>(a);
-  PG_CHECK_LAUNCH();
+  launch_pdl(k_decode_gemm_i8<NP, V>, a.grid, kThreads, smem, c->stream, a);
 }
 
 template <int NP>
@@ -736,8 +740,8 @@ void quantize(pcaone_ctx* c, const T* X, int64_t K, int l, int64_t kpad, const c
     wlen = mtot = K;
   }
   PG_REQUIRE(kpw % kChunk == 0 && kpad % kChunk == 0, PCAONE_EBADARG, "windows must be whole chunks");
-  k_quant<T><<<(unsigned)(kpad / kChunk), kQuantThreads, 0, c->stream>>>(X, kpw, wlen, mtot, l, lp, np, qmax, bq, sig);
-  PG_CHECK_LAUNCH();
+  launch_pdl(k_quant<T>, (unsigned)(kpad / kChunk), kQuantThreads, 0, c->stream, X, kpw, wlen, mtot, l, lp, np, qmax, bq,
+             sig);
   c->launches++;
 }
 

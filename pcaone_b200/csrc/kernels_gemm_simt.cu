@@ -18,6 +18,7 @@
 #include <algorithm>
 
 #include "internal.hpp"
+#include "pdl.hpp"
 #include "rsvd.hpp"
 #include "tall.hpp"
 
@@ -76,6 +77,7 @@ k_decode_gemm(const uint8_t* __restrict__ codes, uint32_t pitch, int64_t rows, i
 #pragma unroll
   for (int q = 0; q < kRPT; ++q) rowp[q] = codes + min(r0 + 32 * q, rows - 1) * (int64_t)pitch;
   for (int t = threadIdx.x; t < 2 * kKC * LDS; t += 32 * G) (&bsm[0][0])[t] = 0.f;  // padded columns stay zero
+  pdl_begin();
   __syncthreads();
   auto issue = [&](int64_t kc, int buf) {
     const int64_t w = kc / run.cpw, k0 = (kc - w * run.cpw) * kKC, kv = run.valid(w) - k0;
@@ -319,7 +321,9 @@ void run_simt(pcaone_ctx* c, const uint8_t* codes, uint32_t pitch, int64_t rows,
               const float* B, int ldb, int l, int ksplit, float* out) {
   const int64_t per = (chunks + ksplit - 1) / ksplit;
   const dim3 grid((unsigned)((rows + kTR - 1) / kTR), (unsigned)ksplit);
-  auto go = [&](auto kern, int G) { kern<<<grid, 32 * G, 0, c->stream>>>(codes, pitch, rows, chunks, run, B, ldb, l, per, out); };
+  auto go = [&](auto kern, int G) {
+    launch_pdl(kern, grid, 32 * G, 0, c->stream, codes, pitch, rows, chunks, run, B, ldb, l, per, out);
+  };
   switch ((l + kCW - 1) / kCW) {
     case 1: go(k_decode_gemm<1>, 1); break;
     case 2: go(k_decode_gemm<2>, 2); break;

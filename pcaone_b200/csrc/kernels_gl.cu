@@ -22,6 +22,7 @@
 #include <vector>
 
 #include "internal.hpp"
+#include "pdl.hpp"
 #include "rsvd.hpp"
 #include "tall.hpp"
 #include "xfer.hpp"
@@ -313,6 +314,7 @@ k_dense_gemm2(const float* __restrict__ A, uint64_t lda, int64_t rows, int64_t K
       if (e < KC * CN) (&bs[buf][0][0])[e] = rb[u];
     }
   };
+  pdl_begin();
   if (kc0 < kc1) {
     load(kc0);
     store(0);
@@ -369,8 +371,7 @@ void launch_dense2(pcaone_ctx* c, const float* A, uint64_t lda, int64_t rows, in
   const int64_t kct = (K + 31) / 32;
   const int64_t per = (kct + ks - 1) / ks;
   dim3 grid((unsigned)((rows + 127) / 128), (unsigned)ks);
-  k_dense_gemm2<AT, CN><<<grid, 256, 0, c->stream>>>(A, lda, rows, K, B, l, per, out);
-  PG_CHECK_LAUNCH();
+  launch_pdl(k_dense_gemm2<AT, CN>, grid, 256, 0, c->stream, A, lda, rows, K, B, l, per, out);
 }
 
 template <bool AT>

@@ -11,6 +11,7 @@
 
 #include <algorithm>
 
+#include "pdl.hpp"
 #include "tall.hpp"
 
 namespace pg {
@@ -49,6 +50,7 @@ __global__ void __cluster_dims__(kTallCluster, 1, 1) __launch_bounds__(kTallThre
   double* red = cpart + NACC * 64;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, q4 = lane >> 2, r4 = lane & 3;
   const int l = a.l, lb = a.lb;
+  pdl_begin();
   if constexpr (PROD) {
     load_square<NT>(a.Rinv, l, 0.0, Rs);
     __syncthreads();
@@ -207,8 +209,7 @@ void launch_tall(pcaone_ctx* c, TallStep s) {
   const int passes = RECT ? 2 : 1;
   s.part = tall_part(c, (size_t)passes * TallCfg<NT, RECT>::kAcc * 64);
   s.counter = tall_counter(c);
-  k_tall<NT, PROD, RECT><<<ncl * kTallCluster, kTallThreads, smem, c->stream>>>(s);
-  PG_CHECK_LAUNCH();
+  launch_pdl(k_tall<NT, PROD, RECT>, ncl * kTallCluster, kTallThreads, smem, c->stream, s);
   c->launches++;
 }
 

@@ -20,6 +20,7 @@
 #include <algorithm>
 
 #include "linalg.hpp"
+#include "pdl.hpp"
 #include "quant.hpp"
 #include "tall.hpp"
 #include "tc_layout.hpp"
@@ -69,6 +70,7 @@ __global__ void __cluster_dims__(kTallCluster, 1, 1) __launch_bounds__(kTallThre
   double* red = cpart + 4 * LT;
   const int l = a.l, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, q4 = lane >> 2, r4 = lane & 3;
   const int ctas = gridDim.x - kTallCluster;
+  pdl_begin();
   load_square<NT>(a.R2i, l, 0.0, Rs);
   for (int t = threadIdx.x; t < 4 * LT; t += kTallThreads) cpart[t] = 0.0;
   __syncthreads();
@@ -163,6 +165,7 @@ __global__ void __launch_bounds__(kApplyThreads) k_apply(UpdateArgs a, const dou
   const int l = a.l, lp = i8_lp(l), np = i8_np(l);
   const int64_t base = (int64_t)blockIdx.x * kI8Chunk;
   const int rows = (int)(a.N - base < kI8Chunk ? (a.N > base ? a.N - base : 0) : kI8Chunk);
+  pdl_begin();
   for (int j = threadIdx.x; j < l; j += kApplyThreads) mult[j] = a.mult[j];
   if (a.i8.bq) {
     tab.fill(a.i8.qmax, l, lp, a.i8.sig, blockIdx.x == 0);
@@ -205,8 +208,7 @@ void launch_flip(pcaone_ctx* c, UpdateArgs a, const double* Q1, double* Q) {
   const int ncl = tall_clusters(a.N, cap - 1) + 1;  // one for the signs
   a.part = tall_part(c, 4 * Tall<NT>::LT);
   a.counter = tall_counter(c);
-  k_flip<NT><<<ncl * kTallCluster, kTallThreads, smem, c->stream>>>(a, Q1, Q);
-  PG_CHECK_LAUNCH();
+  launch_pdl(k_flip<NT>, ncl * kTallCluster, kTallThreads, smem, c->stream, a, Q1, Q);
   c->launches++;
 }
 
@@ -244,8 +246,7 @@ void fused_update(pcaone_ctx* c, UpdateArgs a) {
     default: launch_flip<8>(c, a, Q1, a.Q); break;
   }
   const size_t img = a.i8.bq ? (size_t)i8_np(a.l) * 128 : 0;  // at most 24 KB
-  k_apply<<<(unsigned)(a.kpad / kI8Chunk), kApplyThreads, img, c->stream>>>(a, a.Q);
-  PG_CHECK_LAUNCH();
+  launch_pdl(k_apply, (unsigned)(a.kpad / kI8Chunk), kApplyThreads, img, c->stream, a, a.Q);
   c->launches++;
 }
 
