@@ -158,22 +158,30 @@ __global__ void __cluster_dims__(kTallCluster, 1, 1) __launch_bounds__(kTallThre
   }
   if (!last_cta(a.counter)) return;
 
+  constexpr int kPer = (NACC * 64 + kTallThreads - 1) / kTallThreads;
   if constexpr (RECT) {
-    for (int pass = 0; pass < passes; ++pass)
-      for (int e = threadIdx.x; e < NACC * 64; e += kTallThreads) {
-        const int t = e >> 6, i = t / NB, j = pass * NB + t % NB;
+    for (int pass = 0; pass < passes; ++pass) {
+      double v[kPer];
+      sum_parts<NACC * 64>(a.part + (int64_t)pass * ncl * NACC * 64, ncl, NACC * 64, v);
+#pragma unroll
+      for (int u = 0; u < kPer; ++u) {
+        const int e = threadIdx.x + u * kTallThreads, t = e >> 6, i = t / NB, j = pass * NB + t % NB;
         const int row = 8 * i + ((e & 63) >> 3), col = 8 * j + (e & 7);
-        if (row < l && col < lb)
-          a.X[row * lb + col] = sum_parts(a.part + (int64_t)pass * ncl * NACC * 64 + e, ncl, NACC * 64);
+        if (e < NACC * 64 && row < l && col < lb) a.X[row * lb + col] = v[u];
       }
+    }
   } else {
     double *W = red, *R = W + T::kSq, *X = R + T::kSq, *P = X + T::kSq, *sc = P + T::kSq;
-    for (int e = threadIdx.x; e < NACC * 64; e += kTallThreads) {
-      const double v = sum_parts(a.part + e, ncl, NACC * 64);
+    double v[kPer];
+    sum_parts<NACC * 64>(a.part, ncl, NACC * 64, v);
+#pragma unroll
+    for (int u = 0; u < kPer; ++u) {
+      const int e = threadIdx.x + u * kTallThreads;
       int i = 0, t = e >> 6;
+      if (e >= NACC * 64) break;
       while (t >= NT - i) t -= NT - i++;
       const int row = 8 * i + ((e & 63) >> 3), col = 8 * (i + t) + (e & 7);
-      W[row * LD + col] = (row < l && col < l) ? v : (row == col ? 1.0 : 0.0);
+      W[row * LD + col] = (row < l && col < l) ? v[u] : (row == col ? 1.0 : 0.0);
     }
     if (a.Rprev) load_square<NT>(a.Rprev, l, 1.0, P);
     __syncthreads();

@@ -142,11 +142,20 @@ __global__ void __cluster_dims__(kTallCluster, 1, 1) __launch_bounds__(kTallThre
   cluster_sum(cpart, 4 * LT, 3 * LT, a.part);
   if (!last_cta(a.counter)) return;
   const int ncl = gridDim.x / kTallCluster;
+  double* tot = red;  // the clusters' sums and maxima
+  static_assert(4 * LT <= kTallThreads, "a thread per column statistic");
+  if (threadIdx.x < 4 * LT) {
+    double v = 0.0;
+#pragma unroll 4
+    for (int p = 0; p < ncl; ++p) {
+      const double w = a.part[(int64_t)p * 4 * LT + threadIdx.x];
+      v = (int)threadIdx.x < 3 * LT ? v + w : fmax(v, w);
+    }
+    tot[threadIdx.x] = v;
+  }
+  __syncthreads();
   for (int j = threadIdx.x; j < l; j += kTallThreads) {
-    const double A = sum_parts(a.part + j, ncl, 4 * LT), B = sum_parts(a.part + LT + j, ncl, 4 * LT);
-    const double s = sum_parts(a.part + 2 * LT + j, ncl, 4 * LT);
-    double top = 0.0;
-    for (int p = 0; p < ncl; ++p) top = fmax(top, a.part[(int64_t)p * 4 * LT + 3 * LT + j]);
+    const double A = tot[j], B = tot[LT + j], s = tot[2 * LT + j], top = tot[3 * LT + j];
     const double d = a.D[j];
     const double m = d > 0.0 ? A : B, p = d > 0.0 ? B : A;
     const double f = (m > 2.0 * p) ? -d : d;  // src/RSVD.hpp:85

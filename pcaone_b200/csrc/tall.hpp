@@ -42,7 +42,7 @@ struct Tall {
   static constexpr int LT = 8 * NT, LD = LT + 4;
   static constexpr int kTiles = NT * (NT + 1) / 2;    // tiles on and above the diagonal
   static constexpr int kSq = LT * LD;                 // doubles of an l x l matrix
-  static constexpr int kWarpScratch = kTallWarps * 128;  // two 8 x 8 blocks a warp
+  static constexpr int kWarpScratch = 256 + kTallWarps * 64;  // 8 x 8 blocks of the factorisations
   static __device__ __forceinline__ constexpr int tile(int i, int j) { return i * NT - i * (i - 1) / 2 + (j - i); }
 };
 
@@ -98,91 +98,130 @@ __device__ __forceinline__ void block_store(const double (&d)[2], double* C, int
   *reinterpret_cast<double2*>(C + q * ldc + 2 * r) = make_double2(d[0], d[1]);
 }
 
+// 1 / x for a normal x whose reciprocal is normal, to the last bit or the one before: the hardware's
+// approximation (about 20 bits) and two Newton steps, y += y (1 - x y). The pivots below divide on
+// the dependent chain of the factorisation, where the rounded division is a few hundred cycles.
+__device__ __forceinline__ double fast_reciprocal(double x) {
+  double y;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+  y = fma(y, fma(-x, y, 1.0), y);
+  return fma(y, fma(-x, y, 1.0), y);
+}
+
+// One warp: Cholesky factor R_bb of the symmetric 8 x 8 block Wb (row stride LD) into Rb and its
+// inverse into Xb (upper, zeros below), and the inverse of R_bb^T into Li (8 x 8). Lane r (mod 8)
+// holds row r; a step eliminates one column of the block and of an identity beside it, which ends as
+// the inverse of the unit lower factor; the eight square roots are taken at once, one a lane. A
+// pivot that is not positive, normal and finite is replaced by 1: returns 1 + its index, else 0.
+template <int LD>
+__device__ __forceinline__ int chol_block(const double* Wb, double* Rb, double* Xb, double* Li) {
+  const int lane = threadIdx.x & 31, r8 = lane & 7;
+  double d[8], y[8], own = 1.0;
+  int bad = 0;
+#pragma unroll
+  for (int j = 0; j < 8; ++j) {
+    d[j] = Wb[r8 * LD + j];
+    y[j] = j == r8 ? 1.0 : 0.0;
+  }
+#pragma unroll
+  for (int j = 0; j < 8; ++j) {
+    double p = __shfl_sync(0xffffffffu, d[j], j);
+    if (!(p >= 2.3e-308 && p < 4e307)) {
+      if (!bad) bad = j + 1;
+      p = 1.0;
+    }
+    if (r8 == j) own = p;
+    const double f = r8 > j ? d[j] * fast_reciprocal(p) : 0.0;
+#pragma unroll
+    for (int c = j + 1; c < 8; ++c) d[c] -= f * __shfl_sync(0xffffffffu, d[j], c);
+#pragma unroll
+    for (int c = 0; c <= j; ++c) y[c] -= f * __shfl_sync(0xffffffffu, y[c], j);
+    d[j] = f;
+  }
+  const double root = sqrt(own), iroot = 1.0 / root;
+#pragma unroll
+  for (int j = 0; j < 8; ++j) {
+    const double s = __shfl_sync(0xffffffffu, root, j);
+    d[j] = r8 == j ? s : d[j] * s;
+    y[j] *= iroot;
+  }
+  if (lane < 8) {
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      Rb[j * LD + r8] = d[j];
+      Xb[j * LD + r8] = y[j];
+      Li[r8 * 8 + j] = y[j];
+    }
+  }
+  __syncwarp();
+  return bad;
+}
+
 // Cholesky W = R^T R of the l x l matrix in shared memory (tiles on and above the diagonal read,
 // W overwritten; padded to LT with a unit diagonal) and X = R^-1, both upper with zeros below.
-// Blocks of 8: every warp factors and inverts the diagonal block itself (8 steps in registers:
-// lane r holds row r, columns by shuffle), so a block costs two CTA barriers, then the block
-// row and the trailing tiles are block products spread over the warps. A pivot that is not
-// positive and finite is replaced by 1. Returns 1 + the first such column, else 0 (the same in
-// every thread). sc: kWarpScratch doubles.
+// Blocks of 8: warp 0 factors and inverts the diagonal block (chol_block, 8 steps in registers),
+// the block row and the trailing tiles are block products spread over the warps, and warp 0 goes
+// on from the next diagonal tile to its factor while the others finish the trailing ones, so a
+// block costs its eight dependent steps, one block product and two CTA barriers. Returns 1 + the
+// first column whose pivot was not positive, else 0 (the same in every thread). sc: kWarpScratch
+// doubles.
+// One CTA, cycles for l = 20 / 40: PLACEHOLDER_CHOL (every warp factoring every block itself, rounded
+// reciprocals: 12500 / 21500; the warps' shuffles held one another up).
 template <int NT>
 __device__ __forceinline__ int chol_inverse(double* W, double* R, double* X, double* sc) {
   using T = Tall<NT>;
   constexpr int LD = T::LD;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, r8 = lane & 7;
-  double* my = sc + warp * 128;
-  int bad = 0;
+  const int warp = threadIdx.x >> 5;
+  double* Li = sc;                       // two 8 x 8: of the current and of the next block
+  double* my = sc + 128 + warp * 64;     // kTallWarps x 8 x 8
+  __shared__ int first_bad;
   for (int t = threadIdx.x; t < T::kSq; t += blockDim.x) R[t] = X[t] = 0.0;
+  if (threadIdx.x == 0) first_bad = 0;
   __syncthreads();
-  for (int b = 0; b < NT; ++b) {
-    const double* Wb = W + 8 * b * LD + 8 * b;
-    // unit lower factor first (one reciprocal in a step's dependent chain), then the square roots
-    // of all eight pivots at once, one a lane
-    double d[8], own = 1.0;
-#pragma unroll
-    for (int j = 0; j < 8; ++j) d[j] = Wb[r8 * LD + j];
-#pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      double p = __shfl_sync(0xffffffffu, d[j], j);
-      if (!(p > 0.0) || !isfinite(p)) {
-        if (!bad) bad = 8 * b + j + 1;
-        p = 1.0;
-      }
-      if (r8 == j) own = p;
-      const double f = d[j] * __drcp_rn(p);
-#pragma unroll
-      for (int c = j + 1; c < 8; ++c) d[c] -= f * __shfl_sync(0xffffffffu, d[j], c);
-      d[j] = r8 > j ? f : 0.0;
-    }
-    const double root = sqrt(own), iroot = 1.0 / root;
-    double y[8];  // lane c: column c of the inverse of the lower factor
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      double a = i == r8 ? 1.0 : 0.0;
-#pragma unroll
-      for (int m = 0; m < i; ++m) a -= __shfl_sync(0xffffffffu, d[m], i) * y[m];
-      y[i] = i >= r8 ? a : 0.0;
-    }
-#pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      const double s = __shfl_sync(0xffffffffu, root, j);
-      d[j] = r8 == j ? s : d[j] * s;
-      y[j] *= __shfl_sync(0xffffffffu, iroot, j);
-    }
-    if (lane < 8) {
-#pragma unroll
-      for (int i = 0; i < 8; ++i) my[i * 8 + r8] = y[i];  // inverse of the lower factor
-      if (warp == 0) {
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-          R[(8 * b + j) * LD + 8 * b + r8] = d[j];
-          X[(8 * b + r8) * LD + 8 * b + j] = y[j];
-        }
-      }
-    }
-    __syncwarp();
+  auto factor = [&](int b) {
+    const int o = 8 * b * LD + 8 * b;
+    const int bad = chol_block<LD>(W + o, R + o, X + o, Li + (b & 1) * 64);
+    if (bad && threadIdx.x == 0 && first_bad == 0) first_bad = 8 * b + bad;
+  };
+  if (warp == 0) factor(0);
+  __syncthreads();
+  for (int b = 0; b + 1 < NT; ++b) {
     for (int J = b + 1 + warp; J < NT; J += kTallWarps) {  // block row of R
       double c[2] = {0.0, 0.0};
-      block_mma<false>(c, my, 8, W + 8 * b * LD + 8 * J, LD);
+      block_mma<false>(c, Li + (b & 1) * 64, 8, W + 8 * b * LD + 8 * J, LD);
       block_store(c, R + 8 * b * LD + 8 * J, LD);
     }
     __syncthreads();
-    int t = 0;
-    for (int I = b + 1; I < NT; ++I)
-      for (int J = I; J < NT; ++J, ++t) {
-        if (t % kTallWarps != warp) continue;
-        double c[2];
-        block_load(c, W + 8 * I * LD + 8 * J, LD);
-        block_mma<true>(c, R + 8 * b * LD + 8 * I, LD, R + 8 * b * LD + 8 * J, LD, -1.0);
-        block_store(c, W + 8 * I * LD + 8 * J, LD);
-      }
+    auto trail = [&](int I, int J) {
+      double c[2];
+      block_load(c, W + 8 * I * LD + 8 * J, LD);
+      block_mma<true>(c, R + 8 * b * LD + 8 * I, LD, R + 8 * b * LD + 8 * J, LD, -1.0);
+      block_store(c, W + 8 * I * LD + 8 * J, LD);
+    };
+    if (warp == 0) {
+      trail(b + 1, b + 1);
+      __syncwarp();
+      factor(b + 1);
+    } else {
+      int t = 0;
+      for (int I = b + 1; I < NT; ++I)
+        for (int J = I; J < NT; ++J) {
+          if (I == b + 1 && J == I) continue;
+          if (t++ % (kTallWarps - 1) == warp - 1) trail(I, J);
+        }
+    }
     __syncthreads();
   }
   // block column J of the inverse by warp J: X_IJ = -X_II sum_{I < K <= J} R_IK X_KJ
   for (int J = warp; J < NT; J += kTallWarps)
     for (int I = J - 1; I >= 0; --I) {
-      double c[2] = {0.0, 0.0};
-      for (int K = I + 1; K <= J; ++K) block_mma<false>(c, R + 8 * I * LD + 8 * K, LD, X + 8 * K * LD + 8 * J, LD);
+      double c[2] = {0.0, 0.0}, g[2] = {0.0, 0.0};  // even and odd K apart: two chains of products
+      for (int K = I + 1; K <= J; K += 2) {
+        block_mma<false>(c, R + 8 * I * LD + 8 * K, LD, X + 8 * K * LD + 8 * J, LD);
+        if (K < J) block_mma<false>(g, R + 8 * I * LD + 8 * (K + 1), LD, X + 8 * (K + 1) * LD + 8 * J, LD);
+      }
+      c[0] += g[0];
+      c[1] += g[1];
       block_store(c, my, 8);
       __syncwarp();
       double e[2] = {0.0, 0.0};
@@ -191,7 +230,7 @@ __device__ __forceinline__ int chol_inverse(double* W, double* R, double* X, dou
       __syncwarp();
     }
   __syncthreads();
-  return bad;
+  return first_bad;
 }
 
 // C = A B for upper triangular A, B in shared memory (C may not alias them).
@@ -209,92 +248,116 @@ __device__ __forceinline__ void upper_product(const double* A, const double* B, 
   __syncthreads();
 }
 
+// One warp: modified LU of the 8 x 8 block Tb (row stride LD): step i takes the pivot s = T[i][i],
+// D_i = -sign(s) with sign(0) = +, and eliminates with the shifted pivot u = s - D_i (|u| >= 1).
+// Writes D and the inverses of the two factors (Li unit lower, Ui upper, 8 x 8). Lane r (mod 8)
+// holds row r; the identity beside the block ends as Li, and Ui follows by back substitution.
+template <int LD>
+__device__ __forceinline__ void signs_block(const double* Tb, double* D, double* Li, double* Ui) {
+  const int lane = threadIdx.x & 31, r8 = lane & 7;
+  double t[8], y[8], z[8], ui[8];
+#pragma unroll
+  for (int j = 0; j < 8; ++j) {
+    t[j] = Tb[r8 * LD + j];
+    y[j] = j == r8 ? 1.0 : 0.0;
+  }
+#pragma unroll
+  for (int j = 0; j < 8; ++j) {
+    const double piv = __shfl_sync(0xffffffffu, t[j], j);
+    const double di = piv >= 0.0 ? -1.0 : 1.0;
+    if (lane == 0) D[j] = di;
+    ui[j] = fast_reciprocal(piv - di);
+    const double f = r8 > j ? t[j] * ui[j] : 0.0;
+#pragma unroll
+    for (int c = j + 1; c < 8; ++c) t[c] -= f * __shfl_sync(0xffffffffu, t[c], j);
+#pragma unroll
+    for (int c = 0; c <= j; ++c) y[c] -= f * __shfl_sync(0xffffffffu, y[c], j);
+  }
+#pragma unroll
+  for (int i = 7; i >= 0; --i) {  // lane c: column c of U^-1
+    double a = i == r8 ? 1.0 : 0.0;
+#pragma unroll
+    for (int m = 7; m > i; --m) a -= __shfl_sync(0xffffffffu, t[m], i) * z[m];
+    z[i] = i <= r8 ? a * ui[i] : 0.0;
+  }
+  if (lane < 8) {
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      Li[r8 * 8 + i] = y[i];
+      Ui[i * 8 + r8] = z[i];
+    }
+  }
+  __syncwarp();
+}
+
 // Householder column signs D (LT values, shared memory) of the thin QR whose orthonormal factor
-// has the top l x l block T (shared memory, zero padded, overwritten): modified LU, step i takes
-// the pivot s = T[i][i], D_i = -sign(s) with sign(0) = +, and eliminates with the shifted pivot
-// s - D_i (Ballard et al. 2015). Blocks of 8 as in chol_inverse: the diagonal block and the
-// inverses of its two factors in the registers of every warp, the rest as block products.
+// has the top l x l block T (shared memory, zero padded, overwritten): the modified LU of
+// Ballard et al. 2015 in blocks of 8, warp 0 ahead of the others as in chol_inverse. sc:
+// kWarpScratch doubles.
 template <int NT>
 __device__ __forceinline__ void householder_signs(double* T, double* D, double* sc) {
   constexpr int LD = Tall<NT>::LD;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, r8 = lane & 7;
-  double *mL = sc + warp * 128, *mU = mL + 64;
+  const int warp = threadIdx.x >> 5;
   __syncthreads();
-  for (int b = 0; b < NT; ++b) {
-    double t[8], ui[8];
-    {
-      const double* Tb = T + 8 * b * LD + 8 * b;
-#pragma unroll
-      for (int j = 0; j < 8; ++j) t[j] = Tb[r8 * LD + j];
-    }
-#pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      const double piv = __shfl_sync(0xffffffffu, t[j], j);
-      const double di = piv >= 0.0 ? -1.0 : 1.0;
-      if (threadIdx.x == 0) D[8 * b + j] = di;
-      ui[j] = __drcp_rn(piv - di);
-      const double f = r8 > j ? t[j] * ui[j] : 0.0;
-#pragma unroll
-      for (int c = j + 1; c < 8; ++c) t[c] -= f * __shfl_sync(0xffffffffu, t[c], j);
-      if (r8 > j) t[j] = f;
-    }
-    double y[8], z[8];  // lane c: column c of L^-1 (unit lower) and of U^-1
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      double a = i == r8 ? 1.0 : 0.0;
-#pragma unroll
-      for (int m = 0; m < i; ++m) a -= __shfl_sync(0xffffffffu, t[m], i) * y[m];
-      y[i] = i >= r8 ? a : 0.0;
-    }
-#pragma unroll
-    for (int i = 7; i >= 0; --i) {
-      double a = i == r8 ? 1.0 : 0.0;
-#pragma unroll
-      for (int m = i + 1; m < 8; ++m) a -= __shfl_sync(0xffffffffu, t[m], i) * z[m];
-      z[i] = i <= r8 ? a * ui[i] : 0.0;
-    }
-    if (lane < 8) {
-#pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        mL[i * 8 + r8] = y[i];
-        mU[i * 8 + r8] = z[i];
-      }
-    }
-    __syncwarp();
+  auto factor = [&](int b) {
+    signs_block<LD>(T + 8 * b * LD + 8 * b, D + 8 * b, sc + (b & 1) * 128, sc + (b & 1) * 128 + 64);
+  };
+  if (warp == 0) factor(0);
+  __syncthreads();
+  for (int b = 0; b + 1 < NT; ++b) {
+    const double *Li = sc + (b & 1) * 128, *Ui = Li + 64;
     const int rest = NT - 1 - b;
     for (int q = warp; q < 2 * rest; q += kTallWarps) {  // block row, then block column
       const bool row = q < rest;
       double* P = row ? T + 8 * b * LD + 8 * (b + 1 + q) : T + 8 * (b + 1 + q - rest) * LD + 8 * b;
       double c[2] = {0.0, 0.0};
       if (row)
-        block_mma<false>(c, mL, 8, P, LD);
+        block_mma<false>(c, Li, 8, P, LD);
       else
-        block_mma<false>(c, P, LD, mU, 8);
+        block_mma<false>(c, P, LD, Ui, 8);
       __syncwarp();
       block_store(c, P, LD);
     }
     __syncthreads();
-    for (int q = warp; q < rest * rest; q += kTallWarps) {
-      const int I = b + 1 + q / rest, J = b + 1 + q % rest;
+    auto trail = [&](int I, int J) {
       double c[2];
       block_load(c, T + 8 * I * LD + 8 * J, LD);
       block_mma<false>(c, T + 8 * I * LD + 8 * b, LD, T + 8 * b * LD + 8 * J, LD, -1.0);
       block_store(c, T + 8 * I * LD + 8 * J, LD);
+    };
+    if (warp == 0) {
+      trail(b + 1, b + 1);
+      __syncwarp();
+      factor(b + 1);
+    } else {
+      for (int q = warp; q < rest * rest; q += kTallWarps - 1)  // tile 0 is warp 0's
+        trail(b + 1 + q / rest, b + 1 + q % rest);
     }
     __syncthreads();
   }
 }
 
-// sum_{b < n} x[b * stride] in b order with every load issued before the adds (n <= kTallMaxParts).
-__device__ __forceinline__ double sum_parts(const double* x, int n, int64_t stride) {
-  double v[kTallMaxParts];
+// v[i] = sum_{b < n} x[b * stride + t + i * blockDim] in b order, t the thread, for the i with
+// t + i * blockDim < count: the loads of four b of every element are issued before their adds.
+template <int COUNT>
+__device__ __forceinline__ void sum_parts(const double* x, int n, int64_t stride, double (&v)[(COUNT + kTallThreads - 1) / kTallThreads]) {
+  constexpr int kPer = (COUNT + kTallThreads - 1) / kTallThreads;
 #pragma unroll
-  for (int k = 0; k < kTallMaxParts; ++k) v[k] = k < n ? x[(int64_t)k * stride] : 0.0;
-  double s = 0.0;
+  for (int i = 0; i < kPer; ++i) v[i] = 0.0;
+  for (int b = 0; b < n; b += 4) {
+    double w[4][kPer];
 #pragma unroll
-  for (int k = 0; k < kTallMaxParts; ++k)
-    if (k < n) s += v[k];
-  return s;
+    for (int q = 0; q < 4; ++q)
+#pragma unroll
+      for (int i = 0; i < kPer; ++i) {
+        const int e = threadIdx.x + i * kTallThreads;
+        w[q][i] = b + q < n && e < COUNT ? x[(int64_t)(b + q) * stride + e] : 0.0;
+      }
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+#pragma unroll
+      for (int i = 0; i < kPer; ++i) v[i] += w[q][i];
+  }
 }
 
 // Cluster sum of the CTAs' part[n] (shared memory), in rank order, written to
