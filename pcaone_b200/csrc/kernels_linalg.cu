@@ -34,10 +34,10 @@ struct TallCfg {
 // registers of wider ones go to the accumulators).
 // Measured (ncu, us a launch; before: rows solved by substitution a thread each, 4 x 4 FMA tiles
 // from shared memory, Cholesky with a barrier a column, separate factorisation launches):
-//   Omega update without its operand copy, N = 20000, l = 40: 74 (was 176); N = 5003, l = 20: 44 (71)
-//   whole update with the int8 operand: 87 (216) and 52 (98)
-//   G passes of the epoch tail, M = 500000, l = 40: 71 + 105 (50 + 298, plus two Choleskys of 37);
-//   the tail at M = 50000, N = 2000, l = 20: 92 an epoch (176)
+//   Omega update without its operand copy, N = 20000, l = 40: 60 (was 176); N = 5003, l = 20: 36 (71)
+//   whole update with the int8 operand: 72 (216) and 43 (98)
+//   G passes of the epoch tail, M = 500000, l = 40: 66 + 99 (50 + 298, plus two Choleskys of 37);
+//   the tail at M = 50000, N = 2000, l = 20: 71 an epoch (176)
 template <int NT, bool PROD, bool RECT>
 __global__ void __cluster_dims__(kTallCluster, 1, 1) __launch_bounds__(kTallThreads) k_tall(TallStep a) {
   using T = Tall<NT>;

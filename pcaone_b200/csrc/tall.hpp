@@ -108,51 +108,49 @@ __device__ __forceinline__ double fast_reciprocal(double x) {
   return fma(y, fma(-x, y, 1.0), y);
 }
 
-// One warp: Cholesky factor R_bb of the symmetric 8 x 8 block Wb (row stride LD) into Rb and its
-// inverse into Xb (upper, zeros below), and the inverse of R_bb^T into Li (8 x 8). Lane r (mod 8)
-// holds row r; a step eliminates one column of the block and of an identity beside it, which ends as
-// the inverse of the unit lower factor; the eight square roots are taken at once, one a lane. A
-// pivot that is not positive, normal and finite is replaced by 1: returns 1 + its index, else 0.
+// The 8 x 8 block factorisations run in one warp, lane (g, r) = (lane / 8, lane % 8) holding row r,
+// columns 2 g and 2 g + 1, so that a step is the same few instructions for every column: the code
+// runs once a launch, on a CTA whose SM has not fetched it, and unrolled over the columns of a
+// row a lane it cost more in instruction fetches than in arithmetic.
+
+// Cholesky factor R_bb of the symmetric block Wb (row stride LD) into Rb and its inverse into Xb
+// (upper, zeros below), and the inverse of R_bb^T into Li (8 x 8). A step eliminates one column of
+// the block and of an identity beside it, which ends as the inverse of the unit lower factor;
+// the square roots of the pivots are taken at once at the end. A pivot that is not positive, normal
+// and finite is replaced by 1: returns 1 + the first one's index, else 0.
 template <int LD>
 __device__ __forceinline__ int chol_block(const double* Wb, double* Rb, double* Xb, double* Li) {
-  const int lane = threadIdx.x & 31, r8 = lane & 7;
-  double d[8], y[8], own = 1.0;
+  const int lane = threadIdx.x & 31, r = lane & 7, g = lane >> 3, row0 = lane & 24;
+  double d0 = Wb[r * LD + 2 * g], d1 = Wb[r * LD + 2 * g + 1], own = 1.0;
+  double y0 = r == 2 * g ? 1.0 : 0.0, y1 = r == 2 * g + 1 ? 1.0 : 0.0;
   int bad = 0;
+#pragma unroll 1
+  for (int jj = 0; jj < 4; ++jj)
 #pragma unroll
-  for (int j = 0; j < 8; ++j) {
-    d[j] = Wb[r8 * LD + j];
-    y[j] = j == r8 ? 1.0 : 0.0;
-  }
-#pragma unroll
-  for (int j = 0; j < 8; ++j) {
-    double p = __shfl_sync(0xffffffffu, d[j], j);
-    if (!(p >= 2.3e-308 && p < 4e307)) {
-      if (!bad) bad = j + 1;
-      p = 1.0;
+    for (int h = 0; h < 2; ++h) {
+      const int j = 2 * jj + h;
+      const double dj = h ? d1 : d0;
+      double p = __shfl_sync(0xffffffffu, dj, 8 * jj + j);
+      const double m = __shfl_sync(0xffffffffu, dj, 8 * jj + r);
+      const double w0 = __shfl_sync(0xffffffffu, d0, row0 + j), w1 = __shfl_sync(0xffffffffu, d1, row0 + j);
+      const double v0 = __shfl_sync(0xffffffffu, y0, row0 + j), v1 = __shfl_sync(0xffffffffu, y1, row0 + j);
+      if (!(p >= 2.3e-308 && p < 4e307)) {
+        if (!bad) bad = j + 1;
+        p = 1.0;
+      }
+      if (r == j) own = p;
+      const double f = r > j ? m * fast_reciprocal(p) : 0.0;
+      d0 = 2 * g > j ? d0 - f * w0 : 2 * g == j ? f : d0;
+      d1 = 2 * g + 1 > j ? d1 - f * w1 : 2 * g + 1 == j ? f : d1;
+      y0 -= f * v0;
+      y1 -= f * v1;
     }
-    if (r8 == j) own = p;
-    const double f = r8 > j ? d[j] * fast_reciprocal(p) : 0.0;
-#pragma unroll
-    for (int c = j + 1; c < 8; ++c) d[c] -= f * __shfl_sync(0xffffffffu, d[j], c);
-#pragma unroll
-    for (int c = 0; c <= j; ++c) y[c] -= f * __shfl_sync(0xffffffffu, y[c], j);
-    d[j] = f;
-  }
-  const double root = sqrt(own), iroot = 1.0 / root;
-#pragma unroll
-  for (int j = 0; j < 8; ++j) {
-    const double s = __shfl_sync(0xffffffffu, root, j);
-    d[j] = r8 == j ? s : d[j] * s;
-    y[j] *= iroot;
-  }
-  if (lane < 8) {
-#pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      Rb[j * LD + r8] = d[j];
-      Xb[j * LD + r8] = y[j];
-      Li[r8 * 8 + j] = y[j];
-    }
-  }
+  const double iroot = rsqrt(own), root = own * iroot;
+  const double s0 = __shfl_sync(0xffffffffu, root, 2 * g), s1 = __shfl_sync(0xffffffffu, root, 2 * g + 1);
+  Rb[2 * g * LD + r] = r == 2 * g ? s0 : d0 * s0;
+  Rb[(2 * g + 1) * LD + r] = r == 2 * g + 1 ? s1 : d1 * s1;
+  Xb[2 * g * LD + r] = Li[r * 8 + 2 * g] = y0 * iroot;
+  Xb[(2 * g + 1) * LD + r] = Li[r * 8 + 2 * g + 1] = y1 * iroot;
   __syncwarp();
   return bad;
 }
@@ -165,8 +163,9 @@ __device__ __forceinline__ int chol_block(const double* Wb, double* Rb, double* 
 // block costs its eight dependent steps, one block product and two CTA barriers. Returns 1 + the
 // first column whose pivot was not positive, else 0 (the same in every thread). sc: kWarpScratch
 // doubles.
-// One CTA, cycles for l = 20 / 40: PLACEHOLDER_CHOL (every warp factoring every block itself, rounded
-// reciprocals: 12500 / 21500; the warps' shuffles held one another up).
+// Omega update passes at N = 5003, l = 20 and N = 20000, l = 40: 12.9 and 22.1 us (15.7 and 28.0 with every
+// warp factoring every block itself, unrolled a row a lane, and rounded
+// reciprocals: their shuffles held one another up).
 template <int NT>
 __device__ __forceinline__ int chol_inverse(double* W, double* R, double* X, double* sc) {
   using T = Tall<NT>;
@@ -183,39 +182,40 @@ __device__ __forceinline__ int chol_inverse(double* W, double* R, double* X, dou
     const int bad = chol_block<LD>(W + o, R + o, X + o, Li + (b & 1) * 64);
     if (bad && threadIdx.x == 0 && first_bad == 0) first_bad = 8 * b + bad;
   };
-  if (warp == 0) factor(0);
-  __syncthreads();
-  for (int b = 0; b + 1 < NT; ++b) {
-    for (int J = b + 1 + warp; J < NT; J += kTallWarps) {  // block row of R
+#pragma unroll 1
+  for (int b = -1; b + 1 < NT; ++b) {  // b = -1: the first diagonal block alone
+    if (b >= 0 && b + 1 + warp < NT) {  // block row of R
+      const int J = b + 1 + warp;
       double c[2] = {0.0, 0.0};
       block_mma<false>(c, Li + (b & 1) * 64, 8, W + 8 * b * LD + 8 * J, LD);
       block_store(c, R + 8 * b * LD + 8 * J, LD);
     }
     __syncthreads();
-    auto trail = [&](int I, int J) {
-      double c[2];
-      block_load(c, W + 8 * I * LD + 8 * J, LD);
-      block_mma<true>(c, R + 8 * b * LD + 8 * I, LD, R + 8 * b * LD + 8 * J, LD, -1.0);
-      block_store(c, W + 8 * I * LD + 8 * J, LD);
-    };
+    // trailing tiles (I, J), b < I <= J, in rows: tile 0 is the next diagonal block, warp 0's
+    const int rest = NT - 1 - b;
+#pragma unroll 1
+    for (int q = warp; b >= 0 && q < rest * rest; q += kTallWarps - 1) {
+      const int I = b + 1 + q / rest, J = b + 1 + q % rest;
+      if (J >= I) {
+        double c[2];
+        block_load(c, W + 8 * I * LD + 8 * J, LD);
+        block_mma<true>(c, R + 8 * b * LD + 8 * I, LD, R + 8 * b * LD + 8 * J, LD, -1.0);
+        block_store(c, W + 8 * I * LD + 8 * J, LD);
+      }
+      if (warp == 0) break;
+    }
     if (warp == 0) {
-      trail(b + 1, b + 1);
       __syncwarp();
       factor(b + 1);
-    } else {
-      int t = 0;
-      for (int I = b + 1; I < NT; ++I)
-        for (int J = I; J < NT; ++J) {
-          if (I == b + 1 && J == I) continue;
-          if (t++ % (kTallWarps - 1) == warp - 1) trail(I, J);
-        }
     }
     __syncthreads();
   }
   // block column J of the inverse by warp J: X_IJ = -X_II sum_{I < K <= J} R_IK X_KJ
   for (int J = warp; J < NT; J += kTallWarps)
+#pragma unroll 1
     for (int I = J - 1; I >= 0; --I) {
       double c[2] = {0.0, 0.0}, g[2] = {0.0, 0.0};  // even and odd K apart: two chains of products
+#pragma unroll 1
       for (int K = I + 1; K <= J; K += 2) {
         block_mma<false>(c, R + 8 * I * LD + 8 * K, LD, X + 8 * K * LD + 8 * J, LD);
         if (K < J) block_mma<false>(g, R + 8 * I * LD + 8 * (K + 1), LD, X + 8 * (K + 1) * LD + 8 * J, LD);
@@ -248,45 +248,45 @@ __device__ __forceinline__ void upper_product(const double* A, const double* B, 
   __syncthreads();
 }
 
-// One warp: modified LU of the 8 x 8 block Tb (row stride LD): step i takes the pivot s = T[i][i],
-// D_i = -sign(s) with sign(0) = +, and eliminates with the shifted pivot u = s - D_i (|u| >= 1).
-// Writes D and the inverses of the two factors (Li unit lower, Ui upper, 8 x 8). Lane r (mod 8)
-// holds row r; the identity beside the block ends as Li, and Ui follows by back substitution.
+// Modified LU of the 8 x 8 block Tb (row stride LD): step j takes the pivot s = T[j][j],
+// D_j = -sign(s) with sign(0) = +, and eliminates with the shifted pivot u = s - D_j (|u| >= 1).
+// Writes D and the inverses of the two factors (Li unit lower, Ui upper, 8 x 8), which the
+// elimination's row and column operations leave in two identities beside the block.
 template <int LD>
 __device__ __forceinline__ void signs_block(const double* Tb, double* D, double* Li, double* Ui) {
-  const int lane = threadIdx.x & 31, r8 = lane & 7;
-  double t[8], y[8], z[8], ui[8];
+  const int lane = threadIdx.x & 31, r = lane & 7, g = lane >> 3, row0 = lane & 24;
+  double t0 = Tb[r * LD + 2 * g], t1 = Tb[r * LD + 2 * g + 1], i0 = 1.0, i1 = 1.0;
+  double y0 = r == 2 * g ? 1.0 : 0.0, y1 = r == 2 * g + 1 ? 1.0 : 0.0, z0 = y0, z1 = y1;
+#pragma unroll 1
+  for (int jj = 0; jj < 4; ++jj)
 #pragma unroll
-  for (int j = 0; j < 8; ++j) {
-    t[j] = Tb[r8 * LD + j];
-    y[j] = j == r8 ? 1.0 : 0.0;
-  }
-#pragma unroll
-  for (int j = 0; j < 8; ++j) {
-    const double piv = __shfl_sync(0xffffffffu, t[j], j);
-    const double di = piv >= 0.0 ? -1.0 : 1.0;
-    if (lane == 0) D[j] = di;
-    ui[j] = fast_reciprocal(piv - di);
-    const double f = r8 > j ? t[j] * ui[j] : 0.0;
-#pragma unroll
-    for (int c = j + 1; c < 8; ++c) t[c] -= f * __shfl_sync(0xffffffffu, t[c], j);
-#pragma unroll
-    for (int c = 0; c <= j; ++c) y[c] -= f * __shfl_sync(0xffffffffu, y[c], j);
-  }
-#pragma unroll
-  for (int i = 7; i >= 0; --i) {  // lane c: column c of U^-1
-    double a = i == r8 ? 1.0 : 0.0;
-#pragma unroll
-    for (int m = 7; m > i; --m) a -= __shfl_sync(0xffffffffu, t[m], i) * z[m];
-    z[i] = i <= r8 ? a * ui[i] : 0.0;
-  }
-  if (lane < 8) {
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      Li[r8 * 8 + i] = y[i];
-      Ui[i * 8 + r8] = z[i];
+    for (int h = 0; h < 2; ++h) {
+      const int j = 2 * jj + h;
+      const double tj = h ? t1 : t0, zj = h ? z1 : z0;
+      const double piv = __shfl_sync(0xffffffffu, tj, 8 * jj + j);
+      const double m = __shfl_sync(0xffffffffu, tj, 8 * jj + r), zr = __shfl_sync(0xffffffffu, zj, 8 * jj + r);
+      const double w0 = __shfl_sync(0xffffffffu, t0, row0 + j), w1 = __shfl_sync(0xffffffffu, t1, row0 + j);
+      const double v0 = __shfl_sync(0xffffffffu, y0, row0 + j), v1 = __shfl_sync(0xffffffffu, y1, row0 + j);
+      const double di = piv >= 0.0 ? -1.0 : 1.0;
+      if (lane == 0) D[j] = di;
+      const double inv = fast_reciprocal(piv - di), f = r > j ? m * inv : 0.0;
+      if (2 * g == j) i0 = inv;
+      if (2 * g + 1 == j) i1 = inv;
+      if (2 * g > j) {
+        t0 -= f * w0;
+        z0 -= zr * (w0 * inv);
+      }
+      if (2 * g + 1 > j) {
+        t1 -= f * w1;
+        z1 -= zr * (w1 * inv);
+      }
+      y0 -= f * v0;
+      y1 -= f * v1;
     }
-  }
+  Li[r * 8 + 2 * g] = y0;
+  Li[r * 8 + 2 * g + 1] = y1;
+  Ui[r * 8 + 2 * g] = z0 * i0;
+  Ui[r * 8 + 2 * g + 1] = z1 * i1;
   __syncwarp();
 }
 
@@ -302,12 +302,12 @@ __device__ __forceinline__ void householder_signs(double* T, double* D, double* 
   auto factor = [&](int b) {
     signs_block<LD>(T + 8 * b * LD + 8 * b, D + 8 * b, sc + (b & 1) * 128, sc + (b & 1) * 128 + 64);
   };
-  if (warp == 0) factor(0);
-  __syncthreads();
-  for (int b = 0; b + 1 < NT; ++b) {
+#pragma unroll 1
+  for (int b = -1; b + 1 < NT; ++b) {  // b = -1: the first diagonal block alone
     const double *Li = sc + (b & 1) * 128, *Ui = Li + 64;
     const int rest = NT - 1 - b;
-    for (int q = warp; q < 2 * rest; q += kTallWarps) {  // block row, then block column
+#pragma unroll 1
+    for (int q = warp; b >= 0 && q < 2 * rest; q += kTallWarps) {  // block row, then block column
       const bool row = q < rest;
       double* P = row ? T + 8 * b * LD + 8 * (b + 1 + q) : T + 8 * (b + 1 + q - rest) * LD + 8 * b;
       double c[2] = {0.0, 0.0};
@@ -319,19 +319,18 @@ __device__ __forceinline__ void householder_signs(double* T, double* D, double* 
       block_store(c, P, LD);
     }
     __syncthreads();
-    auto trail = [&](int I, int J) {
+#pragma unroll 1
+    for (int q = warp; b >= 0 && q < rest * rest; q += kTallWarps - 1) {  // tile 0 is warp 0's
+      const int I = b + 1 + q / rest, J = b + 1 + q % rest;
       double c[2];
       block_load(c, T + 8 * I * LD + 8 * J, LD);
       block_mma<false>(c, T + 8 * I * LD + 8 * b, LD, T + 8 * b * LD + 8 * J, LD, -1.0);
       block_store(c, T + 8 * I * LD + 8 * J, LD);
-    };
+      if (warp == 0) break;
+    }
     if (warp == 0) {
-      trail(b + 1, b + 1);
       __syncwarp();
       factor(b + 1);
-    } else {
-      for (int q = warp; q < rest * rest; q += kTallWarps - 1)  // tile 0 is warp 0's
-        trail(b + 1 + q / rest, b + 1 + q % rest);
     }
     __syncthreads();
   }
