@@ -49,7 +49,7 @@ void free_data(pcaone_ctx* c) {
   c->loaded = c->bedT_valid = c->miss_snp_valid = c->miss_ws_valid = false;
   // streamed genotypes: the pinned host buffer and the slots are kept for reuse; their
   // contents are forgotten (a copy still in flight completes first)
-  if (c->copy_stream) cudaStreamSynchronize(c->copy_stream);
+  stream_sync(c);
   c->streamed = false;
   c->slot[0].key = c->slot[1].key = 0;
   c->cur_slot = -1;
@@ -263,7 +263,7 @@ int pcaone_gpu_permute(pcaone_ctx* c, const int32_t* perm) {
     }
     if (c->streamed) {  // the host records are permuted, then counted again
       PG_CUDA(cudaStreamSynchronize(c->stream));
-      if (c->copy_stream) PG_CUDA(cudaStreamSynchronize(c->copy_stream));
+      stream_sync(c);
       stream_permute(c, perm);
       stream_counts(c);
     } else {

@@ -102,13 +102,15 @@ struct pcaone_ctx {
   bool streamed = false;
   uint8_t* h_bed = nullptr;
   size_t h_bed_bytes = 0;
-  cudaStream_t copy_stream = nullptr;
+  cudaStream_t copy_stream = nullptr;  // record copies; the transposition and tiling of a slot follow on:
+  cudaStream_t tile_stream = nullptr;
   size_t slot_budget = 0;  // device bytes per slot (records, transposed copy, tiles)
   struct StreamSlot {
     int b0 = -1, b1 = -1;  // windows held, once `ready` has completed on the copy stream
     uint64_t key = 0;      // data generation, window layout and tile kind of the contents
     uint8_t *rec = nullptr, *recT = nullptr, *t1 = nullptr, *t2 = nullptr;
-    cudaEvent_t ready = nullptr;  // contents complete (copy stream)
+    cudaEvent_t copied = nullptr; // records copied (copy stream)
+    cudaEvent_t ready = nullptr;  // contents complete (tile stream)
     cudaEvent_t idle = nullptr;   // last product reading the slot (main stream)
   } slot[2];
   int slot_windows = 0;   // windows a slot holds for the current layout
@@ -259,6 +261,8 @@ void stream_release(pcaone_ctx* c);
 const uint8_t* stream_codes(const pcaone_ctx* c, int b);
 const uint8_t* stream_codesT(const pcaone_ctx* c, int b);
 void stream_free(pcaone_ctx* c);
+// Waits for the fills of both slots.
+void stream_sync(pcaone_ctx* c);
 // Fails with PCAONE_ESTATE when the genotypes are streamed (calls that need them resident).
 void require_resident(const pcaone_ctx* c, const char* what);
 // Launchers used by the staging (kernels_bed.cu, kernels_gemm_i8.cu)
@@ -271,10 +275,11 @@ void launch_missing_ws_fill(pcaone_ctx* c, cudaStream_t st, const uint8_t* recT,
                             const uint64_t* d_base);
 int64_t missing_snp_scan(pcaone_ctx* c);  // by-SNP row pointers from the counts; total
 int64_t scan_counts(pcaone_ctx* c, const int64_t* cnt, uint64_t n, int64_t* ptr);
-// int8 back end: tile bytes per window (first, second product) and the tiling of one window
+// int8 back end: tile bytes per window (first, second product) and the tiling of nwin consecutive
+// windows of the current layout whose nsnp records start at rec
 void i8_tile_bytes(const pcaone_ctx* c, size_t* w1, size_t* w2);
-void i8_tile_window(pcaone_ctx* c, cudaStream_t st, const uint8_t* rec, int64_t m, const uint8_t* recT,
-                    uint8_t* t1, uint8_t* t2);
+void i8_tile_run(pcaone_ctx* c, cudaStream_t st, const uint8_t* rec, int64_t nsnp, int nwin, const uint8_t* recT,
+                 uint8_t* t1, uint8_t* t2);
 
 // ---------------------------------------------------------------- SIMT decode-GEMM
 // out[s][r][c] = sum_{k in split s} val(code[r][k]) * B[k][c], val(00,01,10,11) = (2,0,1,0)

@@ -415,24 +415,26 @@ __global__ void __launch_bounds__(kThreads, 1) k_decode_gemm_i8(const __grid_con
   }
 }
 
-// Tiled copy of one window's codes for this kernel: block (pair, chunk) = [tile 2p: codes
-// 0-63 of the chunk (128 rows x 16 bytes), codes 64-127][tile 2p+1: same]. src holds `rows`
-// valid rows of `pitch` bytes; rows past `rows` and bytes past the pitch are code 11 (value
-// 0). One thread per (row, 16-byte half chunk).
-__global__ void k_tile_codes_i8(const uint8_t* __restrict__ src, uint32_t pitch, int64_t rows, int64_t pairs,
-                                int64_t chunks, uint8_t* __restrict__ dst) {
+// Tiled copies of the codes of consecutive windows (one blockIdx.y each) for this kernel: block
+// (pair, chunk) of a window = [tile 2p: codes 0-63 of the chunk (128 rows x 16 bytes), codes
+// 64-127][tile 2p+1: same]. Window w's rows lie src_win bytes after those of window w - 1, `pitch`
+// bytes each: min(wlen, total - w wlen) of them are valid; rows past those and bytes past the pitch
+// are code 11 (value 0). One thread per (row, 16-byte half chunk). One launch for all windows
+// (64 of 4 us each before, for a panel of 5003 x 80021).
+__global__ void k_tile_codes_i8(const uint8_t* __restrict__ src, int64_t src_win, uint32_t pitch, int64_t wlen,
+                                int64_t total, int64_t pairs, int64_t chunks, uint8_t* __restrict__ dst) {
   const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  const int64_t halves = 2 * chunks;
+  const int64_t halves = 2 * chunks, w = blockIdx.y;
   if (t >= pairs * 2 * kRows * halves) return;
   const int64_t hc = t % halves, row = t / halves;
   uint4 v = make_uint4(0xFFFFFFFFu, 0xFFFFFFFFu, 0xFFFFFFFFu, 0xFFFFFFFFu);
-  if (row < rows && (hc + 1) * 16 <= (int64_t)pitch)
-    v = *reinterpret_cast<const uint4*>(src + row * (int64_t)pitch + hc * 16);
+  if (row < wlen && w * wlen + row < total && (hc + 1) * 16 <= (int64_t)pitch)
+    v = *reinterpret_cast<const uint4*>(src + w * src_win + row * (int64_t)pitch + hc * 16);
   const int64_t pair = row / (2 * kRows), rin2 = row - pair * 2 * kRows;
   const int64_t tile = rin2 / kRows, rin = rin2 - tile * kRows;
   const int64_t kc = hc >> 1, h = hc & 1;
-  *reinterpret_cast<uint4*>(dst + (pair * chunks + kc) * kPairChunkBytes + tile * 2 * kHalfBytes + h * kHalfBytes +
-                            rin * 16) = v;
+  *reinterpret_cast<uint4*>(dst + ((w * pairs + pair) * chunks + kc) * kPairChunkBytes + tile * 2 * kHalfBytes +
+                            h * kHalfBytes + rin * 16) = v;
 }
 
 // Largest |X[k][c]| over the K rows of a row-major K x l matrix, as the bits of a double
@@ -683,17 +685,7 @@ void ensure_tiles(pcaone_ctx* c) {
   uint8_t* d1 = (uint8_t*)scratch(c, "i8_tile1", (size_t)bands * w1);
   uint8_t* d2 = (uint8_t*)scratch(c, "i8_tile2", (size_t)bands * w2);
   if (c->tiles8_valid && c->tiles8_key == key && c->tile81_ptr == d1 && c->tile82_ptr == d2) return;
-  for (int b = 0; b < bands; ++b) {
-    const int64_t s = (int64_t)c->win.start[b], m = (int64_t)c->win.stop[b] - s;
-    const int64_t n1 = g.p1 * 2 * kRows * 2 * g.c1, n2 = g.p2 * 2 * kRows * 2 * g.c2;
-    k_tile_codes_i8<<<(unsigned)((n1 + 255) / 256), 256, 0, c->stream>>>(c->d_bed + s * c->pitch, c->pitch, m, g.p1,
-                                                                       g.c1, d1 + (size_t)b * w1);
-    PG_CHECK_LAUNCH();
-    k_tile_codes_i8<<<(unsigned)((n2 + 255) / 256), 256, 0, c->stream>>>(
-        c->d_bedT + (int64_t)b * c->Npad * c->win.pitch, c->win.pitch, (int64_t)c->N, g.p2, g.c2, d2 + (size_t)b * w2);
-    PG_CHECK_LAUNCH();
-    c->launches += 2;
-  }
+  i8_tile_run(c, c->stream, c->d_bed, (int64_t)c->M, bands, c->d_bedT, d1, d2);
   c->tiles8_key = key;
   c->tiles8_valid = true;
   c->tile81_ptr = d1;
@@ -852,15 +844,23 @@ void i8_tile_bytes(const pcaone_ctx* c, size_t* w1, size_t* w2) {
   *w2 = (size_t)g.p2 * g.c2 * kPairChunkBytes;
 }
 
-void i8_tile_window(pcaone_ctx* c, cudaStream_t st, const uint8_t* rec, int64_t m, const uint8_t* recT, uint8_t* t1,
-                    uint8_t* t2) {
+void i8_tile_run(pcaone_ctx* c, cudaStream_t st, const uint8_t* rec, int64_t nsnp, int nwin, const uint8_t* recT,
+                 uint8_t* t1, uint8_t* t2) {
   const TileGeom g = tile_geom(c);
   const int64_t n1 = g.p1 * 2 * kRows * 2 * g.c1, n2 = g.p2 * 2 * kRows * 2 * g.c2;
-  k_tile_codes_i8<<<(unsigned)((n1 + 255) / 256), 256, 0, st>>>(rec, c->pitch, m, g.p1, g.c1, t1);
-  PG_CHECK_LAUNCH();
-  k_tile_codes_i8<<<(unsigned)((n2 + 255) / 256), 256, 0, st>>>(recT, c->win.pitch, (int64_t)c->N, g.p2, g.c2, t2);
-  PG_CHECK_LAUNCH();
-  c->launches += 2;
+  const int64_t bs = (int64_t)c->win.blocksize, N = (int64_t)c->N;
+  for (int w0 = 0; w0 < nwin; w0 += 65535) {  // windows beyond the grid's y limit: further launches
+    const int nw = std::min(nwin - w0, 65535);
+    k_tile_codes_i8<<<dim3((unsigned)((n1 + 255) / 256), nw), 256, 0, st>>>(
+        rec + w0 * bs * c->pitch, bs * c->pitch, c->pitch, bs, nsnp - w0 * bs, g.p1, g.c1,
+        t1 + w0 * g.p1 * g.c1 * kPairChunkBytes);
+    PG_CHECK_LAUNCH();
+    k_tile_codes_i8<<<dim3((unsigned)((n2 + 255) / 256), nw), 256, 0, st>>>(
+        recT + (int64_t)w0 * c->Npad * c->win.pitch, (int64_t)c->Npad * c->win.pitch, c->win.pitch, N, N * nw, g.p2, g.c2,
+        t2 + w0 * g.p2 * g.c2 * kPairChunkBytes);
+    PG_CHECK_LAUNCH();
+    c->launches += 2;
+  }
 }
 
 GemmFnT<float> gemm_i8() {

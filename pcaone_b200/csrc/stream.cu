@@ -7,9 +7,9 @@
 // Two device slots each hold up to slot_windows consecutive windows: their SNP-major records
 // (a plain copy of host rows), the sample-major copy per window and, for the int8 back end,
 // the tiled copies of both products. While the products of one slot run on the library's
-// stream, the copy stream fills the other slot with the next windows (H2D copy, transposition
-// and tiling), ordered by two events per slot: `ready` (contents complete) and `idle` (the
-// last product reading the slot). The missing-entry lists and the per-SNP vectors stay on
+// stream, the copy stream and the tile stream fill the other slot with the next windows (H2D copy;
+// transposition and tiling), ordered by three events per slot: `copied` (records there), `ready`
+// (contents complete) and `idle` (the last product reading the slot). The missing-entry lists and the per-SNP vectors stay on
 // the device; they are built from two staging passes when the window layout is set.
 #include <algorithm>
 #include <cstring>
@@ -43,22 +43,21 @@ SlotSizes slot_sizes(const pcaone_ctx* c, bool tiles) {
   return z;
 }
 
-// Stage windows [b0, b1) into slot s on the copy stream.
+// Stage windows [b0, b1) into slot s: the records on the copy stream, what is made of them on the tile
+// stream, so that the next slot's records cross the link while this one's are tiled.
 void stage(pcaone_ctx* c, int s, int b0, int b1, bool tiles) {
   auto& S = c->slot[s];
-  const SlotSizes z = slot_sizes(c, tiles);
   const uint64_t s0 = c->win.start[b0], s1 = c->win.stop[b1 - 1];
   PG_CUDA(cudaStreamWaitEvent(c->copy_stream, S.idle, 0));
+  PG_CUDA(cudaStreamWaitEvent(c->copy_stream, S.ready, 0));  // a fill that no product used reads the records too
   S.key = 0;  // invalid until the host has queued the whole fill
   PG_CUDA(cudaMemcpyAsync(S.rec, c->h_bed + s0 * c->pitch, (size_t)(s1 - s0) * c->pitch, cudaMemcpyHostToDevice,
                           c->copy_stream));
-  launch_transpose_run(c, c->copy_stream, S.rec, s1 - s0, b1 - b0, S.recT);
-  if (tiles)
-    for (int b = b0; b < b1; ++b)
-      i8_tile_window(c, c->copy_stream, S.rec + (size_t)(c->win.start[b] - s0) * c->pitch,
-                     (int64_t)(c->win.stop[b] - c->win.start[b]), S.recT + (size_t)(b - b0) * z.recT,
-                     S.t1 + (size_t)(b - b0) * z.t1, S.t2 + (size_t)(b - b0) * z.t2);
-  PG_CUDA(cudaEventRecord(S.ready, c->copy_stream));
+  PG_CUDA(cudaEventRecord(S.copied, c->copy_stream));
+  PG_CUDA(cudaStreamWaitEvent(c->tile_stream, S.copied, 0));
+  launch_transpose_run(c, c->tile_stream, S.rec, s1 - s0, b1 - b0, S.recT);
+  if (tiles) i8_tile_run(c, c->tile_stream, S.rec, (int64_t)(s1 - s0), b1 - b0, S.recT, S.t1, S.t2);
+  PG_CUDA(cudaEventRecord(S.ready, c->tile_stream));
   S.b0 = b0;
   S.b1 = b1;
   S.key = slot_key(c, tiles);
@@ -74,9 +73,14 @@ int slot_holding(const pcaone_ctx* c, int b, bool tiles) {
 
 }  // namespace
 
+void stream_sync(pcaone_ctx* c) {
+  if (c->copy_stream) cudaStreamSynchronize(c->copy_stream);
+  if (c->tile_stream) cudaStreamSynchronize(c->tile_stream);
+}
+
 void stream_counts(pcaone_ctx* c) {
   // staged through slot 0's record buffer (at least 256 MB here; the RSVD may grow it)
-  if (c->copy_stream) PG_CUDA(cudaStreamSynchronize(c->copy_stream));
+  stream_sync(c);
   const uint64_t rows = std::max<uint64_t>(1, std::min<uint64_t>(c->M, (uint64_t(256) << 20) / c->pitch));
   uint8_t* buf = (uint8_t*)scratch(c, "stream_rec0", rows * c->pitch);
   c->slot[0].key = 0;
@@ -92,7 +96,7 @@ void stream_counts(pcaone_ctx* c) {
 
 void stream_missing_snp(pcaone_ctx* c) {
   if (c->miss_snp_valid) return;
-  if (c->copy_stream) PG_CUDA(cudaStreamSynchronize(c->copy_stream));
+  stream_sync(c);
   PG_CUDA(cudaStreamSynchronize(c->stream));
   missing_snp_scan(c);
   const uint64_t rows = std::max<uint64_t>(1, std::min<uint64_t>(c->M, (uint64_t(256) << 20) / c->pitch));
@@ -111,7 +115,7 @@ void stream_missing_snp(pcaone_ctx* c) {
 void stream_prepare(pcaone_ctx* c, int bands, uint64_t blocksize, bool tiles) {
   PG_REQUIRE(c->streamed && c->h_bed, PCAONE_ESTATE, "no streamed genotypes");
   // buffers may be reallocated below: no fill of a slot may still be in flight
-  if (c->copy_stream) PG_CUDA(cudaStreamSynchronize(c->copy_stream));
+  stream_sync(c);
   set_window_layout(c, bands, blocksize);
   const int nwin = c->win.bands;
   const SlotSizes z = slot_sizes(c, tiles);
@@ -133,6 +137,7 @@ void stream_prepare(pcaone_ctx* c, int bands, uint64_t blocksize, bool tiles) {
     S.recT = recT;
     S.t1 = t1;
     S.t2 = t2;
+    if (!S.copied) PG_CUDA(cudaEventCreateWithFlags(&S.copied, cudaEventDisableTiming));
     if (!S.ready) PG_CUDA(cudaEventCreateWithFlags(&S.ready, cudaEventDisableTiming));
     if (!S.idle) PG_CUDA(cudaEventCreateWithFlags(&S.idle, cudaEventDisableTiming));
   }
@@ -207,7 +212,7 @@ const uint8_t* stream_codesT(const pcaone_ctx* c, int b) {
 }
 
 void stream_load(pcaone_ctx* c, const uint8_t* packed, size_t slot_bytes) {
-  if (c->copy_stream) PG_CUDA(cudaStreamSynchronize(c->copy_stream));
+  stream_sync(c);
   const size_t bytes = (size_t)c->M * c->pitch;
   if (c->h_bed_bytes < bytes) {
     if (c->h_bed) PG_CUDA(cudaFreeHost(c->h_bed));
@@ -217,6 +222,7 @@ void stream_load(pcaone_ctx* c, const uint8_t* packed, size_t slot_bytes) {
     c->h_bed_bytes = bytes;
   }
   if (!c->copy_stream) PG_CUDA(cudaStreamCreateWithFlags(&c->copy_stream, cudaStreamNonBlocking));
+  if (!c->tile_stream) PG_CUDA(cudaStreamCreateWithFlags(&c->tile_stream, cudaStreamNonBlocking));
   // records at the device pitch, padding codes 11 past the samples (as k_unpack sets
   // them in the resident copy), copied by a few host threads
   const uint32_t bpr = c->bpr, pitch = c->pitch, r = c->N & 3u;
@@ -258,8 +264,9 @@ void stream_permute(pcaone_ctx* c, const int32_t* perm) {
 }
 
 void stream_free(pcaone_ctx* c) {
-  if (c->copy_stream) cudaStreamSynchronize(c->copy_stream);
+  stream_sync(c);
   for (auto& S : c->slot) {
+    if (S.copied) cudaEventDestroy(S.copied);
     if (S.ready) cudaEventDestroy(S.ready);
     if (S.idle) cudaEventDestroy(S.idle);
     S = pcaone_ctx::StreamSlot();
@@ -269,6 +276,8 @@ void stream_free(pcaone_ctx* c) {
   c->h_bed_bytes = 0;
   if (c->copy_stream) cudaStreamDestroy(c->copy_stream);
   c->copy_stream = nullptr;
+  if (c->tile_stream) cudaStreamDestroy(c->tile_stream);
+  c->tile_stream = nullptr;
 }
 
 }  // namespace pg
