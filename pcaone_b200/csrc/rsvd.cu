@@ -149,13 +149,8 @@ struct Engine {
   float* omg_float() { return std::is_same<T, float>::value ? reinterpret_cast<float*>(OmgT) : nullptr; }
 
   void init_omega() {
-    std::vector<double> cm((size_t)N * l);
-    omega_host(o.seed, o.rand, N, l, cm.data());
-    double* d_cm = (double*)scratch(c, "r_omg_cm", cm.size() * 8);
-    PG_CUDA(cudaMemcpyAsync(d_cm, cm.data(), cm.size() * 8, cudaMemcpyHostToDevice, c->stream));
-    to_rowmajor(c, d_cm, N, l, Npad, nullptr, Omg, omg_float());
+    omega_device(c, o.seed, o.rand, N, l, Npad, Omg, omg_float());
     colsum(c, Omg, l, N, wsum);
-    PG_CUDA(cudaStreamSynchronize(c->stream));  // the host vector goes out of scope
     gemm.omega_changed(c, Omg, l, Npad);
   }
 

@@ -67,6 +67,8 @@ void gl_grm(pcaone_ctx* c, const double* US, const double* V, int k, double* C, 
 // Frees the context's cuSOLVER handle.
 void gl_release(pcaone_ctx* c);
 
+// The sketch drawn on the device, row-major npad x l (zero past nrow) and its optional FP32 copy.
+void omega_device(pcaone_ctx* c, int seed, int rand, uint64_t nrow, int l, uint64_t npad, double* O, float* Of);
 void omega_host(int seed, int rand, uint64_t nrow, uint32_t ncol, double* out);
 void jacobi_svd(int n, const double* A, double* U, double* s, double* V);
 void run_product(pcaone_ctx* c, int precision, int transpose, int standardize, int ploidy,

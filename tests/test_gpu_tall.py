@@ -29,3 +29,19 @@ def test_rsvd_widths_and_row_edges(gpu, N, k, os_, svd):
     np.testing.assert_allclose(r.S, S, rtol=1e-9)
     np.testing.assert_allclose(r.U.T @ r.U, np.eye(k), atol=1e-9)
     np.testing.assert_allclose(r.V.T @ r.V, np.eye(k), atol=1e-9)
+
+
+@pytest.mark.parametrize("N,k,os_", [(40, 1, 1), (203, 4, 10), (1000, 20, 21), (5003, 12, 20)])
+@pytest.mark.parametrize("rand,seed", [(1, 101), (0, 101), (1, 0), (0, 7), (1, 2147483647), (1, -5)])
+def test_sketch_drawn_on_the_device(gpu, N, k, os_, rand, seed):
+    """One epoch from the seeded sketch (a fraction of a CTA's candidates to several hundred CTAs):
+    singular values of Z^T Omega's range depend on every value of Omega."""
+    bed = random_bed(N, 400, seed=5, miss=0.0)
+    gpu.load_bed(bed.packed, N)
+    kw = dict(k=k, oversamples=os_, maxp=0, tol=0.0, svd=1, seed=seed, rand=rand)
+    r = gpu.rsvd(precision="fp64", **kw)
+    Z, _ = O.standardized_from_bed(bed)  # one epoch by hand: the oracle's loop needs two
+    G = Z.T @ O.omega(seed, N, k + max(os_, k), rand)
+    R = np.linalg.qr(G)[1]
+    S = np.linalg.svd(np.linalg.solve(R.T, (Z @ G).T), compute_uv=False)[:k]
+    np.testing.assert_allclose(r.S, S, rtol=1e-9)
