@@ -182,11 +182,15 @@ int pcaone_gpu_load_bed(pcaone_ctx* c, const uint8_t* packed, uint64_t nsnps, ui
     PG_CUDA(cudaMemsetAsync(c->d_bed + c->M * c->pitch, 0xFF, (c->Mpad - c->M) * c->pitch, c->stream));
     // the records as they lie in the file, to a staging area from which k_unpack writes the rows
     const size_t raw = (size_t)c->M * c->bpr;
-    if (raw < kXferMin || c->bpr > kXferSlot) {
-      uint8_t* stage = (uint8_t*)scratch(c, "bed_stage", raw + 8);
-      PG_CUDA(cudaMemcpyAsync(stage, packed, raw, cudaMemcpyHostToDevice, c->stream));
-      launch_unpack(c, c->stream, stage, 0, c->M);
-      c->launches++;
+    if (raw < kXferMin || c->bpr > kXferSlot) {  // small, or records longer than a slot: 64 MiB at a time
+      const uint64_t rows = std::min<uint64_t>(c->M, std::max<uint64_t>(1, (uint64_t(64) << 20) / c->bpr));
+      uint8_t* stage = (uint8_t*)scratch(c, "bed_stage", rows * c->bpr + 8);
+      for (uint64_t j0 = 0; j0 < c->M; j0 += rows) {
+        const uint64_t n = std::min(rows, c->M - j0);
+        PG_CUDA(cudaMemcpyAsync(stage, packed + j0 * c->bpr, n * c->bpr, cudaMemcpyHostToDevice, c->stream));
+        launch_unpack(c, c->stream, stage, j0, n);
+        c->launches++;
+      }
     } else {
       constexpr size_t slot_pad = kXferSlot + 256;
       uint8_t* stage = (uint8_t*)scratch(c, "bed_stage", (size_t)xfer_workers() * slot_pad);

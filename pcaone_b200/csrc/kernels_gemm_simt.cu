@@ -59,9 +59,12 @@ __device__ __forceinline__ void cp_async_zfill(void* sdst, const void* gsrc, boo
 
 // The codes of a thread's four rows come straight from global memory (16 bytes a row and chunk)
 // and B through two shared-memory buffers of 4-byte asynchronous copies, both one chunk ahead:
-// with one to eight warps a CTA the copies' latency is what bounds it otherwise.
+// with one to eight warps a CTA the copies' latency is what bounds it otherwise. FP32 sums run over
+// kFlush chunks at most and then go to FP64 sums: over the 250000 SNPs of a long run in one
+// go they would lose two digits (eigenvalues of 20000 x 500000: 1e-6 against 3e-8).
 // Runs of a winSVD, M = 30011, N = 1502, l = 15, mean of 266 products: 12.8 us with splits
 // down to one chunk (30.9 staged through registers with four chunks a split at least).
+constexpr int kFlush = 4;
 template <int G>
 __global__ void __launch_bounds__(32 * G)
 k_decode_gemm(const uint8_t* __restrict__ codes, uint32_t pitch, int64_t rows, int64_t chunks, KRun run,
@@ -96,10 +99,14 @@ k_decode_gemm(const uint8_t* __restrict__ codes, uint32_t pitch, int64_t rows, i
   };
 
   float acc[kRPT][kCW];
+  double sum[kRPT][kCW];
 #pragma unroll
   for (int q = 0; q < kRPT; ++q)
 #pragma unroll
-    for (int c = 0; c < kCW; ++c) acc[q][c] = 0.f;
+    for (int c = 0; c < kCW; ++c) {
+      acc[q][c] = 0.f;
+      sum[q][c] = 0.0;
+    }
 
   uint4 cur[kRPT], nxt[kRPT];
   if (kc0 < kc1) {
@@ -136,6 +143,15 @@ k_decode_gemm(const uint8_t* __restrict__ codes, uint32_t pitch, int64_t rows, i
       }
     }
     __syncthreads();  // the buffer is read before it is refilled
+    if ((kc - kc0) % kFlush == kFlush - 1 || kc + 1 == kc1) {
+#pragma unroll
+      for (int q = 0; q < kRPT; ++q)
+#pragma unroll
+        for (int c = 0; c < kCW; ++c) {
+          sum[q][c] += (double)acc[q][c];
+          acc[q][c] = 0.f;
+        }
+    }
 #pragma unroll
     for (int q = 0; q < kRPT; ++q) cur[q] = nxt[q];
   }
@@ -147,7 +163,7 @@ k_decode_gemm(const uint8_t* __restrict__ codes, uint32_t pitch, int64_t rows, i
 #pragma unroll
     for (int c = 0; c < kCW; ++c) {
       const int col = g * kCW + c;
-      if (col < l) o[r * l + col] = acc[q][c];
+      if (col < l) o[r * l + col] = (float)sum[q][c];
     }
   }
 }

@@ -12,7 +12,6 @@
 #include <atomic>
 #include <cstring>
 #include <mutex>
-#include <system_error>
 #include <thread>
 #include <vector>
 
@@ -102,7 +101,7 @@ void xfer_chunks(pcaone_ctx* c, int64_t chunks, const XferChunk& f) {
   th.reserve(workers);
   try {
     for (int t = 1; t < workers; ++t) th.emplace_back(work, t);
-  } catch (const std::system_error&) {  // no more threads: go on with those there are
+  } catch (...) {  // no more threads: go on with those there are
   }
   work(0);
   for (auto& x : th) x.join();

@@ -15,9 +15,9 @@ def counts_of(packed, N):
 
 
 # record bytes 1, 2, 3, 5, 16, 17, 64, 65 (every start alignment), then more than 8 MiB in all: chunks of
-# whole records, the last one ragged, tiny and long records
+# whole records, the last one ragged, tiny and long records, and records longer than a chunk
 @pytest.mark.parametrize("N,M", [(1, 7), (5, 300), (12, 33), (17, 1001), (64, 40), (65, 129), (256, 50), (257, 77),
-                                 (4099, 9003), (17, 1800003), (100003, 411)])
+                                 (4099, 9003), (17, 1800003), (100003, 411), (4200001, 71)])
 def test_load_layout_counts_and_frequencies(gpu, N, M):
     rng = np.random.default_rng(N + M)
     packed = rng.integers(0, 256, (M, (N + 3) // 4), dtype=np.uint8)

@@ -146,3 +146,15 @@ def test_mixed_operand_maxima_across_calls(gpu):
     np.testing.assert_allclose(b.S, a.S, rtol=1e-6)
     S = O.run_pca(bed, k=4, svd=2, bands=8, maxp=4, tol=0.0, shuffle=False)[1]
     np.testing.assert_allclose(b.S, S, rtol=1e-6)
+
+
+def test_fp32_product_over_long_k(gpu):
+    """Enough rows that K is not split: the FP32 sums run over 256 codes at most whatever the length
+    of K, so the error stays below 2^-24 sqrt(256 / 2) of a column's size (0.29 units a rounding,
+    random walk), where one sum over 8192 would be five times that."""
+    N, M, l = 8192, 38000, 64
+    packed = np.random.default_rng(6).integers(0, 256, (M, N // 4), dtype=np.uint8)
+    gpu.load_bed(packed, N)
+    B = np.random.default_rng(7).standard_normal((N, l))
+    ref = gpu.product_t(B, precision="fp64")
+    assert rel_col_err(gpu.product_t(B, precision="fp32"), ref) <= 2.0 ** -24 * np.sqrt(128)
