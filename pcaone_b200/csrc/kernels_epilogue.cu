@@ -57,7 +57,7 @@ __device__ __forceinline__ void reduce_parts(const double* part, int l, double* 
 // written to out (shared memory of this warp). CPL = ceil(l / 8).
 template <int CPL, typename R, typename Wt>
 __device__ __forceinline__ void gather_rows(int64_t e0, int64_t e1, const int32_t* __restrict__ idx,
-                                            const R* __restrict__ rows, int64_t row0, int l, Wt weight,
+                                            const R* rows, int64_t row0, int l, Wt weight,
                                             double* out) {
   constexpr int kSteps = 2;
   const int lane = threadIdx.x & 31, grp = lane >> 3, q = lane & 7;
@@ -124,7 +124,7 @@ __device__ __forceinline__ void gather_rows(int64_t e0, int64_t e1, const int32_
 constexpr int kSumBatch = 16;
 template <int G, bool kWeighted = false, typename Wt = double (*)(int64_t)>
 __device__ __forceinline__ void sum_rows4(int64_t e0, int64_t e1, const int32_t* __restrict__ idx,
-                                          const float* __restrict__ rows, int64_t row0, double* out,
+                                          const float* rows, int64_t row0, double* out,
                                           Wt weight = nullptr) {
   // batch size by row width, so that the kernels stay within three CTAs an SM without
   // spilling: rows of up to 20 values take 24 entries a batch (18 weighted), 24-32 values 16
@@ -151,7 +151,7 @@ __device__ __forceinline__ void sum_rows4(int64_t e0, int64_t e1, const int32_t*
     for (int t = 0; t < T; ++t) {  // every row load of the batch first
       const int src = grp + R * t;
       const int64_t ii = __shfl_sync(0xffffffffu, my, src & 31);
-      v[t] = (active && src < cnt) ? __ldg(rows4 + ii * G + cg) : make_float4(0.f, 0.f, 0.f, 0.f);
+      v[t] = (active && src < cnt) ? chain_load(rows4 + ii * G + cg) : make_float4(0.f, 0.f, 0.f, 0.f);
     }
     nxt = 0;
     nxtw = 0.0;
@@ -190,7 +190,7 @@ __device__ __forceinline__ void sum_rows4(int64_t e0, int64_t e1, const int32_t*
 // 2 CPL (the two instantiations a kernel of that CPL can meet).
 template <int CPL, bool kWeighted = false, typename Wt = double (*)(int64_t)>
 __device__ __forceinline__ void sum_rows(int64_t e0, int64_t e1, const int32_t* __restrict__ idx,
-                                         const float* __restrict__ rows, int64_t row0, int l, double* out,
+                                         const float* rows, int64_t row0, int l, double* out,
                                          Wt weight = nullptr) {
   if ((l >> 2) == 2 * CPL)
     sum_rows4<2 * CPL, kWeighted>(e0, e1, idx, rows, row0, out, weight);
@@ -209,7 +209,7 @@ __device__ __forceinline__ void sum_rows(int64_t e0, int64_t e1, const int32_t* 
 // imputed values are set), 1 = unweighted float4 row sums (no imputed values, FP32 rows,
 // l % 4 == 0), 2 = weighted float4 row sums (imputed values, FP32 rows, l % 4 == 0).
 template <typename T, int CPL, int kMode>
-__global__ void __launch_bounds__(256, CPL <= 5 ? 3 : 2) k_prep(EpiP1 p, const T* __restrict__ D1, T* __restrict__ B2,
+__global__ void __launch_bounds__(256, CPL <= 5 ? 3 : 2) k_prep(EpiP1 p, const T* D1, T* __restrict__ B2,
                        double* h0_part, double* __restrict__ h0, unsigned* counter) {
   extern __shared__ double sh0[];  // warps x l partial h0, then warps x l sparse sums; the reduction's 256
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
@@ -314,7 +314,7 @@ __global__ void k_scale_g(int64_t start, int64_t m, int l, const double* __restr
 // EMU, 5000 samples with rates from Beta(2, 18), 100000 SNPs, l = 20, mean of 133 runs:
 // 86 us (110 with a warp a row).
 template <typename T, int CPL, int kMode>
-__global__ void __launch_bounds__(256, CPL <= 5 ? 3 : 2) k_accum(EpiP2 p, const T* __restrict__ D2, int wpr) {
+__global__ void __launch_bounds__(256, CPL <= 5 ? 3 : 2) k_accum(EpiP2 p, const T* D2, int wpr) {
   extern __shared__ double ssm[];  // warps x l sparse sums
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5, rows = nwarps / wpr;
   const double *mv = p.miss_val, *sc = p.scale, *F = p.F, *mw = p.miss_w;

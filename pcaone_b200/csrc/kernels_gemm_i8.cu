@@ -465,9 +465,9 @@ __global__ void k_colmax(const T* __restrict__ X, int64_t K, int l, unsigned lon
 // N = 5003, M = 80021, l = 20, mean of 133 runs: 7.1 us (13.3).
 constexpr int kQuantThreads = 512;
 template <typename T>
-__global__ void __launch_bounds__(kQuantThreads) k_quant(const T* __restrict__ X, int64_t kpw, int64_t wlen,
+__global__ void __launch_bounds__(kQuantThreads) k_quant(const T* X, int64_t kpw, int64_t wlen,
                                                          int64_t mtot, int l, int lp, int np,
-                                                         const unsigned long long* __restrict__ qmax,
+                                                         const unsigned long long* qmax,
                                                          int8_t* __restrict__ bq, float* __restrict__ sig) {
   __shared__ __align__(16) uint8_t img[192 * 128];
   __shared__ PieceTable tab;

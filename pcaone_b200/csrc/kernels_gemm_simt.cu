@@ -68,7 +68,7 @@ constexpr int kFlush = 4;
 template <int G>
 __global__ void __launch_bounds__(32 * G)
 k_decode_gemm(const uint8_t* __restrict__ codes, uint32_t pitch, int64_t rows, int64_t chunks, KRun run,
-              const float* __restrict__ B, int ldb, int l, int64_t kchunks_per_split,
+              const float* B, int ldb, int l, int64_t kchunks_per_split,
               float* __restrict__ out) {
   constexpr int LDS = G * kCW;              // padded B columns in shared memory
   __shared__ __align__(16) float bsm[2][kKC * LDS];

@@ -258,7 +258,7 @@ k_dense_gemm(const float* __restrict__ A, uint64_t lda, int64_t rows, int64_t K,
 // the current chunk is multiplied. The product is bound by reading A once from HBM.
 template <bool AT, int CN>
 __global__ void __launch_bounds__(256)
-k_dense_gemm2(const float* __restrict__ A, uint64_t lda, int64_t rows, int64_t K, const float* __restrict__ B,
+k_dense_gemm2(const float* __restrict__ A, uint64_t lda, int64_t rows, int64_t K, const float* B,
               int l, int64_t kchunks_per_split, float* __restrict__ out) {
   constexpr int TR = 128, KC = 32, CW = CN / 8;
   __shared__ __align__(16) float as[2][KC][TR + 4];

@@ -61,7 +61,7 @@ __device__ __forceinline__ void solve_rows(const double* Q1, const double* Rs, i
 // reads the rows of Q1 meanwhile).
 template <int NT>
 __global__ void __cluster_dims__(kTallCluster, 1, 1) __launch_bounds__(kTallThreads)
-    k_flip(UpdateArgs a, const double* __restrict__ Q1, double* __restrict__ Q) {
+    k_flip(UpdateArgs a, const double* Q1, double* __restrict__ Q) {
   using T = Tall<NT>;
   constexpr int LT = T::LT, LD = T::LD;
   extern __shared__ __align__(16) double sm[];
@@ -167,7 +167,7 @@ __global__ void __cluster_dims__(kTallCluster, 1, 1) __launch_bounds__(kTallThre
 
 // Omega = Q m over the 128 rows of a CTA (one K chunk of the int8 operand), coalesced.
 constexpr int kApplyThreads = 512;
-__global__ void __launch_bounds__(kApplyThreads) k_apply(UpdateArgs a, const double* __restrict__ Q) {
+__global__ void __launch_bounds__(kApplyThreads) k_apply(UpdateArgs a, const double* Q) {
   extern __shared__ __align__(16) uint8_t img[];  // np x 128 bytes (int8 operand)
   __shared__ PieceTable tab;
   __shared__ double mult[kLmax];
@@ -182,20 +182,30 @@ __global__ void __launch_bounds__(kApplyThreads) k_apply(UpdateArgs a, const dou
       reinterpret_cast<uint4*>(img)[t] = make_uint4(0u, 0u, 0u, 0u);
   }
   __syncthreads();
-#pragma unroll 4
-  for (int t = threadIdx.x; t < rows * l; t += kApplyThreads) {
-    const int rr = t / l, j = t - rr * l;
-    const int64_t o = base * l + t;
-    const double v = Q[o] * mult[j];
-    a.Omg[o] = v;
-    if (a.Omgf) a.Omgf[o] = (float)v;
-    if (a.i8.bq) tab.put(img, rr, j, lp, v);
-    if (a.bt1) {
-      const int64_t kp = tc_pos(base + rr);
-      const float x = (float)v;
-      const __nv_bfloat16 hi = __float2bfloat16_rn(x);
-      a.bt1[bt_elem(j, kp, 2 * a.bt_half)] = hi;
-      a.bt1[bt_elem(a.bt_half + j, kp, 2 * a.bt_half)] = __float2bfloat16_rn(x - __bfloat162float(hi));
+  constexpr int kBatch = 4;  // loads before the stores, which may alias for all the compiler knows
+  for (int t0 = threadIdx.x; t0 < rows * l; t0 += kBatch * kApplyThreads) {
+    double q[kBatch];
+#pragma unroll
+    for (int u = 0; u < kBatch; ++u) {
+      const int t = t0 + u * kApplyThreads;
+      q[u] = t < rows * l ? Q[base * l + t] : 0.0;
+    }
+#pragma unroll
+    for (int u = 0; u < kBatch; ++u) {
+      const int t = t0 + u * kApplyThreads, rr = t / l, j = t - rr * l;
+      if (t >= rows * l) break;
+      const int64_t o = base * l + t;
+      const double v = q[u] * mult[j];
+      a.Omg[o] = v;
+      if (a.Omgf) a.Omgf[o] = (float)v;
+      if (a.i8.bq) tab.put(img, rr, j, lp, v);
+      if (a.bt1) {
+        const int64_t kp = tc_pos(base + rr);
+        const float x = (float)v;
+        const __nv_bfloat16 hi = __float2bfloat16_rn(x);
+        a.bt1[bt_elem(j, kp, 2 * a.bt_half)] = hi;
+        a.bt1[bt_elem(a.bt_half + j, kp, 2 * a.bt_half)] = __float2bfloat16_rn(x - __bfloat162float(hi));
+      }
     }
   }
   if (!a.i8.bq) return;
