@@ -12,23 +12,6 @@
 
 namespace pg {
 
-void* scratch(pcaone_ctx* c, const std::string& name, size_t bytes) {
-  DevBuf& b = c->bufs[name];
-  if (b.bytes < bytes) {
-    if (b.p) PG_CUDA(cudaFree(b.p));
-    b.p = nullptr;
-    b.bytes = 0;
-    size_t alloc = round_up(std::max<size_t>(bytes, 256), 256);
-    PG_CUDA(cudaMalloc(&b.p, alloc));
-    b.bytes = alloc;
-  }
-  return b.p;
-}
-
-static void free_ptr(void* p) {
-  if (p) cudaFree(p);
-}
-
 // Forget the loaded data. Every data buffer is a named scratch buffer of the context (kept,
 // with its capacity, for the next load of the same or a smaller problem; freed by free_all).
 void free_data(pcaone_ctx* c) {
@@ -58,8 +41,7 @@ void free_data(pcaone_ctx* c) {
 
 void free_all(pcaone_ctx* c) {
   free_data(c);
-  for (auto& kv : c->bufs) free_ptr(kv.second.p);
-  c->bufs.clear();
+  free_scratch(c);
   c->bt2_shape = -1;
   c->bt2_ptr = nullptr;
   c->tiles_valid = false;

@@ -174,6 +174,7 @@ struct pcaone_ctx {
 
   // named scratch buffers (grown on demand, freed with the context)
   std::map<std::string, pg::DevBuf> bufs;
+  bool tall_ticket_zero = false;  // the ticket counter "tall_cnt" has been cleared
 
   // kernels whose dynamic shared-memory limit was raised on this context's device
   std::set<const void*> smem_attr_set;
@@ -195,7 +196,9 @@ struct pcaone_ctx {
 
 namespace pg {
 
+// Device buffer of that name, at least `bytes` long (buffers.cu).
 void* scratch(pcaone_ctx* c, const std::string& name, size_t bytes);
+void free_scratch(pcaone_ctx* c);
 void free_all(pcaone_ctx* c);
 
 // ---------------------------------------------------------------- bed kernels (kernels_bed.cu)

@@ -388,13 +388,6 @@ void to_colmajor(pcaone_ctx* c, const double* X, int64_t n, int l, int ld, doubl
   c->launches++;
 }
 
-unsigned* tall_counter(pcaone_ctx* c) {
-  const bool fresh = c->bufs.find("tall_cnt") == c->bufs.end();
-  unsigned* p = (unsigned*)scratch(c, "tall_cnt", sizeof(unsigned));
-  if (fresh) PG_CUDA(cudaMemsetAsync(p, 0, sizeof(unsigned), c->stream));
-  return p;
-}
-
 double* tall_part(pcaone_ctx* c, size_t doubles) {
   return (double*)scratch(c, "tall_part", (size_t)kTallMaxParts * doubles * 8);
 }

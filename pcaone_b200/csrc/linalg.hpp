@@ -33,7 +33,7 @@ struct TallStep {
   unsigned* counter = nullptr;
 };
 void tall_step(pcaone_ctx* c, TallStep s);
-// Ticket counter of the tall kernels (zero between launches) and room for the sums of
+// Ticket counter of the tall kernels (zero between launches; buffers.cu) and room for the sums of
 // kTallMaxParts clusters of up to `doubles` each.
 unsigned* tall_counter(pcaone_ctx* c);
 double* tall_part(pcaone_ctx* c, size_t doubles);
