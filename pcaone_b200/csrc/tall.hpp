@@ -51,8 +51,10 @@ struct Tall {
 __host__ __device__ __forceinline__ int64_t tall_rows_per_cta(int64_t n, int64_t ctas) {
   return ((n + ctas - 1) / ctas + 63) & ~int64_t(63);
 }
-// Clusters for n rows, at most cap of them.
+// Clusters for n rows, at most cap of them (one where the device holds no more at once: what a
+// launch sets aside for other work may leave cap at 0).
 inline int tall_clusters(int64_t n, int cap) {
+  if (cap < 1) cap = 1;
   const int64_t per = kTallCluster * tall_rows_per_cta(n, (int64_t)cap * kTallCluster);
   return (int)((n + per - 1) / per);
 }

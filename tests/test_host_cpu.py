@@ -24,3 +24,12 @@ def run(exe, *args):
 
 def test_buffers_survive_failed_allocations(tmp_path):
     run(program(tmp_path, "buffers_test", "buffers.cu"))
+
+
+def test_row_split_of_the_tall_passes(tmp_path):
+    """Every row count and cluster limit, down to a device that holds one cluster (or none beside the
+    one set aside for the signs): the clusters cover the rows and keep to the limit."""
+    exe = str(tmp_path / "tall")
+    subprocess.check_call([f"{CUDA}/bin/nvcc", "-std=c++17", "-gencode", "arch=compute_100a,code=sm_100a", "-o", exe,
+                           os.path.join(ROOT, "tests", "host", "tall_test.cu")])
+    run(exe)
