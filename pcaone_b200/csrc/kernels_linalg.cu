@@ -43,6 +43,7 @@ __global__ void __cluster_dims__(kTallCluster, 1, 1) __launch_bounds__(kTallThre
   using T = Tall<NT>;
   using C = TallCfg<NT, RECT>;
   constexpr int LD = T::LD, NB = C::NB, NACC = C::kAcc;
+  static_assert(PROD || !RECT, "a cross pass reads the rows of a product");
   constexpr bool kPrefetch = NT <= 5;
   extern __shared__ __align__(16) double sm[];
   double* Rs = sm;
@@ -121,7 +122,7 @@ __global__ void __cluster_dims__(kTallCluster, 1, 1) __launch_bounds__(kTallThre
 #pragma unroll
       for (int e = 0; e < 2; ++e) {
         if constexpr (RECT) {
-          const int64_t row = base + (PROD ? 2 * r4 + e : 4 * e + r4);
+          const int64_t row = base + 2 * r4 + e;
           double b[NB];
 #pragma unroll
           for (int j = 0; j < NB; ++j) {
@@ -396,8 +397,9 @@ void tall_step(pcaone_ctx* c, TallStep s) {
   PG_REQUIRE(s.l >= 1 && s.l <= kLmax && s.lb <= s.l, PCAONE_EBADARG, "sketch width out of range");
   PG_REQUIRE(s.n >= 1 && !(s.A2 && s.Rinv), PCAONE_EBADARG, "bad tall pass");
   PG_REQUIRE(!s.B || s.Q != s.A, PCAONE_EBADARG, "a cross pass may not overwrite its input");
+  PG_REQUIRE(!s.B || s.Rinv, PCAONE_EBADARG, "a cross pass needs the inverse factor");
   if (s.B)
-    s.Rinv ? launch_tall_nt<true, true>(c, s) : launch_tall_nt<false, true>(c, s);
+    launch_tall_nt<true, true>(c, s);
   else
     s.Rinv ? launch_tall_nt<true, false>(c, s) : launch_tall_nt<false, false>(c, s);
 }

@@ -11,7 +11,7 @@ namespace pg {
 //   Gram (B null):  W = q^T q = R^T R:  R, Ri = R^-1; with Rprev also Racc = R Rprev and, with
 //          Rprev_inv = Rprev^-1, Racc_inv = Rprev_inv Ri. status[0] gets 1 + the first column
 //          whose pivot is not positive.
-//   cross (B, n x lb, lb <= l):  X (l x lb) = q^T B; Ri, R, ... unused
+//   cross (B, n x lb, lb <= l; needs Rinv):  X (l x lb) = q^T B; Ri, R, ... unused
 // Square factors are l x l row-major, upper with zeros below; null outputs are not written.
 struct TallStep {
   const double* A = nullptr;
