@@ -21,6 +21,7 @@
 #include <numeric>
 #include <vector>
 
+#include "fp64.hpp"
 #include "internal.hpp"
 #include "linalg.hpp"
 #include "pdl.hpp"
@@ -36,13 +37,6 @@ __device__ __forceinline__ void posterior(double P0, double P1, double pt, doubl
   p0 = P0 * (1.0 - pt) * (1.0 - pt);
   p1 = P1 * 2 * pt * (1.0 - pt);
   p2 = (1 - P0 - P1) * pt * pt;
-}
-
-// 1 / x for the sum of the three weighted likelihoods of an entry, to the last bit or the one before;
-// sums out of the normal range (and NaN) take the division. The division itself was a third of
-// the arithmetic of an entry.
-__device__ __forceinline__ double likelihood_reciprocal(double x) {
-  return x > 1e-300 && x < 1e300 ? fast_reciprocal(x) : 1.0 / x;
 }
 
 // One EM sweep of the allele frequencies: warp per SNP, from F = init in the first sweep. The CTA
@@ -64,7 +58,7 @@ __global__ void __launch_bounds__(256) k_em_maf(const double* __restrict__ P, ui
       const double2 gl = __ldg(row + i);
       double p0, p1, p2;
       posterior(gl.x, gl.y, f, p0, p1, p2);
-      acc += (p1 + 2.0 * p2) * likelihood_reciprocal(p0 + p1 + p2);
+      acc += (p1 + 2.0 * p2) * reciprocal(p0 + p1 + p2);
     }
     for (int o = 16; o; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
     if (lane == 0) {
@@ -132,7 +126,7 @@ __global__ void __launch_bounds__(128) k_posterior_e(const double* __restrict__ 
       }
       double p0, p1, p2;
       posterior(gl.x, gl.y, pt, p0, p1, p2);
-      __stcs(E + (j0 + q) * lde + i, (float)((p1 + 2.0 * p2) * likelihood_reciprocal(p0 + p1 + p2) - 2.0 * f));
+      __stcs(E + (j0 + q) * lde + i, (float)((p1 + 2.0 * p2) * reciprocal(p0 + p1 + p2) - 2.0 * f));
     };
     auto pair = [&](int q) { return __ldcs(reinterpret_cast<const double2*>(P + (j0 + q) * ldp) + i); };
     int q = 0;
@@ -480,7 +474,7 @@ __global__ void __launch_bounds__(128) k_grm_e(const double* __restrict__ P, uin
                                                const double* __restrict__ F, const double* __restrict__ US,
                                                const double* __restrict__ V, int k, uint64_t j0, uint64_t mc,
                                                double* __restrict__ E, uint32_t lde, double* __restrict__ dpart) {
-  __shared__ double sf[kGrmSites], snorm[kGrmSites], sden[kGrmSites], sv[kGrmSites * KM];
+  __shared__ double sf[kGrmSites], snorm[kGrmSites], sh[kGrmSites], sih[kGrmSites], sv[kGrmSites * KM];
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   const uint64_t per = (mc + gridDim.y - 1) / gridDim.y;
   const uint64_t a = (uint64_t)blockIdx.y * per, b = (a + per < mc ? a + per : mc);
@@ -495,7 +489,8 @@ __global__ void __launch_bounds__(128) k_grm_e(const double* __restrict__ P, uin
       const double f = F[j0 + s0 + t], h = 2.0 * f * (1.0 - f), norm = sqrt(h);
       sf[t] = f;
       snorm[t] = norm > 1e-9 ? 1.0 / norm : 1.0;
-      sden[t] = 1.0 / h;
+      sh[t] = h;
+      sih[t] = 1.0 / h;
     }
     if (V)
       for (int t = threadIdx.x; t < ns * KM; t += blockDim.x)
@@ -515,10 +510,10 @@ __global__ void __launch_bounds__(128) k_grm_e(const double* __restrict__ P, uin
       }
       double p0, p1, p2;
       posterior(pp.x, pp.y, pt, p0, p1, p2);
-      const double inv = likelihood_reciprocal(p0 + p1 + p2);
+      const double sum = p0 + p1 + p2, inv = reciprocal(sum);
       E[(s0 + q) * lde + i] = ((p1 + 2.0 * p2) * inv - f2) * snorm[q];
-      const double t = (f2 * f2 * p0 + (1.0 - f2) * (1.0 - f2) * p1 + (2.0 - f2) * (2.0 - f2) * p2) * inv;
-      dc += t * sden[q];
+      const double t = f2 * f2 * p0 + (1.0 - f2) * (1.0 - f2) * p1 + (2.0 - f2) * (2.0 - f2) * p2;
+      dc += quotient(quotient(t, sum, inv), sh[q], sih[q]);
     }
   }
   if (i < N) dpart[(uint64_t)blockIdx.y * N + i] += dc;

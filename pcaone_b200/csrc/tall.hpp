@@ -16,6 +16,7 @@
 
 #include <cooperative_groups.h>
 
+#include "fp64.hpp"
 #include "internal.hpp"
 
 namespace pg {
@@ -98,16 +99,6 @@ __device__ __forceinline__ void block_load(double (&d)[2], const double* C, int 
 __device__ __forceinline__ void block_store(const double (&d)[2], double* C, int ldc) {
   const int q = (threadIdx.x & 31) >> 2, r = threadIdx.x & 3;
   *reinterpret_cast<double2*>(C + q * ldc + 2 * r) = make_double2(d[0], d[1]);
-}
-
-// 1 / x for a normal x whose reciprocal is normal, to the last bit or the one before: the hardware's
-// approximation (about 20 bits) and two Newton steps, y += y (1 - x y). The pivots below divide on
-// the dependent chain of the factorisation, where the rounded division is a few hundred cycles.
-__device__ __forceinline__ double fast_reciprocal(double x) {
-  double y;
-  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-  y = fma(y, fma(-x, y, 1.0), y);
-  return fma(y, fma(-x, y, 1.0), y);
 }
 
 // The 8 x 8 block factorisations run in one warp, lane (g, r) = (lane / 8, lane % 8) holding row r,
