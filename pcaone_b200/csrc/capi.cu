@@ -164,7 +164,8 @@ int pcaone_gpu_load_bed(pcaone_ctx* c, const uint8_t* packed, uint64_t nsnps, ui
     PG_CUDA(cudaMemsetAsync(c->d_bed + c->M * c->pitch, 0xFF, (c->Mpad - c->M) * c->pitch, c->stream));
     // the records as they lie in the file, to a staging area from which k_unpack writes the rows
     const size_t raw = (size_t)c->M * c->bpr;
-    if (raw < kXferMin || c->bpr > kXferSlot) {  // small, or records longer than a slot: 64 MiB at a time
+    const XferSlots slots = c->bpr > kXferSlot ? XferSlots(nullptr) : xfer_slots(c, raw);
+    if (!slots) {  // the caller's memory itself, 64 MiB at a time
       const uint64_t rows = std::min<uint64_t>(c->M, std::max<uint64_t>(1, (uint64_t(64) << 20) / c->bpr));
       uint8_t* stage = (uint8_t*)scratch(c, "bed_stage", rows * c->bpr + 8);
       for (uint64_t j0 = 0; j0 < c->M; j0 += rows) {
@@ -178,7 +179,7 @@ int pcaone_gpu_load_bed(pcaone_ctx* c, const uint8_t* packed, uint64_t nsnps, ui
       uint8_t* stage = (uint8_t*)scratch(c, "bed_stage", (size_t)xfer_workers() * slot_pad);
       const uint64_t rows = kXferSlot / c->bpr;
       const int64_t chunks = (int64_t)((c->M + rows - 1) / rows);
-      xfer_chunks(c, chunks, [&](int64_t i, int t, char* slot, cudaStream_t st) {
+      xfer_chunks(c, slots, chunks, [&](int64_t i, int t, char* slot, cudaStream_t st) {
         const uint64_t j0 = (uint64_t)i * rows, n = std::min(rows, c->M - j0);
         std::memcpy(slot, packed + j0 * c->bpr, n * c->bpr);
         PG_CUDA(cudaMemcpyAsync(stage + t * slot_pad, slot, n * c->bpr, cudaMemcpyHostToDevice, st));

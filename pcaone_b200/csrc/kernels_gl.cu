@@ -675,17 +675,23 @@ __global__ void k_widen(const float* __restrict__ in, size_t n, double* __restri
 }
 
 void gl_widen_f32(pcaone_ctx* c, const float* P, size_t n, double* dP) {
-  constexpr size_t chunk = kXferSlot / 4;  // floats
-  float* stage = (float*)scratch(c, "gl_stage", (size_t)xfer_workers() * kXferSlot);
-  if (n <= chunk) {
-    PG_CUDA(cudaMemcpyAsync(stage, P, n * 4, cudaMemcpyHostToDevice, c->stream));
-    k_widen<<<(unsigned)((n + 2047) / 2048), 256, 0, c->stream>>>(stage, n, dP);
-    PG_CHECK_LAUNCH();
-    c->launches++;
+  const XferSlots slots = xfer_slots(c, n * 4);
+  if (!slots) {  // the caller's memory itself, 64 MiB at a time
+    const size_t piece = std::min<size_t>(n, size_t(16) << 20);
+    float* stage = (float*)scratch(c, "gl_stage", piece * 4);
+    for (size_t o = 0; o < n; o += piece) {
+      const size_t m = std::min(piece, n - o);
+      PG_CUDA(cudaMemcpyAsync(stage, P + o, m * 4, cudaMemcpyHostToDevice, c->stream));
+      k_widen<<<(unsigned)((m + 2047) / 2048), 256, 0, c->stream>>>(stage, m, dP + o);
+      PG_CHECK_LAUNCH();
+      c->launches++;
+    }
     return;
   }
+  constexpr size_t chunk = kXferSlot / 4;  // floats
+  float* stage = (float*)scratch(c, "gl_stage", (size_t)xfer_workers() * kXferSlot);
   const int64_t chunks = (int64_t)((n + chunk - 1) / chunk);
-  xfer_chunks(c, chunks, [&](int64_t i, int t, char* slot, cudaStream_t st) {
+  xfer_chunks(c, slots, chunks, [&](int64_t i, int t, char* slot, cudaStream_t st) {
     const size_t o = (size_t)i * chunk, m = std::min(chunk, n - o);
     float* dst = stage + (size_t)t * chunk;
     std::memcpy(slot, P + o, m * 4);

@@ -1,11 +1,13 @@
 // Copies of pageable host memory. The runtime moves it through one staging buffer with one host
-// thread, and a large fresh result array is faulted in page by page on the way: 2 GB/s here, of a
-// link that does 50. A few threads that each copy 1 MiB chunks between the caller's array and
-// a pinned slot keep the link and the page faults going together (fresh arrays, 64 MB: 3.4 ms
-// against 31; 240 MB: 12.6 ms against 115).
-// Pinning memory takes milliseconds, so sets of slots (8 MiB each) are kept in the process and
-// shared by its contexts: a copy takes a set of its own, at most two idle sets are kept, and the
-// last context's end frees them. Streams belong to the context; the threads live for one call.
+// thread, and a large fresh result array is faulted in page by page on the way. A few threads that each
+// copy 1 MiB chunks between the caller's array and a pinned slot keep the link and the page faults
+// going together. Whole calls, with 16 host cores, two and one (through the runtime: 28, 56 and 2.0 ms):
+// a load of 100 MB of records 3.5, 7.0 and 12.4 ms; an LD call with 256 MB of results 17, 41 and 56 ms, with
+// 10 MB 1.6, 1.4 and 1.9.
+// Sets of slots (8 MiB each) are kept in the process and shared by its contexts: a copy takes a set of its
+// own, at most two idle sets are kept, and the last context's end frees them. Streams belong to
+// the context; the threads live for one call.
+// Where a set cannot be had the runtime's path serves.
 #include "xfer.hpp"
 
 #include <algorithm>
@@ -31,44 +33,54 @@ SlotPool& pool() {
   return *p;
 }
 
-// A set of pinned slots, one a worker, for the length of a copy.
-struct SlotSet {
-  void* p = nullptr;
-  SlotSet() {
-    {
-      std::lock_guard<std::mutex> g(pool().mu);
-      if (!pool().idle.empty()) {
-        p = pool().idle.back();
-        pool().idle.pop_back();
-      }
-    }
-    if (!p) PG_CUDA(cudaHostAlloc(&p, (size_t)xfer_workers() * kXferSlot, cudaHostAllocPortable));
-  }
-  ~SlotSet() {
-    {
-      std::lock_guard<std::mutex> g(pool().mu);
-      if (pool().contexts > 0 && pool().idle.size() < kKeptSets) {
-        pool().idle.push_back(p);
-        return;
-      }
-    }
-    cudaFreeHost(p);
-  }
-  SlotSet(const SlotSet&) = delete;
-  SlotSet& operator=(const SlotSet&) = delete;
-};
+void* idle_set() {
+  std::lock_guard<std::mutex> g(pool().mu);
+  if (pool().idle.empty()) return nullptr;
+  void* p = pool().idle.back();
+  pool().idle.pop_back();
+  return p;
+}
+
 }  // namespace
+
+XferSlots::~XferSlots() {
+  if (!p_) return;
+  {
+    std::lock_guard<std::mutex> g(pool().mu);
+    if (pool().contexts > 0 && pool().idle.size() < kKeptSets) {
+      pool().idle.push_back(p_);
+      return;
+    }
+  }
+  cudaFreeHost(p_);
+}
+
+XferSlots xfer_slots(pcaone_ctx* c, size_t bytes) {
+  if (bytes < kXferMin) return XferSlots(nullptr);
+  void* p = idle_set();
+  if (!p) {
+    if (cudaHostAlloc(&p, (size_t)xfer_workers() * kXferSlot, cudaHostAllocPortable) != cudaSuccess) {
+      (void)cudaGetLastError();
+      return XferSlots(nullptr);
+    }
+  }
+  XferSlots slots(p);
+  c->xfer_streams.resize(xfer_workers(), nullptr);
+  for (cudaStream_t& s : c->xfer_streams)
+    if (!s && cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking) != cudaSuccess) {
+      (void)cudaGetLastError();
+      s = nullptr;
+      return XferSlots(nullptr);
+    }
+  return slots;
+}
 
 int xfer_workers() {
   return (int)std::max(1u, std::min((unsigned)kMaxWorkers, std::thread::hardware_concurrency()));
 }
 
-void xfer_chunks(pcaone_ctx* c, int64_t chunks, const XferChunk& f) {
+void xfer_chunks(pcaone_ctx* c, const XferSlots& slots, int64_t chunks, const XferChunk& f) {
   const int workers = (int)std::min<int64_t>(xfer_workers(), chunks);
-  const SlotSet set;
-  c->xfer_streams.resize(xfer_workers(), nullptr);
-  for (int t = 0; t < workers; ++t)
-    if (!c->xfer_streams[t]) PG_CUDA(cudaStreamCreateWithFlags(&c->xfer_streams[t], cudaStreamNonBlocking));
   PG_CUDA(cudaStreamSynchronize(c->stream));
   std::atomic<int64_t> next{0};
   std::mutex mu;
@@ -78,7 +90,7 @@ void xfer_chunks(pcaone_ctx* c, int64_t chunks, const XferChunk& f) {
     try {
       PG_CUDA(cudaSetDevice(c->device));
       for (int64_t i; (i = next.fetch_add(1)) < chunks;) {
-        f(i, t, (char*)set.p + (size_t)t * kXferSlot, c->xfer_streams[t]);
+        f(i, t, slots.slot(t), c->xfer_streams[t]);
         PG_CUDA(cudaStreamSynchronize(c->xfer_streams[t]));
       }
     } catch (const Error& e) {
@@ -112,13 +124,19 @@ void xfer_chunks(pcaone_ctx* c, int64_t chunks, const XferChunk& f) {
   }
 }
 
+namespace {
+// The runtime's own path.
+void copy_plain(pcaone_ctx* c, void* dst, const void* src, size_t bytes, cudaMemcpyKind kind) {
+  if (bytes) PG_CUDA(cudaMemcpyAsync(dst, src, bytes, kind, c->stream));
+  PG_CUDA(cudaStreamSynchronize(c->stream));
+}
+int64_t chunks_of(size_t bytes) { return (int64_t)((bytes + kXferSlot - 1) / kXferSlot); }
+}  // namespace
+
 void copy_to_host(pcaone_ctx* c, void* dst, const void* src, size_t bytes) {
-  if (bytes < kXferMin) {
-    if (bytes) PG_CUDA(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, c->stream));
-    PG_CUDA(cudaStreamSynchronize(c->stream));
-    return;
-  }
-  xfer_chunks(c, (int64_t)((bytes + kXferSlot - 1) / kXferSlot), [&](int64_t i, int, char* slot, cudaStream_t st) {
+  const XferSlots slots = xfer_slots(c, bytes);
+  if (!slots) return copy_plain(c, dst, src, bytes, cudaMemcpyDeviceToHost);
+  xfer_chunks(c, slots, chunks_of(bytes), [&](int64_t i, int, char* slot, cudaStream_t st) {
     const size_t o = (size_t)i * kXferSlot, n = std::min(kXferSlot, bytes - o);
     PG_CUDA(cudaMemcpyAsync(slot, (const char*)src + o, n, cudaMemcpyDeviceToHost, st));
     PG_CUDA(cudaStreamSynchronize(st));
@@ -127,12 +145,9 @@ void copy_to_host(pcaone_ctx* c, void* dst, const void* src, size_t bytes) {
 }
 
 void copy_to_device(pcaone_ctx* c, void* dst, const void* src, size_t bytes) {
-  if (bytes < kXferMin) {
-    if (bytes) PG_CUDA(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, c->stream));
-    PG_CUDA(cudaStreamSynchronize(c->stream));
-    return;
-  }
-  xfer_chunks(c, (int64_t)((bytes + kXferSlot - 1) / kXferSlot), [&](int64_t i, int, char* slot, cudaStream_t st) {
+  const XferSlots slots = xfer_slots(c, bytes);
+  if (!slots) return copy_plain(c, dst, src, bytes, cudaMemcpyHostToDevice);
+  xfer_chunks(c, slots, chunks_of(bytes), [&](int64_t i, int, char* slot, cudaStream_t st) {
     const size_t o = (size_t)i * kXferSlot, n = std::min(kXferSlot, bytes - o);
     std::memcpy(slot, (const char*)src + o, n);
     PG_CUDA(cudaMemcpyAsync((char*)dst + o, slot, n, cudaMemcpyHostToDevice, st));

@@ -15,9 +15,28 @@ constexpr size_t kXferSlot = size_t(1) << 20;
 // still does 17 to 20 GB/s there (4 MB: 0.24 ms against 0.46; 8 MB: 0.45 against 0.38).
 constexpr size_t kXferMin = size_t(8) << 20;
 
+// A set of pinned slots, one a worker, held for the length of a copy.
+class XferSlots {
+ public:
+  explicit XferSlots(void* p) : p_(p) {}
+  XferSlots(XferSlots&& o) noexcept : p_(o.p_) { o.p_ = nullptr; }
+  XferSlots(const XferSlots&) = delete;
+  XferSlots& operator=(const XferSlots&) = delete;
+  ~XferSlots();
+  explicit operator bool() const { return p_ != nullptr; }
+  char* slot(int worker) const { return (char*)p_ + (size_t)worker * kXferSlot; }
+
+ private:
+  void* p_;
+};
+
+// Slots for a copy of bytes; none where the runtime's own copy serves better (a small copy) or the
+// slots cannot be had.
+XferSlots xfer_slots(pcaone_ctx* c, size_t bytes);
+
 // Runs f for the chunks 0 .. chunks - 1 on a few host threads, after the work queued on the
 // context's stream; returns when all of it is complete.
-void xfer_chunks(pcaone_ctx* c, int64_t chunks, const XferChunk& f);
+void xfer_chunks(pcaone_ctx* c, const XferSlots& slots, int64_t chunks, const XferChunk& f);
 int xfer_workers();
 
 // Synchronous copies, after the work queued on the context's stream.

@@ -18,10 +18,16 @@ struct Call {
     int f = fail.load();
     while (f > 0 && !fail.compare_exchange_weak(f, f - 1)) {
     }
+    if (f > 0) left();
     return f > 0 ? cudaErrorMemoryAllocation : cudaSuccess;
   }
+  static void left();
 };
-inline Call malloc_, memset_;
+inline Call malloc_, memset_, host_alloc, host_free, stream_create, copy;
+inline std::atomic<int> streams{0};
+inline std::atomic<bool> error_left{false};   // a failed call's code not yet taken by cudaGetLastError
+inline const char *pinned_from = nullptr, *pinned_to = nullptr;  // memory the test declares pinned
+inline void Call::left() { error_left = true; }
 }  // namespace fake
 
 #define CHECK(cond)                                              \
@@ -49,6 +55,37 @@ cudaError_t cudaMemsetAsync(void* p, int v, size_t n, cudaStream_t) {
   const cudaError_t e = fake::memset_.run();
   if (e == cudaSuccess) std::memset(p, v, n);
   return e;
+}
+cudaError_t cudaHostAlloc(void** p, size_t n, unsigned) {
+  const cudaError_t e = fake::host_alloc.run();
+  if (e == cudaSuccess) *p = std::malloc(n);
+  return e;
+}
+cudaError_t cudaFreeHost(void* p) {
+  fake::host_free.run();
+  std::free(p);
+  return cudaSuccess;
+}
+cudaError_t cudaStreamCreateWithFlags(cudaStream_t* s, unsigned) {
+  const cudaError_t e = fake::stream_create.run();
+  if (e == cudaSuccess) *s = (cudaStream_t)(size_t)++fake::streams;
+  return e;
+}
+cudaError_t cudaStreamDestroy(cudaStream_t) { return cudaSuccess; }
+cudaError_t cudaStreamSynchronize(cudaStream_t) { return cudaSuccess; }
+cudaError_t cudaSetDevice(int) { return cudaSuccess; }
+cudaError_t cudaMemcpyAsync(void* d, const void* s, size_t n, cudaMemcpyKind, cudaStream_t) {
+  const cudaError_t e = fake::copy.run();
+  if (e == cudaSuccess) std::memcpy(d, s, n);
+  return e;
+}
+cudaError_t cudaPointerGetAttributes(cudaPointerAttributes* a, const void* p) {
+  a->type = (const char*)p >= fake::pinned_from && (const char*)p < fake::pinned_to ? cudaMemoryTypeHost
+                                                                                   : cudaMemoryTypeUnregistered;
+  return cudaSuccess;
+}
+cudaError_t cudaGetLastError() {
+  return fake::error_left.exchange(false) ? cudaErrorMemoryAllocation : cudaSuccess;
 }
 const char* cudaGetErrorString(cudaError_t) { return "fake error"; }
 }

@@ -3,6 +3,8 @@
 import os
 import subprocess
 
+import pytest
+
 from tests.helpers import ROOT
 
 CUDA = os.environ.get("CUDA_HOME", "/usr/local/cuda")
@@ -33,3 +35,13 @@ def test_row_split_of_the_tall_passes(tmp_path):
     subprocess.check_call([f"{CUDA}/bin/nvcc", "-std=c++17", "-gencode", "arch=compute_100a,code=sm_100a", "-o", exe,
                            os.path.join(ROOT, "tests", "host", "tall_test.cu")])
     run(exe)
+
+
+@pytest.fixture(scope="module")
+def xfer(tmp_path_factory):
+    return program(tmp_path_factory.mktemp("xfer"), "xfer_test", "xfer.cu")
+
+
+@pytest.mark.parametrize("case", ["large", "no_slots", "failed", "at_once"])
+def test_large_host_copies(xfer, case):
+    run(xfer, case)
