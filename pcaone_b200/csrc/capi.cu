@@ -164,7 +164,7 @@ int pcaone_gpu_load_bed(pcaone_ctx* c, const uint8_t* packed, uint64_t nsnps, ui
     PG_CUDA(cudaMemsetAsync(c->d_bed + c->M * c->pitch, 0xFF, (c->Mpad - c->M) * c->pitch, c->stream));
     // the records as they lie in the file, to a staging area from which k_unpack writes the rows
     const size_t raw = (size_t)c->M * c->bpr;
-    const XferSlots slots = c->bpr > kXferSlot ? XferSlots(nullptr) : xfer_slots(c, raw);
+    const XferSlots slots = c->bpr > kXferSlot ? XferSlots(nullptr) : xfer_slots(c, packed, raw);
     if (!slots) {  // the caller's memory itself, 64 MiB at a time
       const uint64_t rows = std::min<uint64_t>(c->M, std::max<uint64_t>(1, (uint64_t(64) << 20) / c->bpr));
       uint8_t* stage = (uint8_t*)scratch(c, "bed_stage", rows * c->bpr + 8);

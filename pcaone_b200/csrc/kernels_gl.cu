@@ -675,7 +675,7 @@ __global__ void k_widen(const float* __restrict__ in, size_t n, double* __restri
 }
 
 void gl_widen_f32(pcaone_ctx* c, const float* P, size_t n, double* dP) {
-  const XferSlots slots = xfer_slots(c, n * 4);
+  const XferSlots slots = xfer_slots(c, P, n * 4);
   if (!slots) {  // the caller's memory itself, 64 MiB at a time
     const size_t piece = std::min<size_t>(n, size_t(16) << 20);
     float* stage = (float*)scratch(c, "gl_stage", piece * 4);

@@ -30,9 +30,9 @@ class XferSlots {
   void* p_;
 };
 
-// Slots for a copy of bytes; none where the runtime's own copy serves better (a small copy) or the
-// slots cannot be had.
-XferSlots xfer_slots(pcaone_ctx* c, size_t bytes);
+// Slots for a copy of bytes from or to `host`; none where the runtime's own copy serves better (a small
+// copy, memory that is pinned already) or the slots cannot be had.
+XferSlots xfer_slots(pcaone_ctx* c, const void* host, size_t bytes);
 
 // Runs f for the chunks 0 .. chunks - 1 on a few host threads, after the work queued on the
 // context's stream; returns when all of it is complete.

@@ -71,6 +71,23 @@ void copies_go_on_without_slots() {
   CHECK(calls(fake::copy, [&] { round_trip(&c, 40 * MiB); }) == 80);
 }
 
+void pinned_memory_is_not_staged() {
+  Context c;
+  round_trip(&c, 40 * MiB);
+  const std::vector<char> in = bytes(40 * MiB, 5);
+  std::vector<char> dev(in.size()), out(in.size());
+  fake::pinned_from = in.data();
+  fake::pinned_to = in.data() + in.size();
+  CHECK(calls(fake::copy, [&] { pg::copy_to_device(&c, dev.data(), in.data(), in.size()); }) == 1);
+  fake::pinned_from = out.data();
+  fake::pinned_to = out.data() + out.size();
+  CHECK(calls(fake::copy, [&] { pg::copy_to_host(&c, out.data(), dev.data(), out.size()); }) == 1);
+  CHECK(out == in);
+  fake::pinned_to -= 1;  // the last byte is not
+  CHECK(calls(fake::copy, [&] { pg::copy_to_host(&c, out.data(), dev.data(), out.size()); }) == 40);
+  fake::pinned_from = fake::pinned_to = nullptr;
+}
+
 void failed_copies_leave_the_context_usable() {
   Context c;
   round_trip(&c, 40 * MiB);
@@ -106,6 +123,7 @@ int main(int argc, char** argv) {
   const std::string name = argc > 1 ? argv[1] : "";
   if (name == "large") large_copies_pin_a_set_once();
   else if (name == "no_slots") copies_go_on_without_slots();
+  else if (name == "pinned") pinned_memory_is_not_staged();
   else if (name == "failed") failed_copies_leave_the_context_usable();
   else if (name == "at_once") contexts_copy_at_once();
   else return 2;

@@ -1,4 +1,4 @@
-"""Large host copies on the GPU: several contexts copying at once, and what
+"""Large host copies on the GPU: memory the caller has pinned, several contexts copying at once, and what
 a context that is loaded again keeps of the matrix before."""
 import threading
 
@@ -13,6 +13,44 @@ pytestmark = pytest.mark.gpu
 
 def records(N, M, seed):
     return np.random.default_rng(seed).integers(0, 256, (M, (N + 3) // 4), dtype=np.uint8)
+
+
+def pinned(a):
+    torch = pytest.importorskip("torch")
+    t = torch.empty(a.nbytes, dtype=torch.uint8, pin_memory=True)
+    out = t.numpy().view(a.dtype).reshape(a.shape)
+    out[...] = a
+    return out, t
+
+
+@pytest.mark.parametrize("N,M", [(17, 1800003), (4099, 70001)])
+def test_pinned_records_and_likelihoods(N, M):
+    """Records pinned by the caller (several pieces of 64 MiB, the last ragged): counts as from pageable
+    memory; likelihoods in both types: the same frequencies."""
+    a = records(N, M, 1)
+    p, _keep = pinned(a)
+    with pb.GpuContext(0) as c:
+        c.load_bed(p, N)
+        got = c.counts()
+        for x, y in zip(got, counts_of(a, N)):
+            np.testing.assert_array_equal(x, y)
+        for dtype in (np.float32, np.float64):
+            P = np.random.default_rng(2).random((60001, 2 * 101)).astype(dtype) / 2.5
+            c.load_gl(P.T)
+            F = c.gl_freq(3, 0.0)[0]
+            q, _k = pinned(P)
+            c.load_gl(q.T)
+            np.testing.assert_array_equal(c.gl_freq(3, 0.0)[0], F)
+
+
+def test_pinned_and_pageable_results(gpu):
+    N, M = 301, 30011
+    gpu.load_bed(records(N, M, 3), N)
+    ref = gpu.residuals()
+    assert ref.nbytes > 32 << 20
+    out, _keep = pinned(np.full_like(ref, np.nan))
+    gpu._check(pb.lib().pcaone_gpu_residuals(gpu._h, None, None, None, 0, 0, M, pb._ptr(out)))
+    np.testing.assert_array_equal(out, ref)
 
 
 def test_contexts_copy_at_once():
