@@ -190,6 +190,7 @@ struct pcaone_ctx {
   cudaEvent_t ev_tail = nullptr;
   // streams of the large host copies' workers (xfer.cu)
   std::vector<cudaStream_t> xfer_streams;
+  size_t xfer_paged = 0;  // bytes of large copies made without pinned slots
   double gemm_ms_accum = 0.0;
   int64_t launches = 0, gemm_launches = 0;
 };

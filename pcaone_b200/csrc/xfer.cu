@@ -7,9 +7,11 @@
 // Sets of slots (8 MiB each) are kept in the process and shared by its contexts: a copy takes a set of its
 // own, at most two idle sets are kept, and the last context's end frees them. Streams belong to
 // the context; the threads live for one call.
-// Where a set cannot be had the runtime's path serves, and memory that the caller has pinned goes
-// straight to the link (a load of 100 MB of records: 1.9 ms; through the slots 3.5 with 16
-// host cores, 12.4 with one).
+// Pinning a set takes 3 to 11 ms, so it is pinned once the copies that a context made without one come
+// to kXferPaidOff (first LD call of a context, 2504 x 5000 with 10 MB of results: 1.6 to 3 ms;
+// 10 to 16 with a set pinned at once). Where a set cannot be had the runtime's path serves, and
+// memory that the caller has pinned goes straight to the link (a load of 100 MB of records: 1.9 ms;
+// through the slots 3.5 with 16 host cores, 12.4 with one).
 #include "xfer.hpp"
 
 #include <algorithm>
@@ -69,6 +71,8 @@ XferSlots xfer_slots(pcaone_ctx* c, const void* host, size_t bytes) {
   if (bytes < kXferMin || reachable(host, bytes)) return XferSlots(nullptr);
   void* p = idle_set();
   if (!p) {
+    c->xfer_paged += bytes;
+    if (c->xfer_paged < kXferPaidOff) return XferSlots(nullptr);
     if (cudaHostAlloc(&p, (size_t)xfer_workers() * kXferSlot, cudaHostAllocPortable) != cudaSuccess) {
       (void)cudaGetLastError();
       return XferSlots(nullptr);

@@ -15,6 +15,10 @@ constexpr size_t kXferSlot = size_t(1) << 20;
 // still does 17 to 20 GB/s there (4 MB: 0.24 ms against 0.46; 8 MB: 0.45 against 0.38).
 constexpr size_t kXferMin = size_t(8) << 20;
 
+// A set of slots is pinned for a context whose copies without one have come to this: they took 0.05
+// (recently used pages) to 0.45 ms (fresh ones) a MiB longer, the set takes 3 to 11 ms.
+constexpr size_t kXferPaidOff = size_t(32) << 20;
+
 // A set of pinned slots, one a worker, held for the length of a copy.
 class XferSlots {
  public:
@@ -31,7 +35,7 @@ class XferSlots {
 };
 
 // Slots for a copy of bytes from or to `host`; none where the runtime's own copy serves better (a small
-// copy, memory that is pinned already) or the slots cannot be had.
+// copy, memory that is pinned already, a set not paid off) or the slots cannot be had.
 XferSlots xfer_slots(pcaone_ctx* c, const void* host, size_t bytes);
 
 // Runs f for the chunks 0 .. chunks - 1 on a few host threads, after the work queued on the

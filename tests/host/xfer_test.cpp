@@ -41,6 +41,21 @@ int calls(const fake::Call& k, F&& f) {
   return k.calls - before;
 }
 
+void small_and_cold_copies_take_one_call() {
+  Context c;
+  const std::vector<char> in = bytes(10 * MiB, 3);
+  std::vector<char> dev(in.size());
+  auto copy = [&](size_t n) { pg::copy_to_device(&c, dev.data(), in.data(), n); };
+  CHECK(calls(fake::host_alloc, [&] {
+          for (const size_t n : {size_t(0), size_t(1), 8 * MiB - 1})
+            CHECK(calls(fake::copy, [&] { copy(n); }) == (n ? 1 : 0));
+          for (int i = 0; i < 3; ++i) CHECK(calls(fake::copy, [&] { copy(10 * MiB); }) == 1);  // 30 MiB in all
+        }) == 0);
+  CHECK(calls(fake::host_alloc, [&] { CHECK(calls(fake::copy, [&] { copy(10 * MiB); }) == 10); }) == 1);  // paid off
+  CHECK(calls(fake::host_alloc, [&] { CHECK(calls(fake::copy, [&] { copy(9 * MiB + 5); }) == 10); }) == 0);
+  CHECK(dev == in);
+}
+
 void large_copies_pin_a_set_once() {
   {
     Context c;
@@ -121,7 +136,8 @@ void contexts_copy_at_once() {
 
 int main(int argc, char** argv) {
   const std::string name = argc > 1 ? argv[1] : "";
-  if (name == "large") large_copies_pin_a_set_once();
+  if (name == "cold") small_and_cold_copies_take_one_call();
+  else if (name == "large") large_copies_pin_a_set_once();
   else if (name == "no_slots") copies_go_on_without_slots();
   else if (name == "pinned") pinned_memory_is_not_staged();
   else if (name == "failed") failed_copies_leave_the_context_usable();

@@ -42,6 +42,6 @@ def xfer(tmp_path_factory):
     return program(tmp_path_factory.mktemp("xfer"), "xfer_test", "xfer.cu")
 
 
-@pytest.mark.parametrize("case", ["large", "no_slots", "pinned", "failed", "at_once"])
+@pytest.mark.parametrize("case", ["cold", "large", "no_slots", "pinned", "failed", "at_once"])
 def test_large_host_copies(xfer, case):
     run(xfer, case)
