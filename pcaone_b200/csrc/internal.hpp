@@ -193,6 +193,7 @@ struct pcaone_ctx {
   size_t xfer_paged = 0;  // bytes of large copies made without pinned slots
   double gemm_ms_accum = 0.0;
   int64_t launches = 0, gemm_launches = 0;
+  int64_t graph_epochs = 0;  // epoch bodies launched as graphs
 };
 
 namespace pg {

@@ -503,6 +503,7 @@ struct Engine {
     }
     if (steady_exec[par]) {  // replay, with the host-side counters the body would have advanced
       PG_CUDA(cudaGraphLaunch(steady_exec[par], c->stream));
+      c->graph_epochs++;
       updates += steady_updates;
       c->launches += steady_launches;
       c->gemm_launches += steady_gemm_launches;
@@ -528,7 +529,8 @@ struct Engine {
       if (graph) cudaGraphDestroy(graph);
     }
     if (!ok) {  // capture refused: run this epoch and the rest directly (nothing was executed)
-      (void)cudaGetLastError();
+      const cudaError_t e = cudaGetLastError();
+      if (o.verbose) fprintf(stderr, "epochs are not launched as graphs: %s\n", cudaGetErrorString(e));
       for (auto& ex : steady_exec) {
         if (ex) cudaGraphExecDestroy(ex);
         ex = nullptr;
@@ -544,6 +546,7 @@ struct Engine {
     steady_launches = c->launches - l0;
     steady_gemm_launches = c->gemm_launches - g0;
     PG_CUDA(cudaGraphLaunch(steady_exec[par], c->stream));
+    c->graph_epochs++;
   }
 
   void epoch_halko(int pi) {
@@ -956,6 +959,8 @@ void run_gram(pcaone_ctx* c, int precision, int standardize, int ploidy, const d
     throw Error(PCAONE_EBADARG, "unknown precision");
   }
 }
+
+int64_t graph_epochs(const pcaone_ctx* c) { return c->graph_epochs; }
 
 double* product_t_device(pcaone_ctx* c, const double* B, int l) {
   PG_REQUIRE(c->loaded && !c->dense && !c->streamed, PCAONE_ESTATE, "products need resident packed genotypes");

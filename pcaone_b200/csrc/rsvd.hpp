@@ -70,6 +70,8 @@ void gl_release(pcaone_ctx* c);
 // The sketch drawn on the device, row-major npad x l (zero past nrow) and its optional FP32 copy.
 void omega_device(pcaone_ctx* c, int seed, int rand, uint64_t nrow, int l, uint64_t npad, double* O, float* Of);
 void omega_host(int seed, int rand, uint64_t nrow, uint32_t ncol, double* out);
+// Epoch bodies that the context's RSVDs have launched as graphs.
+int64_t graph_epochs(const pcaone_ctx* c);
 void jacobi_svd(int n, const double* A, double* U, double* s, double* V);
 void run_product(pcaone_ctx* c, int precision, int transpose, int standardize, int ploidy,
                  const double* B, int l, double* out);
