@@ -106,7 +106,7 @@ struct pcaone_ctx {
   cudaStream_t tile_stream = nullptr;
   size_t slot_budget = 0;  // device bytes per slot (records, transposed copy, tiles)
   struct StreamSlot {
-    int b0 = -1, b1 = -1;  // windows held, once `ready` has completed on the copy stream
+    int b0 = -1, b1 = -1;  // windows held, once `ready` has completed on the tile stream
     uint64_t key = 0;      // data generation, window layout and tile kind of the contents
     uint8_t *rec = nullptr, *recT = nullptr, *t1 = nullptr, *t2 = nullptr;
     cudaEvent_t copied = nullptr; // records copied (copy stream)

@@ -463,11 +463,13 @@ void dense_none_b2(pcaone_ctx*, const float*, int, int64_t) {}
 // and the slice's diagonal sum is added to dpart[slice * N + i] (each entry has one owner and
 // the chunks run in stream order, so the sums are deterministic). US: N x k (U diag S) and
 // V: M x k row-major as in k_posterior_e; V null: pt = F_j. KM >= k.
-// Bound by HBM (16 B read, 8 B written per sample-site). The values that depend on the site
-// alone (two divisions and a square root, and the loading row) are worked out once per CTA
-// into shared memory, kGrmSites sites at a time, and the sample's row of US stays in registers;
-// each sample-site is left with one division. N = 1501, M = 40000: 558 us = 2.6 TB/s (1245 with the
-// factors read per site from global memory and six divisions).
+// The values that depend on the site alone (two reciprocals and a square root, and the loading row) are
+// worked out once per CTA into shared memory, kGrmSites sites at a time, and the sample's row of
+// US stays in registers; a sample-site is left with one reciprocal, which both of its quotients
+// use. Bound by the latency of the pairs' loads: the slices, at most 64 so that their diagonal
+// sums stay few, leave ten warps an SM (16% of its places; FP64 pipe 19%, memory 17%).
+// N = 1501, M = 40000: 577 us = 2.5 TB/s (558 without the quotients' refinement, 1245 with the factors
+// read per site from global memory and six divisions).
 constexpr int kGrmSites = 64;
 template <int KM>
 __global__ void __launch_bounds__(128) k_grm_e(const double* __restrict__ P, uint32_t N, uint32_t ldp,

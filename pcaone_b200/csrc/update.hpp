@@ -19,7 +19,7 @@ struct UpdateArgs {
   double* H1 = nullptr;        // the sketch is H1 + H2 (written to H) when H2 is given, else H
   const double* H2 = nullptr;
   double* H = nullptr;
-  double* Q = nullptr;         // N x l work (Q1 then Q)
+  double* Q = nullptr;         // N x l work: the orthonormal factor before the signs
   double* Omg = nullptr;       // N x l: the previous Omega in, the new one out
   float* Omgf = nullptr;       // FP32 operand copy (SIMT path) or null
   OmegaI8 i8;                  // int8 operand (bq null: none)
