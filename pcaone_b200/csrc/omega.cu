@@ -319,16 +319,19 @@ void omega_device(pcaone_ctx* c, int seed, int rand, uint64_t nrow, int l, uint6
   // candidates for n / 2 accepted pairs at acceptance pi / 4 with more than 3% to spare, and again
   // twice as many in the case that was not enough
   const uint64_t kept = (n + 1) / 2;
-  auto* open = (OpenPair*)scratch(c, "omega_open", (1 + kept) * sizeof(OpenPair));
-  PG_CUDA(cudaMemsetAsync(open, 0, sizeof(OpenPair), c->stream));
+  OpenPair* open = nullptr;
   for (uint64_t pairs = (uint64_t)((double)n / 2 / 0.76) + 1024;; pairs *= 2) {
     const unsigned ctas = (unsigned)((pairs + kPairsPerCta - 1) / kPairsPerCta);
-    int64_t* cnt = (int64_t*)scratch(c, "omega_count", (size_t)ctas * 8);
-    int64_t* base = (int64_t*)scratch(c, "omega_base", ((size_t)ctas + 1) * 8);
+    // one buffer for the list and the counts: each allocation is felt in a context's first call
+    const size_t list = round_up((1 + kept) * sizeof(OpenPair), 256), counts = round_up((size_t)ctas * 8, 256);
+    char* work = (char*)scratch(c, "omega_work", list + counts + ((size_t)ctas + 1) * 8);
+    open = (OpenPair*)work;
+    int64_t *cnt = (int64_t*)(work + list), *base = (int64_t*)(work + list + counts);
     k_omega_pairs<<<ctas, kPairsPerCta, 0, c->stream>>>(x0, n, nrow, l, nullptr, cnt, O, Of, open);
     PG_CHECK_LAUNCH();
     c->launches++;
     if ((uint64_t)scan_counts(c, cnt, ctas, base) < kept) continue;
+    PG_CUDA(cudaMemsetAsync(open, 0, sizeof(OpenPair), c->stream));
     k_omega_pairs<<<ctas, kPairsPerCta, 0, c->stream>>>(x0, n, nrow, l, base, cnt, O, Of, open);
     PG_CHECK_LAUNCH();
     c->launches++;
